@@ -99,6 +99,14 @@ def interior_nodes(s) -> int:
     return inlet + mixing
 
 
+def face_nodes(s) -> int:
+    """The inlet, outlet and wall face nodes (no edges and corners)."""
+    z, ib = s.nz - 2, s.ia + s.mnx - 1
+    x = 2 * (s.iny - 2) * z + 2 * (s.mny - 1) * z
+    y = ((s.inx - 2) + (s.ia - 2) + (s.inx - 1 - ib) + (s.mnx - 2)) * z
+    return x + y + 2 * ((s.inx - 2) * (s.iny - 2) + (s.mnx - 2) + (s.mnx - 2) * (s.mny - 1))
+
+
 def w_layout_umean(W: int, u_max: float) -> float:
     """The reference's Umean for a W-layout mixer whose duct profile peaks at
     u_max, computed without the CUDA library (the reference arm must not load
@@ -385,9 +393,11 @@ def run_ours(args, dist: Dist) -> dict | None:
         s.close()
         bulk_ms, bnd_ms = tb / kr, tbd / kr
         bpl = FORM_BYTES[form]
-        # nodes the interior kernel updates: the interior ones, and with the
-        # sweep shape the z wall faces (one per interior column at each end)
-        bulk_nodes = counts["interior"] + (2 * counts["interior"] // (sp.nz - 2) if form == "fp16" else 0)
+        # nodes the interior kernel updates: the interior ones, with the sweep
+        # shape the z wall faces too (one per interior column at each end), in
+        # the FP64 form every face
+        bulk_nodes = counts["interior"] + (face_nodes(sp) if form == "fp64" else
+                                           2 * counts["interior"] // (sp.nz - 2) if form == "fp16" else 0)
         bulk_bytes = bulk_nodes * bpl
         achieved = bulk_bytes / (bulk_ms * 1e-3) / 1e9
         return dict(counts=counts, ms_max=ms_max, clk=clk, bulk_ms=bulk_ms, bnd_ms=bnd_ms, bulk_bytes=bulk_bytes,
@@ -404,6 +414,8 @@ def run_ours(args, dist: Dist) -> dict | None:
                 "frac": main["achieved"] / peaks["hbm_gbs"], "traffic": traffic,
                 "kernel": ("k_sweep4_f16 (interior nodes and z wall faces, %d per launch)" % main["bulk_nodes"]
                            if args.form == "fp16" else
+                           "k_run128_f64 (interior and face nodes, %d per launch)" % main["bulk_nodes"]
+                           if args.form == "fp64" else
                            "k_bulk_%s (interior nodes, %d per launch)" % (args.form, counts["interior"])),
                 "peak_source": peaks["source"],
                 "algorithmic_bytes_per_lup": FORM_BYTES[args.form],
@@ -492,7 +504,8 @@ def run_ours(args, dist: Dist) -> dict | None:
             "data": "synthetic",
             "form": form_text[args.form], "config": config_dict(workload_params(), dist.world),
             "roofline": roofline, "cpu_baseline": cpu, "e2e": e2e, "clocks": clk,
-            "gpu_launches": 3 * args.steps, "forms": forms, "reference_case": refcase, "batched": batched,
+            "gpu_launches": (1 if args.form == "fp64" else 3) * args.steps, "forms": forms,
+            "reference_case": refcase, "batched": batched,
             "served": served}
 
 

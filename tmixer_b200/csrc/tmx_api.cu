@@ -75,10 +75,14 @@ struct tmx_handle {
     cudaStream_t aux = nullptr, aux2 = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr, join2 = nullptr;
     int nface = 0;  // the first nface boundary nodes are face classes
-    int nwall = 0;  // the last nwall are wall faces (StepKernels::walls)
-    // FP32 / FP16 forms: the last nzwall faces are the z wall faces, which
-    // the sweep kernels update (boundary_list)
+    // the last nzwall faces are the z wall faces, which the sweep kernels
+    // update (boundary_list)
     int nzwall = 0;
+    // FP64 form: the run list and grid of k_run_f64, its two run counters
+    int4* runs = nullptr;
+    int nruns = 0, run_slots = 0, run_nt = 256;
+    int* counters = nullptr;
+    int* error = nullptr;  // mapped host memory: set by a kernel whose copies did not arrive
     // one captured step per (state buffer, macroscopic output) combination
     cudaGraphExec_t graph[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
     int sbytes = 8, tbytes = 8;  // storage / arithmetic bytes per value of the form
@@ -91,9 +95,9 @@ struct tmx_handle {
 };
 
 const StepKernels tmx_host::kForms[3] = {
-    {tmx::k_init_f64, tmx::k_bulk_f64, nullptr, nullptr, tmx::k_bound_f64, tmx::k_walls_f64, 8, 8, false, true},
-    {tmx::k_init_f32, tmx::k_bulk_f32, tmx::k_bfaces_f32, tmx::k_bedges_f32, nullptr, nullptr, 4, 4, false, false},
-    {tmx::k_init_f16, tmx::k_bulk_f16, tmx::k_bfaces_f16, tmx::k_bedges_f16, nullptr, nullptr, 2, 4, true, false},
+    {tmx::k_init_f64, nullptr, nullptr, nullptr, {tmx::k_run128_f64, tmx::k_run256_f64}, 8, 8, false, true},
+    {tmx::k_init_f32, tmx::k_bulk_f32, tmx::k_bfaces_f32, tmx::k_bedges_f32, {nullptr, nullptr}, 4, 4, false, false},
+    {tmx::k_init_f16, tmx::k_bulk_f16, tmx::k_bfaces_f16, tmx::k_bedges_f16, {nullptr, nullptr}, 2, 4, true, false},
 };
 
 namespace tmx_host {
@@ -333,16 +337,16 @@ void inlet_profile(const tmx_case& c, std::vector<double>& U1, std::vector<doubl
 }
 
 int boundary_list(const Geom& G, std::vector<int>& nodes, std::vector<unsigned char>& cls, int& nface,
-                  std::vector<int>* class_count, int* nwall, int* nzwall)
+                  std::vector<int>* class_count, int* nzwall)
 {
     struct Entry {
-        int cls, wall, node;
+        int cls, node;
         bool zwall;
     };
     std::vector<Entry> all;
     all.reserve((size_t)boundary_count(G));
     if (class_count) class_count->assign(tmx::K_NCLASSES, 0);
-    bool zsep = nzwall != nullptr && nwall == nullptr;
+    bool zsep = nzwall != nullptr;
     long long zcount = 0, interior2 = 0;
     for (int b = 0; b < 2; b++)
         for (int i = 1; i <= G.nx[b]; i++)
@@ -353,10 +357,6 @@ int boundary_list(const Geom& G, std::vector<int>& nodes, std::vector<unsigned c
                     const int c = classify(G, b, i, j, k);
                     if (c < 0)
                         return fail(TMX_E_INVALID, "internal: boundary node (%d,%d,%d,%d) has no class", b, i, j, k);
-                    const int w = tmx::wall_class(G, b, i, j, k);
-                    if (w != (tmx::is_wall_class(c) ? c : -1))
-                        return fail(TMX_E_INVALID, "internal: wall class %d of node (%d,%d,%d,%d), class %d", w, b, i,
-                                    j, k, c);
                     if (class_count) (*class_count)[c]++;
                     const bool zw = c == tmx::K_FACE_Z1 || c == tmx::K_FACE_ZT;
                     if (zw) {
@@ -366,46 +366,76 @@ int boundary_list(const Geom& G, std::vector<int>& nodes, std::vector<unsigned c
                         if (k != kw || G.nz < 3 || tmx::is_boundary(G, b, i, j, kn)) zsep = false;
                         zcount++;
                     }
-                    all.push_back({c, w, tmx::node_index(G, b, i, j, k), zw});
+                    all.push_back({c, tmx::node_index(G, b, i, j, k), zw});
                 }
             }
     // every z wall node above or below an interior node, and every interior
     // node of planes 2 and nz - 1 under or over one
     if (zcount != 2 * interior2) zsep = false;
-    if (nzwall && nwall == nullptr && !zsep && interior2 > 0)
+    if (nzwall && !zsep && interior2 > 0)
         return fail(TMX_E_INVALID, "internal: the z wall faces do not pair with the interior nodes of planes 2 and %d",
                     G.nz - 1);
     // faces first (with zsep the z wall faces last among them), then edges
-    // and corners (then, with nwall, the wall faces); by class, then node
+    // and corners; by class, then node
     std::vector<std::pair<int, int>> bl;
     bl.reserve(all.size());
-    for (const Entry& e : all) {
-        const int key = (nwall && e.wall >= 0)
-                            ? 512
-                            : (tmx::is_face_class(e.cls) ? (zsep && e.zwall ? 128 : 0) : 256) + e.cls;
-        bl.emplace_back(key, e.node);
-    }
+    for (const Entry& e : all)
+        bl.emplace_back((tmx::is_face_class(e.cls) ? (zsep && e.zwall ? 128 : 0) : 256) + e.cls, e.node);
     std::sort(bl.begin(), bl.end());
     nodes.resize(bl.size());
     cls.resize(bl.size());
     nface = 0;
-    int nw = 0, nzw = 0;
+    int nzw = 0;
     for (size_t t = 0; t < bl.size(); t++) {
         nodes[t] = bl[t].second;
-        if (bl[t].first == 512) {  // the walls in node order
-            int b, i, j, k;
-            tmx::decode(G, nodes[t], b, i, j, k);
-            cls[t] = (unsigned char)tmx::wall_class(G, b, i, j, k);
-            nw++;
-        } else {
-            cls[t] = (unsigned char)(bl[t].first & 127);
-        }
+        cls[t] = (unsigned char)(bl[t].first & 127);
         if (bl[t].first < 256) nface++;
         if (bl[t].first >= 128 && bl[t].first < 256) nzw++;
     }
-    if (nwall) *nwall = nw;
     if (nzwall) *nzwall = nzw;
     return TMX_OK;
+}
+
+// The flags lie in one page of the process, mapped when the first is taken
+// (mapping memory takes about a millisecond, a handle's creation two); beyond
+// its 1024 a flag is mapped by itself.
+namespace {
+constexpr int kFlags = 1024;
+std::mutex g_flag_mu;
+int* g_flags = nullptr;
+bool g_flag_used[kFlags];
+}  // namespace
+
+int* error_flag_take()
+{
+    std::lock_guard<std::mutex> lk(g_flag_mu);
+    const unsigned how = cudaHostAllocMapped | cudaHostAllocPortable;
+    if (!g_flags && cudaHostAlloc((void**)&g_flags, kFlags * sizeof(int), how) != cudaSuccess) {
+        g_flags = nullptr;
+        cudaGetLastError();
+        return nullptr;
+    }
+    for (int i = 0; i < kFlags; i++)
+        if (!g_flag_used[i]) {
+            g_flag_used[i] = true;
+            g_flags[i] = 0;
+            return g_flags + i;
+        }
+    int* f = nullptr;
+    if (cudaHostAlloc((void**)&f, sizeof(int), how) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    *f = 0;
+    return f;
+}
+
+void error_flag_give(int* flag)
+{
+    if (!flag) return;
+    std::lock_guard<std::mutex> lk(g_flag_mu);
+    if (flag >= g_flags && flag < g_flags + kFlags) g_flag_used[flag - g_flags] = false;
+    else cudaFreeHost(flag);
 }
 
 }  // namespace tmx_host
@@ -442,6 +472,12 @@ void free_all(tmx_handle* h)
     cudaFree(h->partial);
     cudaFree(h->tiles);
     h->tiles = nullptr;
+    cudaFree(h->runs);
+    cudaFree(h->counters);
+    error_flag_give(h->error);
+    h->error = nullptr;
+    h->runs = nullptr;
+    h->counters = nullptr;
     cudaFree(h->diag);
     h->diag = nullptr;
     h->mac = h->stats = h->partial = nullptr;
@@ -451,11 +487,38 @@ void free_all(tmx_handle* h)
     h->stream = nullptr;
 }
 
-// Queue the two kernels of one step from buffer `cur`: the boundary kernel on
-// the auxiliary stream, forked from and joined back into the main stream, and
-// the bulk kernel on the main stream.  With ev (4 events) each kernel is
-// bracketed by its own pair of events.  The state and density buffers flip
-// together every step, so one parity index selects both.
+// The FP64 step from buffer `cur`: one launch.  With ev (4 events) the edges
+// and the runs are launched one after the other, so that each event pair times
+// its part alone.
+int enqueue_run(tmx_handle* h, const tmx::StepPtrs& X, int cur, int write_macro, cudaEvent_t* ev)
+{
+    const int ne = h->nb - h->nface, nr = h->nruns;
+    auto launch = [&](int nruns, int nedges) {
+        const int per = h->run_nt / tmx::kBoundaryLanesHost;
+        const int blocks = std::max(1, std::min(h->run_slots, (nedges + per - 1) / per + nruns));
+        h->K->run[h->run_nt > 128]<<<blocks, h->run_nt, tmx::run_smem_host(h->run_nt), h->stream>>>(
+            X, h->G, h->P, write_macro, h->runs, nruns, h->bnode + h->nface, h->bcls + h->nface, nedges, h->counters,
+            cur, h->error);
+    };
+    if (ev) {
+        TMX_CK(cudaEventRecord(ev[2], h->stream));
+        launch(0, ne);
+        TMX_CK(cudaEventRecord(ev[3], h->stream));
+        TMX_CK(cudaEventRecord(ev[0], h->stream));
+        launch(nr, 0);
+        TMX_CK(cudaEventRecord(ev[1], h->stream));
+    } else {
+        launch(nr, ne);
+    }
+    TMX_CK(cudaGetLastError());
+    return TMX_OK;
+}
+
+// Queue one step from buffer `cur`: the face and the edge kernel on the two
+// auxiliary streams, forked from and joined back into the main stream, and the
+// bulk kernel on the main stream (FP64: enqueue_run).  With ev (4 events) each
+// part is bracketed by its own pair of events.  The state and density buffers
+// flip together every step, so one parity index selects both.
 int enqueue_step(tmx_handle* h, int cur, int write_macro, cudaEvent_t* ev)
 {
     const Geom& G = h->G;
@@ -469,47 +532,31 @@ int enqueue_step(tmx_handle* h, int cur, int write_macro, cudaEvent_t* ev)
     X.mcur = h->mom[1 - cur];
     X.uin1 = h->uin_d[0];
     X.uin2 = h->uin_d[1];
+    if (h->K->run[0]) return enqueue_run(h, X, cur, write_macro, ev);
     TMX_CK(cudaEventRecord(h->fork, h->stream));
     TMX_CK(cudaStreamWaitEvent(h->aux, h->fork, 0));
     TMX_CK(cudaStreamWaitEvent(h->aux2, h->fork, 0));
     if (ev) TMX_CK(cudaEventRecord(ev[2], h->aux));
-    const int nf = h->nface, nw = h->nwall, ne = h->nb - h->nface - h->nwall;
+    const int nf = h->nface, ne = h->nb - h->nface;
     const int bt = tmx::kBoundaryThreadsHost, nl = tmx::kBoundaryLanesHost;  // nl threads per node
-    if (h->K->serial) {
-        // one launch, the edge and corner blocks first: their long per-node
-        // chains then run beside the face blocks instead of after them
-        // (W=32 FP64 step 198.5 us against 203.4 us as two launches)
-        const int eb = (nl * ne + bt - 1) / bt, fb = (nl * nf + bt - 1) / bt;
-        if (eb + fb > 0)
-            h->K->bound<<<eb + fb, bt, 0, h->aux>>>(X, h->bnode, h->bcls, nf, ne, eb, G, h->P, write_macro);
-        if (nw > 0)
-            h->K->walls<<<(nw + bt - 1) / bt, bt, 0, h->aux2>>>(X, h->bnode + nf + ne, h->bcls + nf + ne, nw, G, h->P,
-                                                                write_macro);
-    } else {
-        // with a sweep shape the interior kernel updates the z wall faces,
-        // the last nzwall of the face range (zwall_node)
-        const int nfk = sweep_shape(h->shape) ? nf - h->nzwall : nf;
-        if (nfk > 0)
-            h->K->faces<<<(nl * nfk + bt - 1) / bt, bt, 0, h->aux>>>(X, h->bnode, h->bcls, nfk, G, h->P, write_macro);
-        if (ne > 0)
-            h->K->edges<<<(nl * ne + bt - 1) / bt, bt, 0, h->aux2>>>(X, h->bnode + nf, h->bcls + nf, ne, G, h->P,
-                                                                     write_macro);
-    }
+    // with a sweep shape the interior kernel updates the z wall faces, the
+    // last nzwall of the face range (zwall_node)
+    const int nfk = sweep_shape(h->shape) ? nf - h->nzwall : nf;
+    if (nfk > 0)
+        h->K->faces<<<(nl * nfk + bt - 1) / bt, bt, 0, h->aux>>>(X, h->bnode, h->bcls, nfk, G, h->P, write_macro);
+    if (ne > 0)
+        h->K->edges<<<(nl * ne + bt - 1) / bt, bt, 0, h->aux2>>>(X, h->bnode + nf, h->bcls + nf, ne, G, h->P,
+                                                                 write_macro);
     TMX_CK(cudaEventRecord(h->join2, h->aux2));
     if (ev) {  // the boundary time spans both boundary kernels
         TMX_CK(cudaStreamWaitEvent(h->aux, h->join2, 0));
         TMX_CK(cudaEventRecord(ev[3], h->aux));
     }
     TMX_CK(cudaEventRecord(h->join, h->aux));
-    // FP64: the bulk kernel follows the two boundary kernels.  Its blocks and
-    // theirs (about 120 registers each) cannot share an SM, so running them
-    // side by side only stretched the bulk launch (step 204 us side by side,
-    // 202 us in order at W=32).  The reduced-precision boundary kernels (64
-    // registers) do overlap the bulk kernel (FP16 step 75 us side by side,
-    // 85 us in order).
-    // (timed steps, ev given, run the interior kernel after the boundary
-    // kernels in every form, so that each event pair times its kernels alone)
-    if (h->K->serial || ev) {
+    // The boundary kernels (64 registers) run beside the bulk kernel (FP16
+    // step 75 us side by side, 85 us in order); timed steps (ev given) run it
+    // after them, so that each event pair times its kernels alone.
+    if (ev) {
         TMX_CK(cudaStreamWaitEvent(h->stream, h->join, 0));
         TMX_CK(cudaStreamWaitEvent(h->stream, h->join2, 0));
     }
@@ -520,11 +567,19 @@ int enqueue_step(tmx_handle* h, int cur, int write_macro, cudaEvent_t* ev)
     else
         h->K->bulk<<<h->bulk_blocks, 256, 0, h->stream>>>(X, G, h->P, write_macro);
     if (ev) TMX_CK(cudaEventRecord(ev[1], h->stream));
-    if (!h->K->serial && !ev) {
+    if (!ev) {
         TMX_CK(cudaStreamWaitEvent(h->stream, h->join, 0));
         TMX_CK(cudaStreamWaitEvent(h->stream, h->join2, 0));
     }
     TMX_CK(cudaGetLastError());
+    return TMX_OK;
+}
+
+// After the stream has been waited for: whether every step's copies arrived.
+int settled(const tmx_handle* h)
+{
+    if (h->error && *(volatile int*)h->error)
+        return fail(TMX_E_CUDA, "a step of the FP64 form gave up waiting for its copies: the state is not valid");
     return TMX_OK;
 }
 
@@ -732,7 +787,7 @@ int tmx_create(const tmx_case* c, int device, tmx_handle** out)
     // boundary node list, faces first, sorted by class then node index
     std::vector<int> nodes;
     std::vector<unsigned char> cls;
-    rc = boundary_list(G, nodes, cls, h->nface, &h->class_count, h->K->walls ? &h->nwall : nullptr, &h->nzwall);
+    rc = boundary_list(G, nodes, cls, h->nface, &h->class_count, &h->nzwall);
     if (rc) {
         delete h;
         return rc;
@@ -764,6 +819,17 @@ int tmx_create(const tmx_case* c, int device, tmx_handle** out)
     if (e == cudaSuccess && h->nb)
         e = cudaMemcpy(h->bnode, nodes.data(), nodes.size() * sizeof(int), cudaMemcpyHostToDevice);
     if (e == cudaSuccess && h->nb) e = cudaMemcpy(h->bcls, cls.data(), cls.size(), cudaMemcpyHostToDevice);
+    std::vector<int4> runs;
+    if (h->K->run[0]) {
+        h->run_nt = run_threads(G.nnodes);
+        step_runs(G, 0, h->run_nt, runs);
+        h->nruns = (int)runs.size();
+        if (e == cudaSuccess) e = alloc((void**)&h->runs, std::max<size_t>(1, runs.size()) * sizeof(int4));
+        if (e == cudaSuccess) e = alloc((void**)&h->counters, 2 * sizeof(int));
+        if (e == cudaSuccess && !(h->error = error_flag_take())) e = cudaErrorMemoryAllocation;
+        if (e == cudaSuccess && !runs.empty())
+            e = cudaMemcpy(h->runs, runs.data(), runs.size() * sizeof(int4), cudaMemcpyHostToDevice);
+    }
     if (e != cudaSuccess) {
         const int code = (e == cudaErrorMemoryAllocation) ? TMX_E_NOMEM : TMX_E_CUDA;
         free_all(h);
@@ -774,6 +840,16 @@ int tmx_create(const tmx_case* c, int device, tmx_handle** out)
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     h->bulk_blocks = std::max(1, std::min((G.nnodes + 255) / 256, sms * 8));
+    if (h->K->run[0]) {
+        const void* k = (const void*)h->K->run[h->run_nt > 128];
+        const int smem = tmx::run_smem_host(h->run_nt);
+        cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        int per = 1;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, h->run_nt, smem);
+        cudaGetLastError();
+        h->run_slots = sms * std::max(1, per);
+    }
     // the FP16 form's interior as 32 x 4 sweep tiles of 8 planes (the same
     // bits as the flat kernel, faster: W=32 step 61 us against 69 us)
     if (h->K->moments) {
@@ -857,6 +933,8 @@ int tmx_init(tmx_handle* h)
     X.mcur = h->mom[0];
     h->K->init<<<h->bulk_blocks, 256, 0, h->stream>>>(X, h->G, h->P, h->c.rho0);
     TMX_CK(cudaGetLastError());
+    // a step clears the other parity's run counter; the first finds both clear
+    if (h->counters) TMX_CK(cudaMemsetAsync(h->counters, 0, 2 * sizeof(int), h->stream));
     TMX_CK(cudaStreamSynchronize(h->stream));
     h->steps = 0;
     h->inited = true;
@@ -881,7 +959,7 @@ int tmx_sync(tmx_handle* h)
     if (!h) return fail(TMX_E_INVALID, "null handle");
     TMX_CK(cudaSetDevice(h->device));
     TMX_CK(cudaStreamSynchronize(h->stream));
-    return TMX_OK;
+    return settled(h);
 }
 
 long long tmx_steps_done(const tmx_handle* h) { return h ? h->steps : -1; }
@@ -905,6 +983,7 @@ int tmx_checkpoint(tmx_handle* h, void* buf, long long size)
                                                  checkpoint_total(b));
     TMX_CK(cudaSetDevice(h->device));
     TMX_CK(cudaStreamSynchronize(h->stream));
+    if (const int rc = settled(h)) return rc;
     CheckpointHeader hd{};
     std::memcpy(hd.magic, kCheckpointMagic, 8);
     hd.abi = TMX_ABI_VERSION;
@@ -953,6 +1032,10 @@ int tmx_restore(tmx_handle* h, const void* buf, long long size)
         TMX_CK(cudaMemcpy(h->uin_d[0], a.data(), nu * 4, cudaMemcpyHostToDevice));
         TMX_CK(cudaMemcpy(h->uin_d[1], c.data(), nu * 4, cudaMemcpyHostToDevice));
     }
+    if (h->counters) {
+        TMX_CK(cudaMemsetAsync(h->counters, 0, 2 * sizeof(int), h->stream));
+        TMX_CK(cudaStreamSynchronize(h->stream));
+    }
     h->cur = 0;
     h->rcur = 0;
     h->steps = hd.steps;
@@ -977,6 +1060,7 @@ static int box_to_host(tmx_handle* h, int box, const double* dev, double* host_o
     stage.resize(n);
     TMX_CK(cudaMemcpyAsync(stage.data(), dev + G.base[box], n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     TMX_CK(cudaStreamSynchronize(h->stream));
+    if (const int rc = settled(h)) return rc;
     for (int k = 0; k < nz; k++)
         for (int j = 0; j < ny; j++) {
             const double* src = stage.data() + ((size_t)k * ny + j) * nx;
@@ -1064,6 +1148,7 @@ int tmx_mixing(tmx_handle* h, double* rows_out, double* outlet_im)
     std::vector<double> st((size_t)nrow * 9);
     TMX_CK(cudaMemcpyAsync(st.data(), h->stats, st.size() * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     TMX_CK(cudaStreamSynchronize(h->stream));
+    if (const int rc = settled(h)) return rc;
     // running maxima over the rows in the reference's order, starting at 0
     double mx[3] = {0.0, 0.0, 0.0};
     for (int r = 0; r < nrow; r++) {
@@ -1125,6 +1210,7 @@ int tmx_mixing_static(tmx_handle* h, double* rows_out, double* outlet_im)
     TMX_CK(cudaGetLastError());
     TMX_CK(cudaMemcpyAsync(rows_out, rows, (size_t)nrow * 7 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     TMX_CK(cudaStreamSynchronize(h->stream));
+    if (const int rc = settled(h)) return rc;
     if (outlet_im)
         for (int q = 0; q < 3; q++) outlet_im[q] = rows_out[4 + q];
     return TMX_OK;
@@ -1140,6 +1226,7 @@ int tmx_sums(tmx_handle* h, double out[8])
     std::vector<double> p((size_t)kSumBlocks * 6);
     TMX_CK(cudaMemcpyAsync(p.data(), h->partial, p.size() * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     TMX_CK(cudaStreamSynchronize(h->stream));
+    if (const int rc = settled(h)) return rc;
     double s[6] = {0, 0, 0, 0, 0, 0};
     for (int b = 0; b < kSumBlocks; b++)
         for (int m = 0; m < 6; m++) s[m] += p[(size_t)b * 6 + m];
@@ -1178,6 +1265,7 @@ int tmx_pressure_power(tmx_handle* h, double* pressure_rows, double* pressure_x,
     std::vector<double> o((size_t)nout);
     TMX_CK(cudaMemcpyAsync(o.data(), h->diag, o.size() * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     TMX_CK(cudaStreamSynchronize(h->stream));
+    if (const int rc = settled(h)) return rc;
     const double ptop = o[0];
     for (int r = 0; r < nrow; r++) {
         pressure_rows[3 * r] = r + 1;  // mixing rows 1..mny, then inlet row j as j + mny
@@ -1267,7 +1355,7 @@ int tmx_time_steps(tmx_handle* h, int nsteps, double* ms)
     cudaEventDestroy(t1);
     if (rc) return rc;
     *ms = el;
-    return TMX_OK;
+    return settled(h);
 }
 
 int tmx_counts(const tmx_handle* h, long long out[4])

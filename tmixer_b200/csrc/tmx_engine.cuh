@@ -1372,74 +1372,6 @@ __device__ __forceinline__ void closed_pull(const BCtx<PR>& c, int cls, int fld,
         closure_edge(c, cls, fld, v);
 }
 
-// One wall face node (wall_class) in one thread, the four fields in the
-// order of bulk_node: the flow pulled and closed, then the species copied from
-// the interior neighbour's pulls (A and B summed first for the reaction term,
-// then pulled again to collide, then C).  The arithmetic is boundary_lane's:
-// the same sums, moments, outlet density, polynomial and collision.  One loop
-// over the six passes keeps a single copy of the pull and collision code.
-template <class PR>
-__device__ __forceinline__ void wall_node(const StepPtrs& X, const Geom& G, const Phys& P, int write_macro, int g,
-                                          int b, int i, int j, int k, int cls)
-{
-    using T = typename PR::T;
-    const typename PR::S* __restrict__ Pin = (const typename PR::S*)X.pin;
-    typename PR::S* __restrict__ Pout = (typename PR::S*)X.pout;
-    const long long ps = G.ps;
-    int di, dj, dk;
-    face_copy_offset(cls, di, dj, dk);
-    T poly[19];
-    T rho = T(0), ux = T(0), uy = T(0), uz = T(0), ca = T(0), cb = T(0), cc = T(0), rt = T(0);
-#pragma unroll 1
-    for (int s = 0; s < 6; s++) {
-        const int fld = s == 0 ? 0 : (s < 3 ? s : (s < 5 ? s - 2 : 3));  // flow, A, B, A, B, C
-        const int o = fld ? 1 : 0;
-        T v[19];
-#pragma unroll
-        for (int q = 0; q < 19; q++) {
-            const int src = pull_src(G, b, i + o * di, j + o * dj, k + o * dk, q);
-            v[q] = src >= 0 ? PR::decode(Pin + PR::off(fld, q, ps, src), fld, q, nullptr, ps, src) : T(0);
-        }
-        if (s == 0) wall_flow_closure(cls, T(P.rho_out), v);
-        T r = sum19(v);
-        if (s == 0) {
-            // the outlet row's density is pinned to rho_out (Tmixer.cpp:9575-9582)
-            if (b == 1 && j == 1) r = T(P.rho_out);
-            T sxm, sym, szm;
-            momentum(v, sxm, sym, szm);
-            ux = sxm / r;
-            uy = sym / r;
-            uz = szm / r;
-            PR::poly(ux, uy, uz, poly);
-            rho = r;
-        } else if (s == 1) {
-            ca = r;
-            continue;
-        } else if (s == 2) {
-            cb = r;
-            rt = T(P.rateconst) * ca * cb;
-            continue;
-        }
-        if (s == 5) cc = r;
-        collide_store<PR>(Pout, ps, g, fld, v, s == 3 ? ca : (s == 4 ? cb : r), poly, P, rt);
-    }
-    T* __restrict__ Rcur = (T*)X.rcur;
-    Rcur[g] = rho;
-    Rcur[ps + g] = ca;
-    Rcur[2 * ps + g] = cb;
-    Rcur[3 * ps + g] = cc;
-    if (write_macro) {
-        double* Mac = X.mac;
-        Mac[g] = rho;
-        Mac[ps + g] = ux;
-        Mac[2 * ps + g] = uy;
-        Mac[3 * ps + g] = uz;
-        Mac[4 * ps + g] = ca;
-        Mac[5 * ps + g] = cb;
-        Mac[6 * ps + g] = cc;
-    }
-}
-
 // ---------------------------------------------------------------------------
 // boundary nodes of a compact, class-sorted list, four threads per node: lane
 // fld (0 flow, 1 A, 2 B, 3 C) pulls, closes and collides its own field.  Every
@@ -1714,12 +1646,14 @@ __device__ __forceinline__ void bulk_any(const StepPtrs& X, const Geom& G, const
 }
 
 // Kernel definitions for one precision policy; NAME is the kernel-name suffix.
-#define TMX_DEFINE_STEP_KERNELS(PR, NAME)                                                                         \
+#define TMX_DEFINE_INIT_KERNEL(PR, NAME)                                                                          \
     __global__ void k_init_##NAME(StepPtrs X, Geom G, Phys P, double rho0)                                      \
     {                                                                                                           \
         for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < G.nnodes; g += gridDim.x * blockDim.x)          \
             init_node<PR>(X, G, P, rho0, g);                                                                    \
-    }                                                                                                           \
+    }
+#define TMX_DEFINE_STEP_KERNELS(PR, NAME)                                                                         \
+    TMX_DEFINE_INIT_KERNEL(PR, NAME)                                                                            \
     __global__ void __launch_bounds__(256, 2) k_bulk_##NAME(StepPtrs X, Geom G, Phys P, int write_macro)        \
     {                                                                                                           \
         for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < G.nnodes; g += gridDim.x * blockDim.x)          \
@@ -1787,7 +1721,7 @@ __device__ __forceinline__ void load_desc(StepDesc& dst, const MixerDesc* __rest
     TMX_SWEEP_KERNEL(PR, NAME, 4, 4)
 
 // The face and the edge list as two launches (the FP32 and FP16-storage steps;
-// the FP64 step uses k_bound and k_walls).
+// the FP64 step is k_run_f64).
 #define TMX_DEFINE_BOUNDARY_KERNELS(PR, NAME)                                                                     \
     __global__ void __launch_bounds__(kBoundaryThreads) k_bfaces_##NAME(                                       \
         StepPtrs X, const int* bnode, const unsigned char* bcls, int nb, Geom G, Phys P, int write_macro)       \
@@ -1801,34 +1735,6 @@ __device__ __forceinline__ void load_desc(StepDesc& dst, const MixerDesc* __rest
         __shared__ PR::T buf[PR::kOnePass ? kBoundaryThreads / 4 : 1][76];                                      \
         boundary_node<PR, false>(X, bnode, bcls, nb, G, P, write_macro, buf, blockIdx.x);                       \
     }
-
-// Faces and edges in one launch, the first eblocks blocks on the edge and
-// corner list (bnode + nf), the rest on the face list (the FP64 step, whose
-// bulk kernel follows the boundary).
-#define TMX_DEFINE_BOUND_KERNEL(PR, NAME)                                                                         \
-    __global__ void __launch_bounds__(kBoundaryThreads) k_bound_##NAME(StepPtrs X, const int* bnode,           \
-        const unsigned char* bcls, int nf, int ne, int eblocks, Geom G, Phys P, int write_macro)                 \
-    {                                                                                                           \
-        __shared__ PR::T buf[PR::kOnePass ? kBoundaryThreads / 4 : 1][76];                                      \
-        if ((int)blockIdx.x < eblocks)                                                                          \
-            boundary_node<PR, false>(X, bnode + nf, bcls + nf, ne, G, P, write_macro, buf, blockIdx.x);         \
-        else                                                                                                    \
-            boundary_node<PR, true>(X, bnode, bcls, nf, G, P, write_macro, buf, blockIdx.x - eblocks);          \
-    }
-
-// The wall faces (wall_class), one thread per node of a node-sorted list.
-#define TMX_DEFINE_WALL_KERNEL(PR, NAME)                                                                          \
-    __global__ void __launch_bounds__(kBoundaryThreads) k_walls_##NAME(StepPtrs X, const int* wnode,           \
-        const unsigned char* wcls, int nw, Geom G, Phys P, int write_macro)                                     \
-    {                                                                                                           \
-        const int t = blockIdx.x * blockDim.x + threadIdx.x;                                                    \
-        if (t >= nw) return;                                                                                    \
-        const int g = wnode[t];                                                                                 \
-        int b, i, j, k;                                                                                         \
-        decode(G, g, b, i, j, k);                                                                               \
-        wall_node<PR>(X, G, P, write_macro, g, b, i, j, k, wcls[t]);                                            \
-    }
-
 
 // Batched kernels for one precision policy (declared in tmx_kernels.cuh).
 #define TMX_BULK_BATCH(PR, NAME, NT)                                                                              \

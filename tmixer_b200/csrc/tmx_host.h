@@ -6,6 +6,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <vector>
 
 #include "../../include/tmx.h"
@@ -36,10 +37,9 @@ struct StepKernels {
     // the face and edge lists as two launches (forms whose bulk runs beside them)
     void (*faces)(tmx::StepPtrs, const int*, const unsigned char*, int, Geom, Phys, int);
     void (*edges)(tmx::StepPtrs, const int*, const unsigned char*, int, Geom, Phys, int);
-    // faces and edges in one launch (serial forms only)
-    void (*bound)(tmx::StepPtrs, const int*, const unsigned char*, int, int, int, Geom, Phys, int);
-    // the wall faces, one thread per node (null: the face kernel takes them)
-    void (*walls)(tmx::StepPtrs, const int*, const unsigned char*, int, Geom, Phys, int);
+    // the whole step in one launch, by runs of up to 128 or 256 nodes (FP64; the
+    // pointers above are null)
+    void (*run[2])(tmx::StepPtrs, Geom, Phys, int, const int4*, int, const int*, const unsigned char*, int, int*, int, int*);
     int sbytes, tbytes;
     bool moments;  // the form stores per-node FP32 moments next to the populations
     bool serial;   // the bulk kernel runs after the boundary kernels, not beside them
@@ -58,16 +58,14 @@ long long boundary_count(const Geom& G);
 // Class of a boundary node (tmx_classes.h), -1 for a node no case covers.
 int classify(const Geom& G, int b, int i, int j, int k);
 // Boundary nodes sorted faces first, then by class, then by node index; the
-// first nface entries are face classes.  With nwall the wall faces
-// (tmx::wall_class) come last, in node order, and *nwall counts them.
-// Without nwall and with nzwall (the FP32 and FP16 forms), the z wall faces
+// first nface entries are face classes.  With nzwall the z wall faces
 // (K_FACE_Z1, K_FACE_ZT) come last among the faces and *nzwall counts them:
 // each lies above or below an interior node and each interior node of planes
 // 2 and nz - 1 has one (checked; an internal error otherwise), and the sweep
 // kernels update them (zwall_node).  Without interior nodes (nz < 3) they
 // stay in place and *nzwall is 0.  Returns TMX_OK or a failure code.
 int boundary_list(const Geom& G, std::vector<int>& nodes, std::vector<unsigned char>& cls, int& nface,
-                  std::vector<int>* class_count, int* nwall, int* nzwall);
+                  std::vector<int>* class_count, int* nzwall);
 // Inlet profiles Uin1, Uin2 ((iny+3) x (nz+3)) as the reference computes them:
 // the duct series (which depends on iny and nz only) and its mean, then the
 // scaling to umean and the shifts.
@@ -131,6 +129,61 @@ inline void sweep_tiles(const Geom& G, int mixer, int ty, int zchunk, std::vecto
                     out.push_back(make_int4(mixer * 2 + b, x0 | (y0 << 16), z0 | (z1 << 16), 0));
     }
 }
+
+// Threads per block, and so nodes per run, of the FP64 step: 256, whose 2 KB
+// copies get the most from DRAM, or 128 where the finer runs fill the SMs more
+// evenly (step by 128 / 256: 65,536 nodes 23.7 / 30.5 us, 524,288 nodes 116.4 /
+// 118.4 us, 1.8M nodes 358.7 / 357.7 us, 4.9M nodes 969 / 956 us).
+inline int run_threads(long long nodes)
+{
+    return nodes < 2000000 ? 128 : 256;
+}
+// Runs of the FP64 step (tmx_kernels.cuh) for one mixer, of up to nt nodes:
+// every node but the edges and corners, plane by plane; the long runs first,
+// then the short ones (which even out the end of the launch).
+inline void step_runs(const Geom& G, int mixer, int nt, std::vector<int4>& out)
+{
+    std::vector<int4> rest;
+    for (int k = 1; k <= G.nz; k++)
+        for (int b = 0; b < 2; b++) {
+            // columns i0..i1 of row j0 through row j1 (whole rows between)
+            auto add = [&](int kind, int iface, int i0, int j0, int i1, int j1) {
+                if (j1 < j0 || (j1 == j0 && i1 < i0)) return;
+                int g = tmx::node_index(G, b, i0, j0, k), i = i0;
+                const int end = tmx::node_index(G, b, i1, j1, k) + 1;
+                while (g < end) {
+                    // (ends at multiples of 32 nodes: whole 256-byte stores)
+                    const int n = std::min(end - g, nt - g % 32);
+                    (n > nt / 2 ? out : rest)
+                        .push_back(make_int4(g, n | kind << 9 | b << 12 | iface << 13 | mixer << 15, i, k));
+                    g += n;
+                    i = (i - 1 + n) % G.nx[b] + 1;
+                }
+            };
+            const bool wall = k == 1 || k == G.nz;
+            const int rows = k == 1 ? tmx::kRunZ1 : (k == G.nz ? tmx::kRunZT : tmx::kRunRows);
+            const int nx = G.nx[b], ny = G.ny[b];
+            if (b == 0) {
+                add(rows, 0, 1, 2, nx, ny - 1);
+                add(rows, 1, G.ia + 1, 1, G.ib - 1, 1);
+                if (!wall) {
+                    add(tmx::kRunYT, 0, 2, ny, nx - 1, ny);
+                    add(tmx::kRunY1, 0, 2, 1, G.ia - 1, 1);
+                    add(tmx::kRunY1, 0, G.ib + 1, 1, nx - 1, 1);
+                }
+            } else {
+                add(rows, 0, 1, 2, nx, ny - 1);
+                add(rows, 2, 1, ny, nx, ny);
+                if (!wall) add(tmx::kRunY1, 0, 2, 1, nx - 1, 1);
+            }
+        }
+    out.insert(out.end(), rest.begin(), rest.end());
+}
+
+// An int that kernels set when they give up (mapped host memory, 0 to begin
+// with), and its return; null when there is no memory.
+int* error_flag_take();
+void error_flag_give(int* flag);
 
 // Checkpoint layout (tmx_checkpoint, tmx_batch_checkpoint): this header, then
 // the sections in the order of `bytes`: the population buffer the next step

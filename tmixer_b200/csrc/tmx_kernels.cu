@@ -5,12 +5,48 @@
 // operations are the explicit __fma_rn of the correctly rounded constant
 // divisions (tmx_device.cuh).  The step itself is in tmx_engine.cuh.
 #include "tmx_engine.cuh"
+#include "tmx_run64.cuh"
 
 namespace tmx {
 
-TMX_DEFINE_STEP_KERNELS(F64, f64)
-TMX_DEFINE_BOUND_KERNEL(F64, f64)
-TMX_DEFINE_WALL_KERNEL(F64, f64)
+TMX_DEFINE_INIT_KERNEL(F64, f64)
+
+// The FP64 step (tmx_run64.cuh): the first blocks begin with the edge and
+// corner nodes (eight to a warp), all of them go through the runs.
+template <int NT>
+__device__ __forceinline__ void run_step(const StepPtrs& X, const Geom& G, const Phys& P, int write_macro,
+                                         const int4* __restrict__ runs, int nruns, const int* __restrict__ enode,
+                                         const unsigned char* __restrict__ ecls, int ne, int* __restrict__ counters,
+                                         int parity, int* error, RunShared<NT>& S)
+{
+    constexpr int kPer = NT / kBoundaryLanes;
+    if (blockIdx.x == 0 && threadIdx.x == 0) counters[1 - parity] = 0;  // the next step's
+    const int eb = (ne + kPer - 1) / kPer;
+    for (int u = blockIdx.x; u < eb; u += gridDim.x)
+        run_edges(X, G, P, write_macro, [&](int e, int& node, int& cls) {
+            const int at = u * kPer + (threadIdx.x >> 5) * 8 + e;
+            if (at < ne) {
+                node = enode[at];
+                cls = ecls[at];
+            }
+        });
+    // the blocks without edges begin with the first runs
+    const int nb = gridDim.x;
+    run_loop<NT>([&](const int4&) { return run_view(X, G, P); }, runs, nruns, (int)(blockIdx.x + nb - eb % nb) % nb, nb,
+                 counters + parity, write_macro, S, error);
+}
+#define TMX_DEFINE_RUN(NT)                                                                                      \
+    __global__ void __launch_bounds__(NT, 512 / NT) k_run##NT##_f64(                                            \
+        const __grid_constant__ StepPtrs X, const __grid_constant__ Geom G, const __grid_constant__ Phys P,     \
+        int write_macro, const int4* __restrict__ runs, int nruns, const int* __restrict__ enode,               \
+        const unsigned char* __restrict__ ecls, int ne, int* __restrict__ counters, int parity, int* error)     \
+    {                                                                                                           \
+        extern __shared__ __align__(16) unsigned char run_smem[];                                               \
+        run_step<NT>(X, G, P, write_macro, runs, nruns, enode, ecls, ne, counters, parity, error,               \
+                     *(RunShared<NT>*)run_smem);                                                                \
+    }
+TMX_DEFINE_RUN(128)
+TMX_DEFINE_RUN(256)
 TMX_DEFINE_BATCH_KERNELS(F64, f64)
 
 // ---------------------------------------------------------------------------

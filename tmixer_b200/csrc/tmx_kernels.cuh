@@ -28,8 +28,9 @@ constexpr int kBoundaryLanesHost = 4;      // threads per boundary node (one per
 // time; the batch pads each mixer's part of a list to a multiple of it.
 constexpr int kListAlign = kBoundaryThreadsHost / kBoundaryLanesHost;
 
+#define TMX_DECLARE_INIT_KERNEL(NAME) __global__ void k_init_##NAME(StepPtrs X, Geom G, Phys P, double rho0);
 #define TMX_DECLARE_STEP_KERNELS(NAME)                                                                          \
-    __global__ void k_init_##NAME(StepPtrs X, Geom G, Phys P, double rho0);                                     \
+    TMX_DECLARE_INIT_KERNEL(NAME)                                                                               \
     __global__ void k_bulk_##NAME(StepPtrs X, Geom G, Phys P, int write_macro);
 #define TMX_DECLARE_BOUNDARY_KERNELS(NAME)                                                                      \
     __global__ void k_bfaces_##NAME(StepPtrs X, const int* bnode, const unsigned char* bcls, int nb, Geom G,    \
@@ -37,15 +38,28 @@ constexpr int kListAlign = kBoundaryThreadsHost / kBoundaryLanesHost;
     __global__ void k_bedges_##NAME(StepPtrs X, const int* bnode, const unsigned char* bcls, int nb, Geom G,    \
                                     Phys P, int write_macro);
 
-TMX_DECLARE_STEP_KERNELS(f64)
+TMX_DECLARE_INIT_KERNEL(f64)
 TMX_DECLARE_STEP_KERNELS(f32)
 TMX_DECLARE_STEP_KERNELS(f16)
 TMX_DECLARE_BOUNDARY_KERNELS(f32)
 TMX_DECLARE_BOUNDARY_KERNELS(f16)
-__global__ void k_bound_f64(StepPtrs X, const int* bnode, const unsigned char* bcls, int nf, int ne, int eblocks,
-                            Geom G, Phys P, int write_macro);
-__global__ void k_walls_f64(StepPtrs X, const int* wnode, const unsigned char* wcls, int nw, Geom G, Phys P,
-                            int write_macro);
+
+// Runs of the FP64 step (tmx_run64.cuh): {first node, nodes | kind << 9 |
+// box << 12 | iface << 13 | mixer << 15, x of the first node, z}, up to
+// NT consecutive nodes of one plane of a box, NT the kernel's threads (128 or
+// 256; run_threads in tmx_host.h).  iface: the row whose ey = 1 (1) or ey = -1
+// (2) sources lie in the other box.
+enum RunKind { kRunRows = 0, kRunZ1, kRunZT, kRunYT, kRunY1 };
+constexpr int run_smem_host(int nt) { return 2 * 19 * (nt + 4) * 8 + 64; }  // RunShared
+// Edge and corner nodes enode[0..ne), then the runs; counters[parity] hands
+// out the runs, counters[1 - parity] is cleared for the next step.
+#define TMX_DECLARE_RUN(NT)                                                                                     \
+    __global__ void k_run##NT##_f64(const __grid_constant__ StepPtrs X, const __grid_constant__ Geom G,         \
+                                    const __grid_constant__ Phys P, int write_macro, const int4* runs,          \
+                                    int nruns, const int* enode, const unsigned char* ecls, int ne,             \
+                                    int* counters, int parity, int* error);
+TMX_DECLARE_RUN(128)
+TMX_DECLARE_RUN(256)
 
 // One mixer of a batch: its buffers for either parity of the batch's step
 // counter, its geometry and its physics constants (device memory, read by

@@ -1,0 +1,491 @@
+// tmx_run64.cuh -- the step of the plain FP64 form: one kernel over every node
+// but the edges and corners, fed through shared memory (device code; the
+// kernels that instantiate it are in tmx_kernels.cu).
+//
+// A block of NT threads takes one run at a time: up to NT consecutive nodes
+// of one plane, all interior rows (whose ends are the inlets or the mixing
+// box's x walls), or a row of the y walls, the outlet or a z wall (step_runs
+// in tmx_host.h).  A run's sources of one direction are consecutive too, so
+// they come as one bulk copy of 8 NT bytes, 19 to a field, and the wall faces
+// cost what an interior node does: their closure, and another node to copy the
+// species from.
+//
+// Two slots of 19 x (NT + 4) values hold one field each.  A field is read into
+// registers and its slot filled again at once (by the last warp to read it),
+// so that two fields are in flight while one is collided, past the end of the
+// run into the next one.  B, whose sum the collision of A needs, is summed
+// before and read when A is done.
+//
+// What bounds it: DRAM.  Moving these bytes in this way without arithmetic
+// (bulk copies of 256 nodes, two slots, two blocks per SM, plain stores) runs
+// at 5.9 to 6.3 TB/s; the same bytes by 8-byte cp.async in runs of 32 nodes at
+// 4.7 TB/s, whatever the number in flight.
+#pragma once
+#include "tmx_engine.cuh"
+
+namespace tmx {
+
+__device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void mbar_init(unsigned bar, int count)
+{
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_expect(unsigned bar, unsigned bytes)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+// Wait for a phase of a barrier; false if it does not come within some
+// seconds (the caller gives up and reports it).
+__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity)
+{
+    for (int i = 0; i < (1 << 22); i++) {
+        unsigned done;
+        asm volatile(
+            "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+            : "=r"(done)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (done) return true;
+    }
+    return false;
+}
+__device__ __forceinline__ void bulk_load(unsigned dst, const void* src, unsigned bytes, unsigned bar)
+{
+    asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(bar)
+                 : "memory");
+}
+
+// What the step reads and writes of one mixer.
+struct RunView {
+    const double* pin;
+    double *pout, *rcur, *mac;
+    const double *uin1, *uin2;
+    const Geom* G;
+    const Phys* P;
+};
+__device__ __forceinline__ RunView run_view(const StepPtrs& X, const Geom& G, const Phys& P)
+{
+    return RunView{(const double*)X.pin, (double*)X.pout, (double*)X.rcur, X.mac, (const double*)X.uin1,
+                   (const double*)X.uin2, &G, &P};
+}
+
+// A run, the same for the whole block: its first node, nodes, kind and box, and
+// the strides of its sources.  Direction q of node h (the node itself for the
+// flow, node + shift for the species) comes from h - ex - ez * sz, for ey = 1
+// from h + op - ex - ez * szp, for ey = -1 from h + om - ex - ez * szm: the own
+// box's strides, or on the two rows that meet at the opening the other box's
+// (bulk_src).
+struct Run {
+    int g0, n, kind, b, i0, nx;
+    int shift, op, om, ops, oms, sz, szp, szm;
+};
+__host__ __device__ inline int run_mixer(const int4& t) { return t.y >> 15; }
+__host__ __device__ inline Run run_of(const Geom& G, const int4& t)
+{
+    Run R;
+    R.g0 = t.x;
+    R.n = t.y & 511;
+    R.kind = (t.y >> 9) & 7;
+    R.b = (t.y >> 12) & 1;
+    const int iface = (t.y >> 13) & 3, k0 = t.w - 1;
+    R.i0 = t.z;
+    R.nx = box_nx(G, R.b);
+    R.sz = R.szp = R.szm = R.nx * box_ny(G, R.b);
+    R.op = -R.nx;
+    R.om = R.nx;
+    if (iface == 1) {
+        R.szp = G.mnx * G.mny;
+        R.op = G.base[1] + (k0 * G.mny + G.mny - 1) * G.mnx + 1 - G.ia - k0 * R.sz;
+    } else if (iface == 2) {
+        R.szm = G.inx * G.iny;
+        R.om = k0 * R.szm + G.ia - 1 - G.base[1] - (k0 * G.mny + G.mny - 1) * G.mnx;
+    }
+    const int dk = R.kind == kRunZ1 ? 1 : (R.kind == kRunZT ? -1 : 0);
+    R.shift = dk ? dk * R.sz : (R.kind == kRunYT ? -R.nx : (R.kind == kRunY1 ? R.nx : 0));
+    R.ops = R.op + dk * (R.szp - R.sz);
+    R.oms = R.om + dk * (R.szm - R.sz);
+    return R;
+}
+// A thread's node of a run: active, x, face class (-1: interior, -2: interior
+// beside a junction edge) and the x shift to the species' source node.
+struct RunNode {
+    bool act;
+    int cls, xs;
+};
+__host__ __device__ inline RunNode run_node(const Geom& G, const Run& R, int t)
+{
+    RunNode N;
+    N.act = t < R.n;
+    N.cls = -1;
+    N.xs = 0;
+    const int i = (R.i0 - 1 + t) % R.nx + 1;  // the run may pass the end of a row
+    const bool lo = i == 1, hi = i == R.nx;
+    if (R.kind == kRunRows) {
+        if (lo | hi) {
+            N.cls = R.b ? (lo ? K_FACE_MX1 : K_FACE_MXT) : (lo ? K_INLET1 : K_INLET2);
+            if (R.b) N.xs = lo ? 1 : -1;
+        } else if (!R.b && (i == G.ia || i == G.ib) && (R.g0 + t) / R.nx % G.iny == 1) {
+            N.cls = -2;
+        }
+    } else if (R.kind == kRunZ1 || R.kind == kRunZT) {
+        N.act = N.act && !lo && !hi;  // the ends of the rows are edges
+        N.cls = R.kind == kRunZ1 ? K_FACE_Z1 : K_FACE_ZT;
+    } else {
+        N.cls = R.kind == kRunYT ? K_FACE_YT : (R.b ? K_OUTLET : K_FACE_Y1);
+    }
+    return N;
+}
+// The offset of direction (ex, ey, ez)'s source of a field from the node.
+__host__ __device__ inline int run_offset(const Run& R, int fld, int ex, int ey, int ez)
+{
+    const int o = ey > 0 ? (fld ? R.ops : R.op) : (ey < 0 ? (fld ? R.oms : R.om) : 0);
+    return (fld ? R.shift : 0) + o - ex - ez * (ey > 0 ? R.szp : (ey < 0 ? R.szm : R.sz));
+}
+// Whether a field's direction has sources at all (the flow of a wall row has
+// none from beyond the wall; the closure sets those).
+__host__ __device__ inline bool run_pulls(const Run& R, int fld, int ey, int ez)
+{
+    if (fld) return true;
+    return !((R.kind == kRunZ1 && ez > 0) || (R.kind == kRunZT && ez < 0) || (R.kind == kRunYT && ey < 0) ||
+             (R.kind == kRunY1 && ey > 0));
+}
+// The window of a direction in its plane (first value and number, both even: a
+// bulk copy starts and ends at 16 bytes): the run's sources and one more at
+// either end, for the x walls' neighbours.  Plane p of the 76; the last values
+// stop at the end of the buffer.
+__host__ __device__ inline void run_window(const Run& R, int off, int p, long long ps, int& first, int& count)
+{
+    first = (R.g0 + off - 1) & ~1;
+    count = (R.n + 5) & ~1;
+    const long long left = (76 - p) * ps - first;
+    if (count > left) count = (int)left;
+}
+
+// Shared memory of a block of NT threads: the two slots (rows of a window of up
+// to NT + 4 values), the next runs, the barriers.
+template <int NT>
+struct __align__(16) RunShared {
+    static constexpr int kRow = NT + 4;
+    double slot[2][19 * kRow];
+    int4 run[2];  // by the run's ordinal in the block; n = 0: none
+    unsigned long long full[2];
+    int done[2];  // warps that have read a slot
+};
+static_assert(sizeof(RunShared<128>) == run_smem_host(128) && sizeof(RunShared<256>) == run_smem_host(256),
+              "host copy of the size");
+
+// The same value from every lane, so that the compiler knows that a warp
+// shares it (and keeps what follows from it in uniform registers).
+__device__ __forceinline__ int4 run_shared(const int4& t)
+{
+    return make_int4(__shfl_sync(0xffffffffu, t.x, 0), __shfl_sync(0xffffffffu, t.y, 0),
+                     __shfl_sync(0xffffffffu, t.z, 0), __shfl_sync(0xffffffffu, t.w, 0));
+}
+
+// Fill a slot with field fld of run t (one warp; lane q copies direction q).
+template <int NT>
+__device__ __forceinline__ void run_fill(RunShared<NT>& S, int slot, const RunView& M, const Run& R, int fld)
+{
+    const int q = threadIdx.x & 31;
+    const unsigned bar = smem_addr(&S.full[slot]);
+    int ex = 0, ey = 0, ez = 0;
+#pragma unroll
+    for (int d = 0; d < 19; d++)
+        if (q == d) {
+            ex = EX(d);
+            ey = EY(d);
+            ez = EZ(d);
+        }
+    const bool mine = q < 19 && run_pulls(R, fld, ey, ez);
+    const long long ps = M.G->ps;
+    const int p = fld * 19 + q;
+    int first = 0, count = 0;
+    if (mine) run_window(R, run_offset(R, fld, ex, ey, ez), p, ps, first, count);
+    const unsigned bytes = __reduce_add_sync(0xffffffffu, (unsigned)count) * 8u;
+    if (q == 0) mbar_expect(bar, bytes);
+    __syncwarp();
+    if (mine)
+        bulk_load(smem_addr(&S.slot[slot][q * (NT + 4)]), M.pin + p * ps + first, (unsigned)count * 8u, bar);
+}
+
+// Where a thread's values of a field lie: in row q of the slot one or two
+// beyond the thread's number, by the parity of the source that the window
+// begins with.  The parity of the ten kinds of direction (ey, ex != 0,
+// ez != 0), as bits; kRunEven: rows and planes of even length, where only the
+// x component counts.
+__host__ __device__ constexpr int run_bit(int q) { return (EY(q) + 1) * 4 + (EX(q) != 0) * 2 + (EZ(q) != 0); }
+constexpr unsigned kRunEven = 0x333;
+__host__ __device__ inline unsigned run_parities(const Run& R, int fld)
+{
+    unsigned m = 0;
+    for (int ey = -1; ey <= 1; ey++)
+        for (int x = 0; x < 2; x++)
+            for (int z = 0; z < 2; z++)
+                m |= ((unsigned)(R.g0 + run_offset(R, fld, x, ey, z) - 1) & 1u) << ((ey + 1) * 4 + x * 2 + z);
+    return m;
+}
+template <int NT>
+__device__ __forceinline__ void run_read(const double* __restrict__ row, unsigned par, double (&v)[19])
+{
+    if (par == kRunEven) {
+#pragma unroll
+        for (int q = 0; q < 19; q++) v[q] = row[q * (NT + 4) + (EX(q) == 0 ? 2 : 1)];
+    } else {
+#pragma unroll
+        for (int q = 0; q < 19; q++) v[q] = row[q * (NT + 4) + 1 + ((par >> run_bit(q)) & 1)];
+    }
+}
+template <int NT>
+__device__ __forceinline__ double run_sum(const double* __restrict__ row, unsigned par)
+{
+    double s = 0.0;
+    if (par == kRunEven) {
+#pragma unroll
+        for (int q = 0; q < 19; q++) {
+            const double x = row[q * (NT + 4) + (EX(q) == 0 ? 2 : 1)];
+            s = q ? s + x : x;
+        }
+    } else {
+#pragma unroll
+        for (int q = 0; q < 19; q++) {
+            const double x = row[q * (NT + 4) + 1 + ((par >> run_bit(q)) & 1)];
+            s = q ? s + x : x;
+        }
+    }
+    return s;
+}
+
+// The populations that an inlet node's closure sets, of a species in its slot
+// (closure_face).
+template <int NT>
+__device__ __forceinline__ void run_inlet_species(double* row, unsigned par, int cls, double cin)
+{
+    const double w1 = 2.0 / 18.0 * cin, w2 = 2.0 / 36.0 * cin;
+    auto at = [&](int q) -> double& { return row[q * (NT + 4) + 1 + ((par >> run_bit(q)) & 1)]; };
+    const bool one = cls == K_INLET1;
+    constexpr int in[5] = {1, 7, 10, 11, 14}, out[5] = {3, 9, 8, 13, 12};  // opposite pairs
+#pragma unroll
+    for (int e = 0; e < 5; e++) {
+        const double w = e ? w2 : w1;
+        if (one) at(in[e]) = -at(out[e]) + w;
+        else at(out[e]) = -at(in[e]) + w;
+    }
+}
+
+// Collide and store one field of a node: f * c1 + c2 * feq plus the
+// reaction's w_q * rt * m (collide_store's operations; m is -1 for A and B and
+// 2 for C, products that do not round; the flow adds -0.0, which changes no
+// value).
+__device__ __forceinline__ void run_collide(double* __restrict__ p, long long ps, const double (&v)[19], double r,
+                                            const double (&poly)[19], double c1, double c2, double w0, double w1,
+                                            double w2)
+{
+#pragma unroll
+    for (int q = 0; q < 19; q++) {
+        const double o = v[q] * c1 + c2 * feq_div(r * poly[q], q);
+        *p = o + (q == 0 ? w0 : (q <= 6 ? w1 : w2));
+        p += ps;
+    }
+}
+// The same for a density so small that the equilibrium needs the IEEE division
+// (rare): a loop over local memory.
+__device__ __forceinline__ void run_collide_exact(double* __restrict__ p, long long ps, const double (&v)[19], double r,
+                                                  const double (&poly)[19], double c1, double c2, double w0, double w1,
+                                                  double w2)
+{
+    double pl[19], vl[19];
+#pragma unroll
+    for (int q = 0; q < 19; q++) {
+        pl[q] = poly[q];
+        vl[q] = v[q];
+    }
+#pragma unroll 1
+    for (int q = 0; q < 19; q++) {
+        const double o = vl[q] * c1 + c2 * __ddiv_rn(r * pl[q], q == 0 ? 3.0 : (q <= 6 ? 18.0 : 36.0));
+        *p = o + (q == 0 ? w0 : (q <= 6 ? w1 : w2));
+        p += ps;
+    }
+}
+
+// Up to eight edge and corner nodes, four lanes each; at(e, node, cls) gives
+// entry e of the warp's share (node -1: none).
+template <class At>
+__device__ __forceinline__ void run_edges(const StepPtrs& X, const Geom& G, const Phys& P, int write_macro, const At& at)
+{
+    const int lane = threadIdx.x & 31;
+    int node = -1, cls = 0;
+    at(lane >> 2, node, cls);
+    const unsigned mask = __ballot_sync(0xffffffffu, node >= 0);
+    if (node >= 0) boundary_lane<F64, false>(X, G, P, write_macro, node, cls, lane & 3, mask, lane & ~3);
+}
+
+// The runs of one block: the first by its number, then by the launch's counter
+// (dynamic: the blocks that begin with edges take fewer).  get(t) gives the
+// buffers, geometry and constants of run t's mixer.  error: set when a copy
+// does not arrive.
+template <int NT, class Get>
+__device__ __forceinline__ void run_loop(const Get& get, const int4* __restrict__ runs, int nruns, int first,
+                                         int nblocks, int* __restrict__ counter, int write_macro, RunShared<NT>& S,
+                                         int* error)
+{
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    constexpr int kWarps = NT / 32;
+    if (first >= nruns) return;  // (the whole block)
+    if (t == 0) {
+        for (int s = 0; s < 2; s++) {
+            mbar_init(smem_addr(&S.full[s]), 1);
+            S.done[s] = 0;
+        }
+        S.run[0] = runs[first];
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    if (warp == 0) {
+        const int4 r = S.run[0];
+        const RunView M = get(r);
+        const Run R = run_of(*M.G, r);
+        run_fill(S, 0, M, R, 0);
+        run_fill(S, 1, M, R, 1);
+    }
+    for (int ord = 0;; ord ^= 1) {
+        // (each barrier goes through two phases a run: the parities repeat)
+        if (!mbar_wait(smem_addr(&S.full[0]), 0)) {
+            *error = 1;
+            return;
+        }
+        const int4 tr = S.run[ord];
+        if ((tr.y & 511) == 0) return;
+        const RunView M = get(tr);
+        const Phys& P = *M.P;
+        const long long ps = M.G->ps;
+        const int g = tr.x + t;
+        RunNode N;
+        unsigned par, parc;
+        {
+            const Run R = run_of(*M.G, tr);
+            N = run_node(*M.G, R, t);
+            par = run_parities(R, 0);
+            parc = run_parities(R, 1);
+        }
+        const bool inlet = N.cls == K_INLET1 || N.cls == K_INLET2;
+        double* __restrict__ p = M.pout + g;
+        // the next run: its index now, its entry after the flow, there for
+        // all before the block has read B
+        int next = 0;
+        if (t == NT - 1) next = nblocks + atomicAdd(counter, 1);
+
+        double poly[19], v[19];
+        double r = 0.0, cb = 0.0, m = -0.0, rt = 0.0;
+#pragma unroll 1
+        for (int f = 0; f < 4; f++) {
+            const int s = f & 1;
+            if (s && !mbar_wait(smem_addr(&S.full[1]), f >> 1)) {
+                *error = 1;
+                return;
+            }
+            run_read<NT>(&S.slot[s][t + (f ? N.xs : 0)], par, v);
+            // the slot is free once every warp has read it; the last fills it
+            // with the field after the next
+            __syncwarp();
+            int last = 0;
+            if (lane == 0) {
+                asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], 1;"
+                             : "=r"(last)
+                             : "r"(smem_addr(&S.done[s]))
+                             : "memory");
+            }
+            last = __shfl_sync(0xffffffffu, last, 0);
+            if (last == kWarps - 1) {
+                if (lane == 0) S.done[s] = 0;
+                const int4 rf = S.run[f < 2 ? ord : ord ^ 1];
+                if (rf.y & 511) {
+                    const RunView MF = get(rf);
+                    run_fill(S, s, MF, run_of(*MF.G, rf), f ^ 2);
+                } else if (f == 2 && lane == 0) {
+                    mbar_expect(smem_addr(&S.full[0]), 0);  // wakes the block to leave
+                }
+            }
+            if (f == 0) {
+                // the closure, the moments, the polynomial that the four fields share
+                if (N.act) {
+                    if (inlet) {
+                        BCtx<F64> c{};
+                        c.uin1 = M.uin1;
+                        c.uin2 = M.uin2;
+                        c.G = M.G;
+                        c.P = M.P;
+                        decode(*M.G, g, c.b, c.i, c.j, c.k);
+                        closure_face<F64>(c, N.cls, 0, v);
+                    } else if (N.cls >= 0) {
+                        wall_flow_closure(N.cls, P.rho_out, v);
+                    }
+                    r = sum19(v);
+                    // the outlet row's density is pinned to rho_out (Tmixer.cpp:9575-9582)
+                    if (N.cls == K_OUTLET) r = P.rho_out;
+                    double sxm, sym, szm;
+                    momentum(v, sxm, sym, szm);
+                    const double ux = sxm / r, uy = sym / r, uz = szm / r;
+                    eq_poly(ux, uy, uz, poly);
+                    if (write_macro) {
+                        M.mac[ps + g] = ux;
+                        M.mac[2 * ps + g] = uy;
+                        M.mac[3 * ps + g] = uz;
+                    }
+                }
+                if (t == NT - 1) {
+                    if (next < nruns) cp_async16(&S.run[ord ^ 1], runs + next);
+                    else S.run[ord ^ 1] = make_int4(0, 0, 1, 1);
+                }
+                par = parc;
+            } else if (f != 2) {
+                if (inlet) {
+                    BCtx<F64> c{};
+                    c.P = M.P;
+                    closure_face<F64>(c, N.cls, f, v);
+                }
+                r = sum19(v);
+            }
+            if (f == 1) {
+                // B, of which the collision of A needs the sum
+                if (t == NT - 1) {
+                    cp_async_commit();
+                    cp_async_wait_all();
+                }
+                if (!mbar_wait(smem_addr(&S.full[0]), 1)) {
+                    *error = 1;
+                    return;
+                }
+                double* __restrict__ rb = &S.slot[0][t + N.xs];
+                if (inlet) {
+                    run_inlet_species<NT>(rb, par, N.cls, P.cin[1][N.cls == K_INLET2]);
+                    // (written here, filled again by a bulk copy)
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                }
+                cb = run_sum<NT>(rb, par);
+                rt = P.rateconst * r * cb;
+                m = -1.0;
+            } else if (f == 2) {
+                r = cb;
+            } else if (f == 3) {
+                m = 2.0;
+            }
+            if (N.act) {
+                // densities the closures read next step: the faces', and those
+                // of the interior nodes beside the junction edges
+                // (Tmixer.cpp:8609, :8851)
+                if (N.cls != -1) M.rcur[f * ps + g] = r;
+                if (write_macro) M.mac[(f ? 3 + f : 0) * ps + g] = r;
+                const double c1 = P.c1[f], c2 = P.c2[f];
+                const double w0 = f ? (wq(0) * rt) * m : m, w1 = f ? (wq(1) * rt) * m : m, w2 = f ? (wq(7) * rt) * m : m;
+                if (tiny_density(r))
+                    run_collide_exact(p, ps, v, r, poly, c1, c2, w0, w1, w2);
+                else
+                    run_collide(p, ps, v, r, poly, c1, c2, w0, w1, w2);
+                p += 19 * ps;
+            }
+        }
+    }
+}
+
+}  // namespace tmx
