@@ -28,7 +28,7 @@ static int check(const Geom& G, int nt)
                 const int p = fld * 19 + q;
                 first[fld][q] = count[fld][q] = 0;
                 if (!run_pulls(R, fld, EY(q), EZ(q))) continue;
-                run_window(R, run_offset(R, fld, EX(q), EY(q), EZ(q)), p, G.ps, first[fld][q], count[fld][q]);
+                run_window(R.g0, R.n, run_offset(R, fld, EX(q), EY(q), EZ(q)), p, G.ps, first[fld][q], count[fld][q]);
                 const long long at = p * G.ps + first[fld][q];
                 if (at < 0 || at % 2 || count[fld][q] % 2 || count[fld][q] > nt + 4 || at + count[fld][q] > 76 * G.ps)
                     return std::printf("window %lld + %d\n", at, count[fld][q]), 1;
@@ -55,7 +55,9 @@ static int check(const Geom& G, int nt)
             default: break;
             }
             for (int fld = 0; fld < 4; fld++) {
-                const unsigned par = run_parities(R, fld);
+                unsigned par = 0;
+                for (int q = 0; q < 19; q++)
+                    par |= ((unsigned)(R.g0 + run_offset(R, fld, EX(q), EY(q), EZ(q)) - 1) & 1u) << q;
                 for (int q = 0; q < 19; q++) {
                     const int want = fld ? pull_src(G, b, i + di, j + dj, k + dk, q) : pull_src(G, b, i, j, k, q);
                     if (want < 0) {
@@ -63,8 +65,8 @@ static int check(const Geom& G, int nt)
                         continue;
                     }
                     // the value that the thread reads from its slot's row
-                    const int at = e + (fld ? N.xs : 0) + 1 + (par >> run_bit(q) & 1);
-                    if (par == kRunEven && (int)(par >> run_bit(q) & 1) != (EX(q) == 0)) return std::printf("even\n"), 1;
+                    const int at = e + (fld ? N.xs : 0) + 1 + (par >> q & 1);
+                    if (par == kRunEven && (int)(par >> q & 1) != (EX(q) == 0)) return std::printf("even\n"), 1;
                     if (at >= count[fld][q] || first[fld][q] + at != want)
                         return std::printf("field %d direction %d of node %d: %d, not %d\n", fld, q, g,
                                            first[fld][q] + at, want),

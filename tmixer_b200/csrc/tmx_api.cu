@@ -494,7 +494,7 @@ int enqueue_run(tmx_handle* h, const tmx::StepPtrs& X, int cur, int write_macro,
 {
     const int ne = h->nb - h->nface, nr = h->nruns;
     auto launch = [&](int nruns, int nedges) {
-        const int per = h->run_nt / tmx::kBoundaryLanesHost;
+        const int per = h->run_nt / 32;  // a warp per edge node
         const int blocks = std::max(1, std::min(h->run_slots, (nedges + per - 1) / per + nruns));
         h->K->run[h->run_nt > 128]<<<blocks, h->run_nt, tmx::run_smem_host(h->run_nt), h->stream>>>(
             X, h->G, h->P, write_macro, h->runs, nruns, h->bnode + h->nface, h->bcls + h->nface, nedges, h->counters,
@@ -538,7 +538,7 @@ int enqueue_step(tmx_handle* h, int cur, int write_macro, cudaEvent_t* ev)
     TMX_CK(cudaStreamWaitEvent(h->aux2, h->fork, 0));
     if (ev) TMX_CK(cudaEventRecord(ev[2], h->aux));
     const int nf = h->nface, ne = h->nb - h->nface;
-    const int bt = tmx::kBoundaryThreadsHost, nl = tmx::kBoundaryLanesHost;  // nl threads per node
+    const int bt = tmx::kBoundaryThreadsHost, nl = tmx::kBoundaryLanesHost;  // nl threads per face
     // with a sweep shape the interior kernel updates the z wall faces, the
     // last nzwall of the face range (zwall_node)
     const int nfk = sweep_shape(h->shape) ? nf - h->nzwall : nf;

@@ -149,7 +149,40 @@ struct F64 {
         o[3] = o[3] + (w * rt) * T(2);
         store4(Pout, q, ps, g, o, f);
     }
+    __device__ static void collide_edge(S* __restrict__ Pout, int q, long long ps, int g, const T* n, const T (&r)[4],
+                                        T pw, const Phys& P, T w, T rt)
+    {
+#pragma unroll 1
+        for (int m = 0; m < 4; m++) {
+            const T rm = m == 0 ? r[0] : (m == 1 ? r[1] : (m == 2 ? r[2] : r[3])), x = rm * pw;
+            const T f = tiny(rm) ? __ddiv_rn(x, q == 0 ? 3.0 : (q <= 6 ? 18.0 : 36.0)) : feq_div(x, q);
+            T o = n[m * 20 + q] * P.c1[m] + P.c2[m] * f;
+            if (m == 3) o = o + (w * rt) * T(2);
+            else if (m) o = o - w * rt;
+            Pout[off(m, q, ps, g)] = o;
+        }
+    }
 };
+
+// The four fields of direction q of an edge node from its shared-memory row
+// (n[20 f + q]) by collide_dir (FP64: a loop over the fields with the same
+// operations, which is shorter).
+template <class PR>
+__device__ __forceinline__ void collide_edge_pairs(typename PR::S* __restrict__ Pout, int q, long long ps, int g,
+                                                   const typename PR::T* n, const typename PR::T (&r)[4],
+                                                   typename PR::T pw, const Phys& P, typename PR::T w,
+                                                   typename PR::T rt)
+{
+    using T = typename PR::T;
+    const T in[4] = {n[q], n[20 + q], n[40 + q], n[60 + q]};
+    T c1[4], c2[4];
+#pragma unroll
+    for (int m = 0; m < 4; m++) {
+        c1[m] = T(P.c1[m]);
+        c2[m] = T(P.c2[m]);
+    }
+    PR::collide_dir(Pout, q, ps, g, in, r, pw, c1, c2, w, rt);
+}
 
 // FP32 arithmetic and storage.
 struct F32 {
@@ -254,6 +287,11 @@ struct F32 {
 #pragma unroll
         for (int m = 0; m < 4; m++)
             if (m >= first && m < last) v[m] = u[m];
+    }
+    __device__ static void collide_edge(S* Pout, int q, long long ps, int g, const T* n, const T (&r)[4], T pw,
+                                        const Phys& P, T w, T rt)
+    {
+        collide_edge_pairs<F32>(Pout, q, ps, g, n, r, pw, P, w, rt);
     }
     __device__ static T decode(const S* p, int, int, const float4*, long long, int) { return __ldg(p); }
     __device__ static void encode(S* p, T v, T) { *p = v; }
@@ -394,6 +432,11 @@ struct F16 {
 #pragma unroll
         for (int m = 0; m < 4; m++)
             if (m >= first && m < last) v[m] = u[m];
+    }
+    __device__ static void collide_edge(S* Pout, int q, long long ps, int g, const T* n, const T (&r)[4], T pw,
+                                        const Phys& P, T w, T rt)
+    {
+        collide_edge_pairs<F16>(Pout, q, ps, g, n, r, pw, P, w, rt);
     }
     __device__ static T decode(const S* p, int fld, int q, const float4* M, long long, int src)
     {
@@ -987,7 +1030,10 @@ struct CornerSpec {
     signed char avg[3][2];
     signed char cp[2];
 };
-static __constant__ CornerSpec kCorner[16] = {
+struct CornerTable {
+    CornerSpec c[16];
+};
+constexpr CornerTable kCorners = {{
     {{{1, 3}, {4, 2}, {6, 5}, {10, 8}, {14, 12}, {17, 15}}, 2, {{9, 7}, {11, 13}, {0, 0}}, {16, 18}},    // 1 G'
     {{{3, 1}, {4, 2}, {6, 5}, {17, 15}, {13, 11}, {9, 7}}, 2, {{10, 8}, {12, 14}, {0, 0}}, {16, 18}},    // 2 F'
     {{{1, 3}, {2, 4}, {6, 5}, {7, 9}, {18, 16}, {14, 12}}, 2, {{10, 8}, {11, 13}, {0, 0}}, {15, 17}},    // 3 H'
@@ -1004,14 +1050,15 @@ static __constant__ CornerSpec kCorner[16] = {
     {{{6, 5}, {8, 10}, {13, 11}, {14, 12}, {17, 15}, {18, 16}}, 3, {{9, 7}, {4, 2}, {1, 3}}, {-1, -1}},  // 14 C'
     {{{5, 6}, {8, 10}, {11, 13}, {12, 14}, {15, 17}, {16, 18}}, 3, {{1, 3}, {4, 2}, {9, 7}}, {-1, -1}},  // 15 C
     {{{5, 6}, {7, 9}, {11, 13}, {12, 14}, {15, 17}, {16, 18}}, 3, {{1, 3}, {4, 2}, {8, 10}}, {-1, -1}},  // 16 D
-};
+}};
+static __constant__ CornerTable kCorner = kCorners;
 
 // Corner closure on a local copy (runtime indices; 16 nodes per mixer).
 template <class PR>
 __device__ __forceinline__ void corner_closure(const BCtx<PR>& c, int fld, int n, typename PR::T R, typename PR::T* t)
 {
     using T = typename PR::T;
-    const CornerSpec& s = kCorner[n];
+    const CornerSpec& s = kCorner.c[n];
     for (int m = 0; m < 6; m++) t[s.bb[m][0]] = t[s.bb[m][1]];
     T fa[3];
     for (int m = 0; m < s.navg; m++) fa[m] = T(0.5) * (own_fn(c, fld, s.avg[m][0]) + own_fn(c, fld, s.avg[m][1]));
@@ -1334,6 +1381,300 @@ __device__ __forceinline__ void closure_edge(const BCtx<PR>& c, int cls, int fld
         }
     } break;
     }
+}
+
+// ---------------------------------------------------------------------------
+// edges and corners (Tmixer.cpp:2030-2605, :4238-5571, :5572-7785, :7786-9033)
+//
+// Every closure of an edge or corner node is of one shape: directions that
+// bounce back, on edges with a quarter of the momentum along the edge taken
+// off the ones that run along it; pairs averaged from the node's own
+// post-collision values ("undo streaming"); and at most one pair closed from a
+// density.  So a class is a few bit masks over the directions (EdgeRule), and a
+// warp takes one node, lane q its direction q: all loads of the node are in
+// flight at once and the code is short.  (Four lanes per node with
+// the closures written out by class took 20 us for a launch of any size:
+// thousands of instructions in a row, most of it waiting for them to be fetched.)
+// ---------------------------------------------------------------------------
+
+struct EdgeRule {
+    unsigned back;    // directions set to their opposite's value
+    unsigned minus;   // ... less a quarter of the momentum along the edge
+    unsigned plus;    // ... and those with it added
+    unsigned avg;     // directions set to the mean of their own two values
+    unsigned closed;  // the pair closed from a density
+    int axis;         // along the edge: 0 x, 1 y, 2 z
+};
+constexpr int OPP(int q)
+{
+    for (int p = 0; p < 19; p++)
+        if (EX(p) == -EX(q) && EY(p) == -EY(q) && EZ(p) == -EZ(q)) return p;
+    return 0;
+}
+constexpr int edge_comp(int q, int axis) { return axis == 0 ? EX(q) : (axis == 1 ? EY(q) : EZ(q)); }
+// The edge between walls with inward normals n1 along axis a1 and n2 along a2.
+// The pair that points along neither is closed from a density, or averaged.
+constexpr EdgeRule edge_rule(int a1, int n1, int a2, int n2, bool density)
+{
+    EdgeRule r{};
+    r.axis = 3 - a1 - a2;
+    for (int q = 1; q < 19; q++) {
+        const int i1 = edge_comp(q, a1) * n1, i2 = edge_comp(q, a2) * n2, e = edge_comp(q, r.axis);
+        if (i1 * i2 < 0) {
+            (density ? r.closed : r.avg) |= 1u << q;
+        } else if (i1 > 0 || i2 > 0) {
+            r.back |= 1u << q;
+            if (e > 0) r.minus |= 1u << q;
+            if (e < 0) r.plus |= 1u << q;
+        }
+    }
+    return r;
+}
+constexpr EdgeRule corner_rule(int n)
+{
+    EdgeRule r{};
+    const CornerSpec& s = kCorners.c[n];
+    for (int m = 0; m < 6; m++) r.back |= 1u << s.bb[m][0];
+    for (int m = 0; m < s.navg; m++) r.avg |= (1u << s.avg[m][0]) | (1u << s.avg[m][1]);
+    if (s.cp[0] >= 0) r.closed = (1u << s.cp[0]) | (1u << s.cp[1]);
+    return r;
+}
+// the junction edges: every pair but the closed one averaged
+constexpr EdgeRule junction_rule(int a, int b)
+{
+    EdgeRule r{};
+    r.closed = (1u << a) | (1u << b);
+    r.avg = 0x7fffeu & ~r.closed;
+    return r;
+}
+constexpr EdgeRule edge_rule_of(int cls)
+{
+    switch (cls) {
+    case K_EDGE_Y1_ZTOP: return edge_rule(1, 1, 2, -1, false);   // Cases 2, 3 (:2030-2342)
+    case K_EDGE_X1_ZTOP: return edge_rule(0, 1, 2, -1, true);    // Case 4 (:2343-2476)
+    case K_EDGE_XT_ZTOP: return edge_rule(0, -1, 2, -1, true);   // Case 6 (:2477-2605)
+    case K_EDGE_YT_ZT: return edge_rule(1, -1, 2, -1, false);    // Case 20 (:4238-4385)
+    case K_EDGE_YT_Z1: return edge_rule(1, -1, 2, 1, false);     // Case 21 (:4386-4533)
+    case K_EDGE_X1_Z1: return edge_rule(0, 1, 2, 1, true);       // Case 22 (:4534-4656)
+    case K_EDGE_XT_Z1: return edge_rule(0, -1, 2, 1, true);      // Case 23 (:4657-4779)
+    case K_EDGE_X1_Y1: return edge_rule(0, 1, 1, 1, true);       // Case 24 (:4780-4909)
+    case K_EDGE_X1_YT: return edge_rule(0, 1, 1, -1, true);      // Case 25 (:4910-5032)
+    case K_EDGE_XT_Y1: return edge_rule(0, -1, 1, 1, true);      // Case 26 (:5033-5159)
+    case K_EDGE_XT_YT: return edge_rule(0, -1, 1, -1, true);     // Case 27 (:5160-5281)
+    case K_EDGE_Y1_Z1: return edge_rule(1, 1, 2, 1, false);      // Cases 28, 29 (:5282-5571)
+    case K_MEDGE_AB: return edge_rule(1, 1, 2, 1, true);         // (:7788-7868)
+    case K_MEDGE_ApBp: return edge_rule(1, 1, 2, -1, true);      // (:7870-7950)
+    case K_MEDGE_AAp: return edge_rule(0, 1, 1, 1, true);        // (:7951-8043)
+    case K_MEDGE_BBp: return edge_rule(0, -1, 1, 1, true);       // (:8044-8136)
+    case K_MEDGE_AD: return edge_rule(0, 1, 2, 1, false);        // (:8137-8244)
+    case K_MEDGE_ApDp: return edge_rule(0, 1, 2, -1, false);     // (:8245-8344)
+    case K_MEDGE_BC: return edge_rule(0, -1, 2, 1, false);       // (:8345-8445)
+    case K_MEDGE_BpCp: return edge_rule(0, -1, 2, -1, false);    // (:8446-8550)
+    case K_JUNC_DD: return junction_rule(7, 9);                  // (:8551-8792)
+    case K_JUNC_CC: return junction_rule(8, 10);                 // (:8793-9033)
+    default: return cls >= K_CORNER_1 && cls <= K_CORNER_16 ? corner_rule(cls - K_CORNER_1) : EdgeRule{};
+    }
+}
+struct EdgeRules {
+    EdgeRule r[K_NCLASSES];
+};
+constexpr EdgeRules make_edge_rules()
+{
+    EdgeRules t{};
+    for (int c = 0; c < K_NCLASSES; c++) t.r[c] = edge_rule_of(c);
+    return t;
+}
+static __constant__ EdgeRules kEdgeRules = make_edge_rules();
+
+// Direction q < 19 (a run-time value): its lattice vector and opposite, from
+// two bits and five bits each.
+constexpr unsigned long long pack_dirs(int axis)
+{
+    unsigned long long m = 0;
+    for (int q = 0; q < 19; q++) m |= (unsigned long long)(edge_comp(q, axis) + 1) << (2 * q);
+    return m;
+}
+constexpr unsigned long long pack_opp(int first)
+{
+    unsigned long long m = 0;
+    for (int q = first; q < first + 10 && q < 19; q++) m |= (unsigned long long)OPP(q) << (5 * (q - first));
+    return m;
+}
+constexpr unsigned long long kDirX = pack_dirs(0), kDirY = pack_dirs(1), kDirZ = pack_dirs(2), kOppLo = pack_opp(0),
+                             kOppHi = pack_opp(10);
+__device__ __forceinline__ void dir_of(int q, int& ex, int& ey, int& ez, int& opp)
+{
+    ex = (int)((kDirX >> (2 * q)) & 3) - 1;
+    ey = (int)((kDirY >> (2 * q)) & 3) - 1;
+    ez = (int)((kDirZ >> (2 * q)) & 3) - 1;
+    opp = (int)((q < 10 ? kOppLo >> (5 * q) : kOppHi >> (5 * (q - 10))) & 31);
+}
+
+// The density an edge or corner node's pair is closed from: of the previous
+// step at node (b, i, j, k), except the flow's where flow says otherwise.
+enum EdgeDensity { kDensPrev = 0, kDensOutlet, kDensInlet1, kDensInlet2, kDensZero };
+__device__ __forceinline__ void edge_density(const Geom& G, int cls, int& i, int& j, int& k, int& flow, int& species)
+{
+    flow = species = kDensPrev;
+    switch (cls) {
+    case K_EDGE_X1_ZTOP:
+    case K_EDGE_XT_ZTOP: k = G.nz - 1; break;
+    // the inlet's flow density of this step (Tmixer.cpp:2612-2615, :2675-2678)
+    case K_EDGE_X1_Z1: k = 2; flow = kDensInlet1; break;
+    case K_EDGE_XT_Z1: k = 2; flow = kDensInlet2; break;
+    case K_EDGE_X1_Y1: j = 2; flow = kDensInlet1; break;
+    case K_EDGE_X1_YT: j = G.iny - 1; flow = kDensInlet1; break;
+    case K_EDGE_XT_Y1: j = 2; flow = kDensInlet2; break;
+    case K_EDGE_XT_YT: j = G.iny - 1; flow = kDensInlet2; break;
+    case K_MEDGE_AB:
+    case K_MEDGE_ApBp:
+    case K_MEDGE_AAp:
+    case K_MEDGE_BBp: j = 2; flow = kDensOutlet; break;
+    case K_JUNC_DD:
+    case K_JUNC_CC: j = 2; break;
+    default:
+        // inlet corners: the density of the adjacent x-y edge node; outlet
+        // corners: rho_out, the species read the row below the outlet, which is 0
+        if (cls < K_CORNER_1 + 8) {
+            k = k == G.nz ? G.nz - 1 : 2;
+        } else {
+            flow = kDensOutlet;
+            species = kDensZero;
+        }
+    }
+}
+
+constexpr int kEdgeBuf = 5 * 20;   // a warp's values in shared memory: 19 of each field and of an inlet node
+
+// Edge or corner node g of class cls by one warp (all lanes).  The arithmetic is
+// that of the reference's cases in order: the sums in index order on one lane.
+template <class PR>
+__device__ __forceinline__ void edge_node(const StepPtrs& X, const Geom& G, const Phys& P, int write_macro, int g,
+                                          int cls, typename PR::T* buf)
+{
+    using T = typename PR::T;
+    const typename PR::S* __restrict__ Pin = (const typename PR::S*)X.pin;
+    const float4* __restrict__ Mom = X.mprev;
+    const T* __restrict__ Rprev = (const T*)X.rprev;
+    const long long ps = G.ps;
+    const int lane = threadIdx.x & 31, q = lane < 19 ? lane : 18;
+    const bool mine = lane < 19;
+    const EdgeRule& rule = kEdgeRules.r[cls];
+    int b, i, j, k, ex, ey, ez, opp;
+    decode(G, g, b, i, j, k);
+    dir_of(q, ex, ey, ez, opp);
+    const unsigned bit = mine ? 1u << q : 0u;
+
+    // the pulled values, the own two of an averaged direction, and the densities
+    T v[4] = {T(0), T(0), T(0), T(0)}, own[4], R = T(0), U = T(0), w = T(0);
+    const int s0 = pull_src_e(G, b, i, j, k, ex, ey, ez);
+    if (mine && s0 >= 0) PR::decode_fields(Pin, Mom, ps, q, ex, ey, ez, T(wq(q)), s0, v, 0, 4);
+    if (bit & rule.avg)
+#pragma unroll
+        for (int f = 0; f < 4; f++)
+            own[f] = T(0.5) * (PR::decode(Pin + PR::off(f, q, ps, g), f, q, Mom, ps, g) +
+                               PR::decode(Pin + PR::off(f, opp, ps, g), f, opp, Mom, ps, g));
+    // Case 4's species C keeps p13, its own value (Tmixer.cpp:2474)
+    const bool keep = cls == K_EDGE_X1_ZTOP;
+    if (keep && lane == 13) own[3] = PR::decode(Pin + PR::off(3, 13, ps, g), 3, 13, Mom, ps, g);
+    int inlet = 0;
+    if (rule.closed) {
+        int di = i, dj = j, dk = k, flow, species;
+        edge_density(G, cls, di, dj, dk, flow, species);
+        const int what = lane == 0 ? flow : species;
+        if (lane < 4) {
+            if (what == kDensPrev) R = __ldg(Rprev + (long long)lane * ps + node_index(G, b, di, dj, dk));
+            else if (what == kDensOutlet) R = T(P.rho_out);
+        }
+        if (flow == kDensInlet1 || flow == kDensInlet2) {
+            inlet = flow == kDensInlet1 ? 1 : 2;
+            const int s1 = pull_src_e(G, 0, di, dj, dk, ex, ey, ez);
+            if (mine && s1 >= 0) w = PR::decode(Pin + PR::off(0, q, ps, s1), 0, q, Mom, ps, s1);
+            U = __ldg((const T*)(inlet == 1 ? X.uin1 : X.uin2) + dj * (G.nz + 3) + dk);
+        }
+    }
+    if (mine) {
+#pragma unroll
+        for (int f = 0; f < 4; f++) buf[f * 20 + q] = bit & rule.avg ? own[f] : v[f];
+        if (inlet) buf[80 + q] = w;
+    }
+    __syncwarp();
+    // bounce back: from directions that no closure changes, as is the momentum
+    // along the edge
+    if (bit & rule.back) {
+        const int a = rule.axis == 0 ? 1 : (rule.axis == 1 ? 2 : 5), c = rule.axis == 0 ? 3 : (rule.axis == 1 ? 4 : 6);
+#pragma unroll
+        for (int f = 0; f < 4; f++) {
+            T x = buf[f * 20 + opp];
+            if (bit & (rule.minus | rule.plus)) {
+                const T A = T(0.25) * (buf[f * 20 + a] - buf[f * 20 + c]);
+                x = bit & rule.minus ? x - A : x + A;
+            }
+            buf[f * 20 + q] = x;
+        }
+    }
+    __syncwarp();
+    // the closed pair, field f on lane f
+    if (rule.closed) {
+        if (lane < 4) {
+            if (inlet && lane == 0) {
+                const T* n = buf + 80;
+                const T along = n[0] + n[2] + n[4] + n[5] + n[6] + n[15] + n[16] + n[17] + n[18];
+                if (inlet == 1)
+                    R = (T(1) / (T(1) - U)) * (along + T(2) * (n[3] + n[8] + n[9] + n[12] + n[13]));
+                else
+                    R = (T(1) / (T(1) + (U))) * (along + T(2) * (n[1] + n[7] + n[10] + n[11] + n[14]));
+            }
+            T* n = buf + lane * 20;
+            T s = n[0];  // (the closed pair is never direction 0)
+#pragma unroll
+            for (int d = 1; d < 19; d++)
+                if (!((rule.closed >> d) & 1)) s = s + n[d];
+            const T c = T(0.5) * (R - s);
+            n[__ffs(rule.closed) - 1] = c;
+            n[31 - __clz(rule.closed)] = c;
+        }
+        __syncwarp();
+        if (keep && lane == 13) buf[60 + 13] = own[3];
+        __syncwarp();
+    }
+    // density of field f on lane f; momentum on lanes 4, 5, 6
+    T r = T(0);
+    if (lane < 4) {
+        const T* n = buf + lane * 20;
+        r = n[0];
+#pragma unroll
+        for (int d = 1; d < 19; d++) r += n[d];
+        // the outlet row's density is pinned to rho_out (Tmixer.cpp:9575-9582)
+        if (lane == 0 && b == 1 && j == 1) r = T(P.rho_out);
+    } else if (lane < 7) {
+        // (the first term of each sum is positive)
+        const unsigned long long dirs = lane == 4 ? kDirX : (lane == 5 ? kDirY : kDirZ);
+        const int first = lane == 4 ? 1 : (lane == 5 ? 2 : 5);
+        r = buf[first];
+#pragma unroll
+        for (int d = 1; d < 19; d++) {
+            const int e = (int)((dirs >> (2 * d)) & 3) - 1;
+            if (e != 0 && d != first) r = e > 0 ? r + buf[d] : r - buf[d];
+        }
+    }
+    const T u = r / __shfl_sync(0xffffffffu, r, 0);
+    if (lane < 4) ((T*)X.rcur)[lane * ps + g] = r;
+    if (write_macro && lane < 7) X.mac[(lane == 0 ? 0 : (lane < 4 ? 3 + lane : lane - 3)) * ps + g] = lane < 4 ? r : u;
+    const T rr[4] = {__shfl_sync(0xffffffffu, r, 0), __shfl_sync(0xffffffffu, r, 1), __shfl_sync(0xffffffffu, r, 2),
+                     __shfl_sync(0xffffffffu, r, 3)};
+    const T ux = __shfl_sync(0xffffffffu, u, 4), uy = __shfl_sync(0xffffffffu, u, 5), uz = __shfl_sync(0xffffffffu, u, 6);
+    if (mine) {
+        const T wt = T(wq(q)), rt = T(P.rateconst) * rr[1] * rr[2];
+        PR::collide_edge((typename PR::S*)X.pout, q, ps, g, buf, rr, PR::pw_dir(ex, ey, ez, wt, ux, uy, uz), P, wt, rt);
+    }
+    if (PR::kMoments) {
+        if (lane == 0) X.mcur[2 * (long long)g] = make_float4((float)rr[0], (float)rr[1], (float)rr[2], (float)rr[3]);
+        if (lane == 1)
+            X.mcur[2 * (long long)g + 1] =
+                make_float4((float)ux, (float)uy, (float)uz, omt_term((float)ux, (float)uy, (float)uz));
+    }
+    __syncwarp();  // buf is free again
 }
 
 // The post-closure populations of field fld of the boundary node in c.  A

@@ -11,29 +11,24 @@ namespace tmx {
 
 TMX_DEFINE_INIT_KERNEL(F64, f64)
 
-// The FP64 step (tmx_run64.cuh): the first blocks begin with the edge and
-// corner nodes (eight to a warp), all of them go through the runs.
+// The FP64 step (tmx_run64.cuh): the runs, and the edge and corner nodes, a
+// warp each, which the warps take while their block's first run is on its way
+// (on a small mixer the blocks without a run take them).
 template <int NT>
 __device__ __forceinline__ void run_step(const StepPtrs& X, const Geom& G, const Phys& P, int write_macro,
                                          const int4* __restrict__ runs, int nruns, const int* __restrict__ enode,
                                          const unsigned char* __restrict__ ecls, int ne, int* __restrict__ counters,
                                          int parity, int* error, RunShared<NT>& S)
 {
-    constexpr int kPer = NT / kBoundaryLanes;
+    const int warp = threadIdx.x >> 5, nb = gridDim.x;
     if (blockIdx.x == 0 && threadIdx.x == 0) counters[1 - parity] = 0;  // the next step's
-    const int eb = (ne + kPer - 1) / kPer;
-    for (int u = blockIdx.x; u < eb; u += gridDim.x)
-        run_edges(X, G, P, write_macro, [&](int e, int& node, int& cls) {
-            const int at = u * kPer + (threadIdx.x >> 5) * 8 + e;
-            if (at < ne) {
-                node = enode[at];
-                cls = ecls[at];
-            }
-        });
-    // the blocks without edges begin with the first runs
-    const int nb = gridDim.x;
-    run_loop<NT>([&](const int4&) { return run_view(X, G, P); }, runs, nruns, (int)(blockIdx.x + nb - eb % nb) % nb, nb,
-                 counters + parity, write_macro, S, error);
+    run_loop<NT>([&](const int4&) { return run_view(X, G, P); }, runs, nruns, blockIdx.x, nb, counters + parity,
+                 write_macro, S, error, [&] {
+                     // the blocks without a run first
+                     const int at = (int)(blockIdx.x + nb - nruns % nb) % nb;
+                     for (int e = at * (NT / 32) + warp; e < ne; e += nb * (NT / 32))
+                         run_edge(X, G, P, write_macro, enode[e], ecls[e], S.edge[warp]);
+                 });
 }
 #define TMX_DEFINE_RUN(NT)                                                                                      \
     __global__ void __launch_bounds__(NT, 512 / NT) k_run##NT##_f64(                                            \

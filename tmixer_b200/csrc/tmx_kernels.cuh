@@ -50,8 +50,8 @@ TMX_DECLARE_BOUNDARY_KERNELS(f16)
 // 256; run_threads in tmx_host.h).  iface: the row whose ey = 1 (1) or ey = -1
 // (2) sources lie in the other box.
 enum RunKind { kRunRows = 0, kRunZ1, kRunZT, kRunYT, kRunY1 };
-constexpr int run_smem_host(int nt) { return 2 * 19 * (nt + 4) * 8 + 64; }  // RunShared
-// Edge and corner nodes enode[0..ne), then the runs; counters[parity] hands
+constexpr int run_smem_host(int nt) { return 2 * 19 * (nt + 4) * 8 + nt / 32 * 800 + 400; }  // RunShared
+// The runs, and the edge and corner nodes enode[0..ne); counters[parity] hands
 // out the runs, counters[1 - parity] is cleared for the next step.
 #define TMX_DECLARE_RUN(NT)                                                                                     \
     __global__ void k_run##NT##_f64(const __grid_constant__ StepPtrs X, const __grid_constant__ Geom G,         \
@@ -73,7 +73,7 @@ struct MixerDesc {
 // Batched step kernels: one launch covers every mixer of a batch.
 //   bulk    a persistent grid walks a list of cell blocks {mixer, first
 //           node, node count, 0}; NT threads per block (128, 256 or 512).
-//   faces / edges   boundary-node lists of {node, mixer * 256 + class},
+//   faces / edges   boundary-node lists of {node, mixer * 256 + class}, 
 //           four threads per node, persistent grid; each mixer's part
 //           starts at a multiple of kListAlign, padded with node -1.
 // counts[0..2] = number of cell blocks, face nodes, edge nodes (device

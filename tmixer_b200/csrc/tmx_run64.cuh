@@ -154,10 +154,10 @@ __host__ __device__ inline bool run_pulls(const Run& R, int fld, int ey, int ez)
 // bulk copy starts and ends at 16 bytes): the run's sources and one more at
 // either end, for the x walls' neighbours.  Plane p of the 76; the last values
 // stop at the end of the buffer.
-__host__ __device__ inline void run_window(const Run& R, int off, int p, long long ps, int& first, int& count)
+__host__ __device__ inline void run_window(int g0, int n, int off, int p, long long ps, int& first, int& count)
 {
-    first = (R.g0 + off - 1) & ~1;
-    count = (R.n + 5) & ~1;
+    first = (g0 + off - 1) & ~1;
+    count = (n + 5) & ~1;
     const long long left = (76 - p) * ps - first;
     if (count > left) count = (int)left;
 }
@@ -168,9 +168,12 @@ template <int NT>
 struct __align__(16) RunShared {
     static constexpr int kRow = NT + 4;
     double slot[2][19 * kRow];
-    int4 run[2];  // by the run's ordinal in the block; n = 0: none
+    int4 run[2];         // by the run's ordinal in the block; n = 0: none
+    int off[2][2][20];   // ... its offsets by direction, of the flow and of the species
+    unsigned par[2][2];  // ... and the parities that they begin with
     unsigned long long full[2];
     int done[2];  // warps that have read a slot
+    double edge[NT / 32][kEdgeBuf];
 };
 static_assert(sizeof(RunShared<128>) == run_smem_host(128) && sizeof(RunShared<256>) == run_smem_host(256),
               "host copy of the size");
@@ -183,48 +186,54 @@ __device__ __forceinline__ int4 run_shared(const int4& t)
                      __shfl_sync(0xffffffffu, t.z, 0), __shfl_sync(0xffffffffu, t.w, 0));
 }
 
-// Fill a slot with field fld of run t (one warp; lane q copies direction q).
+// What a block needs of its run number ord (in S.run): the offsets of the
+// sources and their parities (one warp; lane q does direction q).
+constexpr int kRunNone = -0x7fffffff;  // no sources
 template <int NT>
-__device__ __forceinline__ void run_fill(RunShared<NT>& S, int slot, const RunView& M, const Run& R, int fld)
+__device__ __forceinline__ void run_prepare(RunShared<NT>& S, int ord, const Geom& G)
 {
-    const int q = threadIdx.x & 31;
-    const unsigned bar = smem_addr(&S.full[slot]);
-    int ex = 0, ey = 0, ez = 0;
+    const int lane = threadIdx.x & 31, q = lane < 19 ? lane : 18;
+    const Run R = run_of(G, S.run[ord]);
+    int ex, ey, ez, opp;
+    dir_of(q, ex, ey, ez, opp);
 #pragma unroll
-    for (int d = 0; d < 19; d++)
-        if (q == d) {
-            ex = EX(d);
-            ey = EY(d);
-            ez = EZ(d);
-        }
-    const bool mine = q < 19 && run_pulls(R, fld, ey, ez);
+    for (int c = 0; c < 2; c++) {
+        const int off = run_offset(R, c, ex, ey, ez);
+        const unsigned par = __ballot_sync(0xffffffffu, ((R.g0 + off - 1) & 1) && lane < 19);
+        if (lane < 19) S.off[ord][c][q] = run_pulls(R, c, ey, ez) ? off : kRunNone;
+        if (lane == 0) S.par[ord][c] = par;
+    }
+}
+
+// Fill a slot with field fld of run number ord (one warp; lane q copies
+// direction q).
+template <int NT>
+__device__ __forceinline__ void run_fill(RunShared<NT>& S, int slot, int ord, const RunView& M, int fld)
+{
+    const int q = threadIdx.x & 31, p = fld * 19 + q;
+    const unsigned bar = smem_addr(&S.full[slot]);
+    const int off = q < 19 ? S.off[ord][fld ? 1 : 0][q] : kRunNone;
     const long long ps = M.G->ps;
-    const int p = fld * 19 + q;
     int first = 0, count = 0;
-    if (mine) run_window(R, run_offset(R, fld, ex, ey, ez), p, ps, first, count);
+    if (off != kRunNone) run_window(S.run[ord].x, S.run[ord].y & 511, off, p, ps, first, count);
     const unsigned bytes = __reduce_add_sync(0xffffffffu, (unsigned)count) * 8u;
     if (q == 0) mbar_expect(bar, bytes);
     __syncwarp();
-    if (mine)
+    if (count)
         bulk_load(smem_addr(&S.slot[slot][q * (NT + 4)]), M.pin + p * ps + first, (unsigned)count * 8u, bar);
 }
 
 // Where a thread's values of a field lie: in row q of the slot one or two
 // beyond the thread's number, by the parity of the source that the window
-// begins with.  The parity of the ten kinds of direction (ey, ex != 0,
-// ez != 0), as bits; kRunEven: rows and planes of even length, where only the
-// x component counts.
-__host__ __device__ constexpr int run_bit(int q) { return (EY(q) + 1) * 4 + (EX(q) != 0) * 2 + (EZ(q) != 0); }
-constexpr unsigned kRunEven = 0x333;
-__host__ __device__ inline unsigned run_parities(const Run& R, int fld)
+// begins with (bit q).  kRunEven: rows and planes of even length, where only
+// the x component counts.
+constexpr unsigned run_even()
 {
     unsigned m = 0;
-    for (int ey = -1; ey <= 1; ey++)
-        for (int x = 0; x < 2; x++)
-            for (int z = 0; z < 2; z++)
-                m |= ((unsigned)(R.g0 + run_offset(R, fld, x, ey, z) - 1) & 1u) << ((ey + 1) * 4 + x * 2 + z);
+    for (int q = 0; q < 19; q++) m |= (EX(q) == 0 ? 1u : 0u) << q;
     return m;
 }
+constexpr unsigned kRunEven = run_even();
 template <int NT>
 __device__ __forceinline__ void run_read(const double* __restrict__ row, unsigned par, double (&v)[19])
 {
@@ -233,7 +242,7 @@ __device__ __forceinline__ void run_read(const double* __restrict__ row, unsigne
         for (int q = 0; q < 19; q++) v[q] = row[q * (NT + 4) + (EX(q) == 0 ? 2 : 1)];
     } else {
 #pragma unroll
-        for (int q = 0; q < 19; q++) v[q] = row[q * (NT + 4) + 1 + ((par >> run_bit(q)) & 1)];
+        for (int q = 0; q < 19; q++) v[q] = row[q * (NT + 4) + 1 + ((par >> q) & 1)];
     }
 }
 template <int NT>
@@ -249,7 +258,7 @@ __device__ __forceinline__ double run_sum(const double* __restrict__ row, unsign
     } else {
 #pragma unroll
         for (int q = 0; q < 19; q++) {
-            const double x = row[q * (NT + 4) + 1 + ((par >> run_bit(q)) & 1)];
+            const double x = row[q * (NT + 4) + 1 + ((par >> q) & 1)];
             s = q ? s + x : x;
         }
     }
@@ -262,7 +271,7 @@ template <int NT>
 __device__ __forceinline__ void run_inlet_species(double* row, unsigned par, int cls, double cin)
 {
     const double w1 = 2.0 / 18.0 * cin, w2 = 2.0 / 36.0 * cin;
-    auto at = [&](int q) -> double& { return row[q * (NT + 4) + 1 + ((par >> run_bit(q)) & 1)]; };
+    auto at = [&](int q) -> double& { return row[q * (NT + 4) + 1 + ((par >> q) & 1)]; };
     const bool one = cls == K_INLET1;
     constexpr int in[5] = {1, 7, 10, 11, 14}, out[5] = {3, 9, 8, 13, 12};  // opposite pairs
 #pragma unroll
@@ -308,30 +317,28 @@ __device__ __forceinline__ void run_collide_exact(double* __restrict__ p, long l
     }
 }
 
-// Up to eight edge and corner nodes, four lanes each; at(e, node, cls) gives
-// entry e of the warp's share (node -1: none).
-template <class At>
-__device__ __forceinline__ void run_edges(const StepPtrs& X, const Geom& G, const Phys& P, int write_macro, const At& at)
+// An edge or corner node, out of line: its registers are not the runs' concern.
+__device__ __noinline__ void run_edge(const StepPtrs& X, const Geom& G, const Phys& P, int write_macro, int node, int cls,
+                                      double* buf)
 {
-    const int lane = threadIdx.x & 31;
-    int node = -1, cls = 0;
-    at(lane >> 2, node, cls);
-    const unsigned mask = __ballot_sync(0xffffffffu, node >= 0);
-    if (node >= 0) boundary_lane<F64, false>(X, G, P, write_macro, node, cls, lane & 3, mask, lane & ~3);
+    edge_node<F64>(X, G, P, write_macro, node, cls, buf);
 }
 
-// The runs of one block: the first by its number, then by the launch's counter
-// (dynamic: the blocks that begin with edges take fewer).  get(t) gives the
-// buffers, geometry and constants of run t's mixer.  error: set when a copy
-// does not arrive.
-template <int NT, class Get>
+// The runs of one block: the first by its number, then by the launch's counter.
+// get(t) gives the buffers, geometry and constants of run t's mixer.  error: set
+// when a copy does not arrive.  meanwhile(): what the warps do while the first
+// run's copies are on their way.
+template <int NT, class Get, class Mean>
 __device__ __forceinline__ void run_loop(const Get& get, const int4* __restrict__ runs, int nruns, int first,
                                          int nblocks, int* __restrict__ counter, int write_macro, RunShared<NT>& S,
-                                         int* error)
+                                         int* error, const Mean& meanwhile)
 {
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     constexpr int kWarps = NT / 32;
-    if (first >= nruns) return;  // (the whole block)
+    if (first >= nruns) {  // (the whole block)
+        meanwhile();
+        return;
+    }
     if (t == 0) {
         for (int s = 0; s < 2; s++) {
             mbar_init(smem_addr(&S.full[s]), 1);
@@ -342,12 +349,13 @@ __device__ __forceinline__ void run_loop(const Get& get, const int4* __restrict_
     }
     __syncthreads();
     if (warp == 0) {
-        const int4 r = S.run[0];
-        const RunView M = get(r);
-        const Run R = run_of(*M.G, r);
-        run_fill(S, 0, M, R, 0);
-        run_fill(S, 1, M, R, 1);
+        const RunView M = get(S.run[0]);
+        run_prepare(S, 0, *M.G);
+        __syncwarp();
+        run_fill(S, 0, 0, M, 0);
+        run_fill(S, 1, 0, M, 1);
     }
+    meanwhile();
     for (int ord = 0;; ord ^= 1) {
         // (each barrier goes through two phases a run: the parities repeat)
         if (!mbar_wait(smem_addr(&S.full[0]), 0)) {
@@ -360,15 +368,15 @@ __device__ __forceinline__ void run_loop(const Get& get, const int4* __restrict_
         const Phys& P = *M.P;
         const long long ps = M.G->ps;
         const int g = tr.x + t;
-        RunNode N;
-        unsigned par, parc;
+        // the node's class, x shift and activity, in one register
+        int what;
         {
-            const Run R = run_of(*M.G, tr);
-            N = run_node(*M.G, R, t);
-            par = run_parities(R, 0);
-            parc = run_parities(R, 1);
+            const RunNode N = run_node(*M.G, run_of(*M.G, tr), t);
+            what = (N.cls << 3) | ((N.xs + 1) << 1) | (int)N.act;
         }
-        const bool inlet = N.cls == K_INLET1 || N.cls == K_INLET2;
+        const auto cls = [&] { return what >> 3; };
+        const auto inlet = [&] { return cls() == K_INLET1 || cls() == K_INLET2; };
+        const auto act = [&] { return (what & 1) != 0; };
         double* __restrict__ p = M.pout + g;
         // the next run: its index now, its entry after the flow, there for
         // all before the block has read B
@@ -376,7 +384,7 @@ __device__ __forceinline__ void run_loop(const Get& get, const int4* __restrict_
         if (t == NT - 1) next = nblocks + atomicAdd(counter, 1);
 
         double poly[19], v[19];
-        double r = 0.0, cb = 0.0, m = -0.0, rt = 0.0;
+        double r = 0.0, cb = 0.0, rt = 0.0;
 #pragma unroll 1
         for (int f = 0; f < 4; f++) {
             const int s = f & 1;
@@ -384,7 +392,7 @@ __device__ __forceinline__ void run_loop(const Get& get, const int4* __restrict_
                 *error = 1;
                 return;
             }
-            run_read<NT>(&S.slot[s][t + (f ? N.xs : 0)], par, v);
+            run_read<NT>(&S.slot[s][t + (f ? ((what >> 1) & 3) - 1 : 0)], S.par[ord][f ? 1 : 0], v);
             // the slot is free once every warp has read it; the last fills it
             // with the field after the next
             __syncwarp();
@@ -398,31 +406,30 @@ __device__ __forceinline__ void run_loop(const Get& get, const int4* __restrict_
             last = __shfl_sync(0xffffffffu, last, 0);
             if (last == kWarps - 1) {
                 if (lane == 0) S.done[s] = 0;
-                const int4 rf = S.run[f < 2 ? ord : ord ^ 1];
-                if (rf.y & 511) {
-                    const RunView MF = get(rf);
-                    run_fill(S, s, MF, run_of(*MF.G, rf), f ^ 2);
+                const int of = f < 2 ? ord : ord ^ 1;
+                if (S.run[of].y & 511) {
+                    run_fill(S, s, of, get(S.run[of]), f ^ 2);
                 } else if (f == 2 && lane == 0) {
                     mbar_expect(smem_addr(&S.full[0]), 0);  // wakes the block to leave
                 }
             }
             if (f == 0) {
                 // the closure, the moments, the polynomial that the four fields share
-                if (N.act) {
-                    if (inlet) {
+                if (act()) {
+                    if (inlet()) {
                         BCtx<F64> c{};
                         c.uin1 = M.uin1;
                         c.uin2 = M.uin2;
                         c.G = M.G;
                         c.P = M.P;
                         decode(*M.G, g, c.b, c.i, c.j, c.k);
-                        closure_face<F64>(c, N.cls, 0, v);
-                    } else if (N.cls >= 0) {
-                        wall_flow_closure(N.cls, P.rho_out, v);
+                        closure_face<F64>(c, cls(), 0, v);
+                    } else if (cls() >= 0) {
+                        wall_flow_closure(cls(), P.rho_out, v);
                     }
                     r = sum19(v);
                     // the outlet row's density is pinned to rho_out (Tmixer.cpp:9575-9582)
-                    if (N.cls == K_OUTLET) r = P.rho_out;
+                    if (cls() == K_OUTLET) r = P.rho_out;
                     double sxm, sym, szm;
                     momentum(v, sxm, sym, szm);
                     const double ux = sxm / r, uy = sym / r, uz = szm / r;
@@ -437,46 +444,45 @@ __device__ __forceinline__ void run_loop(const Get& get, const int4* __restrict_
                     if (next < nruns) cp_async16(&S.run[ord ^ 1], runs + next);
                     else S.run[ord ^ 1] = make_int4(0, 0, 1, 1);
                 }
-                par = parc;
             } else if (f != 2) {
-                if (inlet) {
+                if (inlet()) {
                     BCtx<F64> c{};
                     c.P = M.P;
-                    closure_face<F64>(c, N.cls, f, v);
+                    closure_face<F64>(c, cls(), f, v);
                 }
                 r = sum19(v);
             }
             if (f == 1) {
                 // B, of which the collision of A needs the sum
-                if (t == NT - 1) {
+                if (warp == kWarps - 1) {
                     cp_async_commit();
                     cp_async_wait_all();
+                    __syncwarp();
+                    if (S.run[ord ^ 1].y & 511) run_prepare(S, ord ^ 1, *get(S.run[ord ^ 1]).G);
                 }
                 if (!mbar_wait(smem_addr(&S.full[0]), 1)) {
                     *error = 1;
                     return;
                 }
-                double* __restrict__ rb = &S.slot[0][t + N.xs];
-                if (inlet) {
-                    run_inlet_species<NT>(rb, par, N.cls, P.cin[1][N.cls == K_INLET2]);
+                double* __restrict__ rb = &S.slot[0][t + ((what >> 1) & 3) - 1];
+                if (inlet()) {
+                    run_inlet_species<NT>(rb, S.par[ord][1], cls(), P.cin[1][cls() == K_INLET2]);
                     // (written here, filled again by a bulk copy)
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 }
-                cb = run_sum<NT>(rb, par);
+                cb = run_sum<NT>(rb, S.par[ord][1]);
                 rt = P.rateconst * r * cb;
-                m = -1.0;
             } else if (f == 2) {
                 r = cb;
-            } else if (f == 3) {
-                m = 2.0;
             }
-            if (N.act) {
+            if (act()) {
                 // densities the closures read next step: the faces', and those
                 // of the interior nodes beside the junction edges
                 // (Tmixer.cpp:8609, :8851)
-                if (N.cls != -1) M.rcur[f * ps + g] = r;
+                if (cls() != -1) M.rcur[f * ps + g] = r;
                 if (write_macro) M.mac[(f ? 3 + f : 0) * ps + g] = r;
                 const double c1 = P.c1[f], c2 = P.c2[f];
+                const double m = f == 0 ? -0.0 : (f == 3 ? 2.0 : -1.0);
                 const double w0 = f ? (wq(0) * rt) * m : m, w1 = f ? (wq(1) * rt) * m : m, w2 = f ? (wq(7) * rt) * m : m;
                 if (tiny_density(r))
                     run_collide_exact(p, ps, v, r, poly, c1, c2, w0, w1, w2);
