@@ -95,9 +95,9 @@ struct tmx_handle {
 };
 
 const StepKernels tmx_host::kForms[3] = {
-    {tmx::k_init_f64, nullptr, nullptr, nullptr, {tmx::k_run128_f64, tmx::k_run256_f64}, 8, 8, false, true},
-    {tmx::k_init_f32, tmx::k_bulk_f32, tmx::k_bfaces_f32, tmx::k_bedges_f32, {nullptr, nullptr}, 4, 4, false, false},
-    {tmx::k_init_f16, tmx::k_bulk_f16, tmx::k_bfaces_f16, tmx::k_bedges_f16, {nullptr, nullptr}, 2, 4, true, false},
+    {tmx::k_init_f64, nullptr, nullptr, nullptr, {tmx::k_run128_f64, tmx::k_run256_f64}, 8, 8, false},
+    {tmx::k_init_f32, tmx::k_bulk_f32, tmx::k_bfaces_f32, tmx::k_bedges_f32, {nullptr, nullptr}, 4, 4, false},
+    {tmx::k_init_f16, tmx::k_bulk_f16, tmx::k_bfaces_f16, tmx::k_bedges_f16, {nullptr, nullptr}, 2, 4, true},
 };
 
 namespace tmx_host {

@@ -53,8 +53,7 @@ struct BatchKernels {
     BoundaryBatchFn faces, edges;
 };
 const BatchKernels kBatchForms[3] = {
-    {{tmx::k_bulk_batch128_f64, tmx::k_bulk_batch256_f64, tmx::k_bulk_batch512_f64}, tmx::k_bfaces_batch_f64,
-     tmx::k_bedges_batch_f64},
+    {{nullptr, nullptr, nullptr}, nullptr, nullptr},  // FP64: k_run_batch_f64
     {{tmx::k_bulk_batch128_f32, tmx::k_bulk_batch256_f32, tmx::k_bulk_batch512_f32}, tmx::k_bfaces_batch_f32,
      tmx::k_bedges_batch_f32},
     {{tmx::k_bulk_batch128_f16, tmx::k_bulk_batch256_f16, tmx::k_bulk_batch512_f16}, tmx::k_bfaces_batch_f16,
@@ -205,7 +204,10 @@ struct tmx_batch {
     int cap_faces = 0;
     int2* d_edges = nullptr;
     int cap_edges = 0;
-    int* d_counts = nullptr;
+    int* d_counts = nullptr;  // kCounts ints (tmx_kernels.cuh)
+    int4* d_runs = nullptr;   // FP64 form: runs of every mixer
+    int cap_runs = 0;
+    int* error = nullptr;     // FP64 form: set by a step whose copies did not arrive (error_flag_take)
     int* d_slots = nullptr;
     double* d_im = nullptr;
     int* d_flags = nullptr;  // per-slot health flags (tmx_batch_health)
@@ -226,7 +228,7 @@ struct tmx_batch {
     int sms = 148;
     int grid_bulk[3] = {0, 0, 0};
     int grid_sweep[4] = {0, 0, 0, 0};  // by TMX_SHAPE_SWEEP* kind
-    int grid_faces = 0, grid_edges = 0;
+    int grid_faces = 0, grid_edges = 0, grid_run = 0;
     int nblocks = 0, nfaces = 0, nedges = 0, ntiles = 0, nactive = 0;
     cudaGraphExec_t graph[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
 };
@@ -292,7 +294,8 @@ MixerDesc desc_of(const tmx_batch* b, const Slot& s)
 int rebuild(tmx_batch* b)
 {
     std::vector<MixerDesc> desc(b->slots.size());
-    std::vector<int4> blocks, tiles;
+    std::vector<int4> blocks, tiles, runs;
+    const bool fp64 = b->precision == TMX_FP64;
     std::vector<int2> faces, edges;
     int nactive = 0;
     for (size_t m = 0; m < b->slots.size(); m++) {
@@ -302,10 +305,12 @@ int rebuild(tmx_batch* b)
         desc[m] = desc_of(b, s);
         for (int g0 = 0; g0 < s.G.nnodes; g0 += b->cells)
             blocks.push_back(make_int4((int)m, g0, std::min(b->cells, s.G.nnodes - g0), 0));
+        if (fp64) step_runs(s.G, (int)m, tmx::kRunBatchThreads, runs);
         if (b->sweep) sweep_tiles(s.G, (int)m, sweep_shape(b->sweep)->ty, b->zchunk, tiles);
         // with a sweep shape the interior kernel updates the z wall faces,
         // the last nzwall of the face range (zwall_node)
-        const int nfk = b->sweep ? s.nface - s.nzwall : s.nface;
+        // (and the FP64 form's runs every face)
+        const int nfk = fp64 ? 0 : (b->sweep ? s.nface - s.nzwall : s.nface);
         for (size_t t = 0; t < s.nodes.size(); t++) {
             const int2 e = make_int2(s.nodes[t], (int)m * 256 + s.cls[t]);
             if ((int)t < s.nface) {
@@ -325,6 +330,7 @@ int rebuild(tmx_batch* b)
     if (e == cudaSuccess) e = grow(b, b->d_faces, b->cap_faces, (int)std::max<size_t>(1, faces.size()));
     if (e == cudaSuccess) e = grow(b, b->d_edges, b->cap_edges, (int)std::max<size_t>(1, edges.size()));
     if (e == cudaSuccess) e = grow(b, b->d_tiles, b->cap_tiles, (int)std::max<size_t>(1, tiles.size()));
+    if (e == cudaSuccess) e = grow(b, b->d_runs, b->cap_runs, (int)std::max<size_t>(1, runs.size()));
     if (e != cudaSuccess) {
         cudaGetLastError();
         return fail(e == cudaErrorMemoryAllocation ? TMX_E_NOMEM : TMX_E_CUDA, "batch tables: %s",
@@ -340,7 +346,9 @@ int rebuild(tmx_batch* b)
     if (!faces.empty()) TMX_CK(cudaMemcpyAsync(b->d_faces, faces.data(), faces.size() * sizeof(int2), h2d, b->stream));
     if (!edges.empty()) TMX_CK(cudaMemcpyAsync(b->d_edges, edges.data(), edges.size() * sizeof(int2), h2d, b->stream));
     if (!tiles.empty()) TMX_CK(cudaMemcpyAsync(b->d_tiles, tiles.data(), tiles.size() * sizeof(int4), h2d, b->stream));
-    const int counts[4] = {(int)blocks.size(), (int)faces.size(), (int)edges.size(), (int)tiles.size()};
+    if (!runs.empty()) TMX_CK(cudaMemcpyAsync(b->d_runs, runs.data(), runs.size() * sizeof(int4), h2d, b->stream));
+    const int counts[5] = {(int)blocks.size(), (int)faces.size(), (int)edges.size(), (int)tiles.size(),
+                           (int)runs.size()};
     TMX_CK(cudaMemcpyAsync(b->d_counts, counts, sizeof counts, h2d, b->stream));
     TMX_CK(cudaStreamSynchronize(b->stream));
     b->nblocks = counts[0];
@@ -358,6 +366,25 @@ int rebuild(tmx_batch* b)
 // alone (tmx_batch_step_timed).
 int enqueue(tmx_batch* b, int parity, int write_macro, cudaEvent_t* ev = nullptr)
 {
+    if (b->precision == TMX_FP64) {
+        auto launch = [&](int what) {
+            tmx::k_run_batch_f64<<<b->grid_run, tmx::kRunBatchThreads, tmx::run_smem_host(tmx::kRunBatchThreads),
+                                   b->stream>>>(b->d_desc, b->d_runs, b->d_edges, b->d_counts, parity, write_macro,
+                                                what, b->error);
+        };
+        if (ev) {
+            TMX_CK(cudaEventRecord(ev[2], b->stream));
+            launch(2);
+            TMX_CK(cudaEventRecord(ev[3], b->stream));
+            TMX_CK(cudaEventRecord(ev[0], b->stream));
+            launch(1);
+            TMX_CK(cudaEventRecord(ev[1], b->stream));
+        } else {
+            launch(3);
+        }
+        TMX_CK(cudaGetLastError());
+        return TMX_OK;
+    }
     TMX_CK(cudaEventRecord(b->fork, b->stream));
     TMX_CK(cudaStreamWaitEvent(b->aux, b->fork, 0));
     TMX_CK(cudaStreamWaitEvent(b->aux2, b->fork, 0));
@@ -371,9 +398,8 @@ int enqueue(tmx_batch* b, int parity, int write_macro, cudaEvent_t* ev = nullptr
         TMX_CK(cudaEventRecord(ev[3], b->aux));
     }
     TMX_CK(cudaEventRecord(b->join, b->aux));
-    // in order for FP64, side by side for the reduced-precision forms (as the
-    // single-mixer step; StepKernels::serial)
-    if (b->K->serial || b->bound_after || ev) {
+    // side by side unless bound_after
+    if (b->bound_after || ev) {
         TMX_CK(cudaStreamWaitEvent(b->stream, b->join, 0));
         TMX_CK(cudaStreamWaitEvent(b->stream, b->join2, 0));
     }
@@ -386,7 +412,7 @@ int enqueue(tmx_batch* b, int parity, int write_macro, cudaEvent_t* ev = nullptr
             b->d_desc, b->d_blocks, b->d_counts, parity, write_macro);
     TMX_CK(cudaGetLastError());
     if (ev) TMX_CK(cudaEventRecord(ev[1], b->stream));
-    if (!b->K->serial && !b->bound_after && !ev) {
+    if (!b->bound_after && !ev) {
         TMX_CK(cudaStreamWaitEvent(b->stream, b->join, 0));
         TMX_CK(cudaStreamWaitEvent(b->stream, b->join2, 0));
     }
@@ -420,6 +446,20 @@ int step_one(tmx_batch* b, int write_macro)
 
 void set_grids(tmx_batch* b)
 {
+    if (b->precision == TMX_FP64) {
+        // one launch of as many blocks as fit; bound_bps only shows in the shape
+        const void* k = (const void*)tmx::k_run_batch_f64;
+        const int smem = tmx::run_smem_host(tmx::kRunBatchThreads);
+        cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        int per = 1;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, tmx::kRunBatchThreads, smem);
+        cudaGetLastError();
+        b->bound_fit = per = std::max(1, per);
+        b->grid_run = b->sms * per;
+        b->grid_faces = b->sms * (b->bound_bps > 0 ? std::min(b->bound_bps, per) : per);
+        return;
+    }
     for (int v = 0; v < 3; v++) {
         int per = 1;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)b->B->bulk[v], kBulkThreads[v], 0);
@@ -470,6 +510,14 @@ int init_slot(tmx_batch* b, Slot& s)
     return TMX_OK;
 }
 
+// After the stream has been waited for: whether every step's copies arrived.
+int settled(const tmx_batch* b)
+{
+    if (b->error && *(volatile int*)b->error)
+        return fail(TMX_E_CUDA, "a step of the FP64 batch gave up waiting for its copies: the state is not valid");
+    return TMX_OK;
+}
+
 bool valid_slot(const tmx_batch* b, int slot) { return slot >= 0 && slot < (int)b->slots.size() && b->slots[slot].used; }
 
 }  // namespace
@@ -511,8 +559,9 @@ int tmx_batch_create(int precision, long long budget_bytes, int device, tmx_batc
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->join, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->join2, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&b->d_counts, 4 * sizeof(int));
-    if (e == cudaSuccess) e = cudaMemset(b->d_counts, 0, 4 * sizeof(int));
+    if (e == cudaSuccess) e = cudaMalloc((void**)&b->d_counts, tmx::kCounts * sizeof(int));
+    if (e == cudaSuccess) e = cudaMemset(b->d_counts, 0, tmx::kCounts * sizeof(int));
+    if (e == cudaSuccess && precision == TMX_FP64 && !(b->error = error_flag_take())) e = cudaErrorMemoryAllocation;
     if (e != cudaSuccess) {
         cudaGetLastError();
         tmx_batch_destroy(b);
@@ -648,6 +697,7 @@ int tmx_batch_checkpoint(tmx_batch* b, int slot, void* buf, long long bytes)
         return fail(TMX_E_INVALID, "checkpoint buffer of %lld bytes, %lld needed", bytes, checkpoint_total(sec));
     TMX_CK(cudaSetDevice(b->device));
     TMX_CK(cudaStreamSynchronize(b->stream));
+    if (const int rc = settled(b)) return rc;
     CheckpointHeader hd{};
     std::memcpy(hd.magic, kCheckpointMagic, 8);
     hd.abi = TMX_ABI_VERSION;
@@ -719,7 +769,7 @@ int tmx_batch_sync(tmx_batch* b)
     if (!b) return fail(TMX_E_INVALID, "null batch");
     TMX_CK(cudaSetDevice(b->device));
     TMX_CK(cudaStreamSynchronize(b->stream));
-    return TMX_OK;
+    return settled(b);
 }
 
 int tmx_batch_slots(const tmx_batch* b, int* slots, int cap, int* n)
@@ -768,7 +818,7 @@ int tmx_batch_outlet_im(tmx_batch* b, const int* slots, int n, double* im_out)
     TMX_CK(cudaGetLastError());
     TMX_CK(cudaMemcpyAsync(im_out, b->d_im, (size_t)n * 3 * sizeof(double), cudaMemcpyDeviceToHost, b->stream));
     TMX_CK(cudaStreamSynchronize(b->stream));
-    return TMX_OK;
+    return settled(b);
 }
 
 int tmx_batch_health(tmx_batch* b, const int* slots, int n, int* bad)
@@ -798,7 +848,7 @@ int tmx_batch_health(tmx_batch* b, const int* slots, int n, int* bad)
     TMX_CK(cudaMemcpyAsync(flags.data(), b->d_flags, flags.size() * sizeof(int), cudaMemcpyDeviceToHost, b->stream));
     TMX_CK(cudaStreamSynchronize(b->stream));
     for (int e = 0; e < n; e++) bad[e] = flags[(size_t)slots[e]];
-    return TMX_OK;
+    return settled(b);
 }
 
 int tmx_batch_fields(tmx_batch* b, int slot, int box, int field, double* host_out)
@@ -814,6 +864,7 @@ int tmx_batch_fields(tmx_batch* b, int slot, int box, int field, double* host_ou
     const size_t n = (size_t)nx * ny * nz;
     std::vector<double> stage(n);
     TMX_CK(cudaStreamSynchronize(b->stream));
+    if (const int rc = settled(b)) return rc;
     TMX_CK(cudaMemcpy(stage.data(), s.mac + (size_t)field * G.ps + G.base[box], n * sizeof(double),
                       cudaMemcpyDeviceToHost));
     for (int k = 0; k < nz; k++)
@@ -890,7 +941,7 @@ int tmx_batch_boundary(const tmx_batch* b, int* blocks_per_sm, int* after)
 {
     if (!b || !blocks_per_sm) return fail(TMX_E_INVALID, "null argument");
     *blocks_per_sm = b->grid_faces / std::max(1, b->sms);
-    if (after) *after = (b->K->serial || b->bound_after) ? 1 : 0;
+    if (after) *after = (b->precision == TMX_FP64 || b->bound_after) ? 1 : 0;
     return TMX_OK;
 }
 
@@ -931,7 +982,9 @@ int tmx_batch_tune(tmx_batch* b, int steps_per_trial, int* threads_out, int* cel
         cudaEventElapsedTime(&ms, t0, t1);
         ms_step = ms / steps_per_trial;
     };
-    for (int v = 0; v < 3 && rc == TMX_OK; v++)
+    // the FP64 form has one kernel: its shape stays as it is
+    if (b->precision == TMX_FP64) trial(best);
+    for (int v = 0; v < 3 && rc == TMX_OK && b->precision != TMX_FP64; v++)
         for (int ci = 0; ci < 4 && rc == TMX_OK; ci++) {
             const int cells = kCellChoices[ci];
             if (cells < kBulkThreads[v]) continue;
@@ -966,7 +1019,7 @@ int tmx_batch_tune(tmx_batch* b, int steps_per_trial, int* threads_out, int* cel
     if (rc == TMX_OK) rc = tmx_batch_set_shape(b, kBulkThreads[bv], bc);
     if (rc == TMX_OK && bs) rc = tmx_batch_set_sweep(b, bs, bz);
     const int bchoices[4] = {1, 2, 4, 0};
-    for (int after = 0; after < (b->K->serial ? 1 : 2) && rc == TMX_OK; after++)
+    for (int after = 0; after < (b->precision == TMX_FP64 ? 0 : 2) && rc == TMX_OK; after++)
         for (int i = 0; i < 4 && rc == TMX_OK; i++) {
             if (bchoices[i] >= b->bound_fit) continue;  // the same grid as 0
             rc = tmx_batch_set_boundary(b, bchoices[i], after);
@@ -1088,6 +1141,8 @@ void tmx_batch_destroy(tmx_batch* b)
     cudaFree(b->d_edges);
     cudaFree(b->d_tiles);
     cudaFree(b->d_counts);
+    cudaFree(b->d_runs);
+    error_flag_give(b->error);
     cudaFree(b->d_slots);
     cudaFree(b->d_im);
     cudaFree(b->d_flags);

@@ -549,97 +549,6 @@ __device__ __forceinline__ int bulk_src(const Geom& G, int g, int i, int k, int 
     return g - (EX(q) + EY(q) * sy + EZ(q) * sz);
 }
 
-template <class PR>
-__device__ __forceinline__ void bulk_load(const typename PR::S* __restrict__ Pin, const float4* __restrict__ M,
-                                          long long ps, int fld, const Geom& G, int g, int i, int k, int sy, int sz,
-                                          int iface, typename PR::T (&v)[19])
-{
-#pragma unroll
-    for (int q = 0; q < 19; q++) {
-        const int src = bulk_src(G, g, i, k, sy, sz, iface, q);
-        v[q] = PR::decode(Pin + PR::off(fld, q, ps, src), fld, q, M, ps, src);
-    }
-}
-
-// One interior node; boundary nodes are left to the boundary kernels.
-template <class PR>
-__device__ __forceinline__ void bulk_node(const StepPtrs& X, const Geom& G, const Phys& P, int write_macro, int g)
-{
-    using T = typename PR::T;
-    const typename PR::S* __restrict__ Pin = (const typename PR::S*)X.pin;
-    typename PR::S* __restrict__ Pout = (typename PR::S*)X.pout;
-    const float4* __restrict__ M = X.mprev;
-    const long long ps = G.ps;
-    int b, i, j, k;
-    decode(G, g, b, i, j, k);
-    if (is_boundary(G, b, i, j, k)) return;
-    const int sy = box_nx(G, b), sz = box_nx(G, b) * box_ny(G, b);
-    const int iface = (b == 0 && j == 1) ? 1 : ((b == 1 && j == G.mny) ? 2 : 0);
-
-    // flow: moments, equilibrium polynomial (shared by all four fields: they
-    // use the flow velocity, Tmixer.cpp:1602-1830), collision
-    T poly[19];
-    T rho, ux, uy, uz;
-    {
-        T f[19];
-        bulk_load<PR>(Pin, M, ps, 0, G, g, i, k, sy, sz, iface, f);
-        rho = sum19(f);
-        T sxm, sym, szm;
-        momentum(f, sxm, sym, szm);
-        ux = sxm / rho;
-        uy = sym / rho;
-        uz = szm / rho;
-        PR::poly(ux, uy, uz, poly);
-        collide_store<PR>(Pout, ps, g, 0, f, rho, poly, P, T(0));
-    }
-    // species A and B: the reaction needs both densities before either
-    // collides, so their populations are loaded twice (the second time from
-    // cache) rather than held in registers
-    T ca, cb;
-    {
-        T a[19];
-        bulk_load<PR>(Pin, M, ps, 1, G, g, i, k, sy, sz, iface, a);
-        ca = sum19(a);
-        bulk_load<PR>(Pin, M, ps, 2, G, g, i, k, sy, sz, iface, a);
-        cb = sum19(a);
-    }
-    const T rt = T(P.rateconst) * ca * cb;
-    T cc;
-    {
-        T a[19];
-        bulk_load<PR>(Pin, M, ps, 1, G, g, i, k, sy, sz, iface, a);
-        collide_store<PR>(Pout, ps, g, 1, a, ca, poly, P, rt);
-        bulk_load<PR>(Pin, M, ps, 2, G, g, i, k, sy, sz, iface, a);
-        collide_store<PR>(Pout, ps, g, 2, a, cb, poly, P, rt);
-        bulk_load<PR>(Pin, M, ps, 3, G, g, i, k, sy, sz, iface, a);
-        cc = sum19(a);
-        collide_store<PR>(Pout, ps, g, 3, a, cc, poly, P, rt);
-    }
-    // densities the junction edges read next step (Tmixer.cpp:8609, :8851)
-    if (b == 0 && j == 2 && (i == G.ia || i == G.ib)) {
-        T* Rcur = (T*)X.rcur;
-        Rcur[g] = rho;
-        Rcur[ps + g] = ca;
-        Rcur[2 * ps + g] = cb;
-        Rcur[3 * ps + g] = cc;
-    }
-    if (PR::kMoments) {
-        X.mcur[2 * (long long)g] = make_float4((float)rho, (float)ca, (float)cb, (float)cc);
-        X.mcur[2 * (long long)g + 1] =
-            make_float4((float)ux, (float)uy, (float)uz, omt_term((float)ux, (float)uy, (float)uz));
-    }
-    if (write_macro) {
-        double* Mac = X.mac;
-        Mac[g] = rho;
-        Mac[ps + g] = ux;
-        Mac[2 * ps + g] = uy;
-        Mac[3 * ps + g] = uz;
-        Mac[4 * ps + g] = ca;
-        Mac[5 * ps + g] = cb;
-        Mac[6 * ps + g] = cc;
-    }
-}
-
 // Writer records of the FP16 form for lp_interior: read from global memory at
 // the source node (the flat bulk kernel) ...
 struct RecGlobal {
@@ -1697,22 +1606,6 @@ __device__ __forceinline__ void face_copy_offset(int cls, int& di, int& dj, int&
     }
 }
 
-template <class PR, bool FACES>
-__device__ __forceinline__ void closed_pull(const BCtx<PR>& c, int cls, int fld, typename PR::T (&v)[19])
-{
-    // one pull for the four lanes, the species lanes of a copy class from
-    // the interior neighbour: the warp runs the 19 pulls once, not once per
-    // branch
-    int di = 0, dj = 0, dk = 0;
-    if (FACES && fld > 0) face_copy_offset(cls, di, dj, dk);
-    pull_node(c, fld, c.b, c.i + di, c.j + dj, c.k + dk, v);
-    if (di | dj | dk) return;
-    if (FACES)
-        closure_face(c, cls, fld, v);
-    else
-        closure_edge(c, cls, fld, v);
-}
-
 // ---------------------------------------------------------------------------
 // boundary nodes of a compact, class-sorted list, four threads per node: lane
 // fld (0 flow, 1 A, 2 B, 3 C) pulls, closes and collides its own field.  Every
@@ -1723,71 +1616,6 @@ __device__ __forceinline__ void closed_pull(const BCtx<PR>& c, int cls, int fld,
 // ---------------------------------------------------------------------------
 constexpr int kBoundaryThreads = 128;
 constexpr int kBoundaryLanes = 4;
-
-// Lane fld of boundary node g (class cls); mask holds the active lanes of
-// the warp and lead the first lane of this node's group of four.
-template <class PR, bool FACES>
-__device__ __forceinline__ void boundary_lane(const StepPtrs& X, const Geom& G, const Phys& P, int write_macro, int g,
-                                              int cls, int fld, unsigned mask, int lead)
-{
-    using T = typename PR::T;
-    typename PR::S* __restrict__ Pout = (typename PR::S*)X.pout;
-    T* __restrict__ Rcur = (T*)X.rcur;
-    double* __restrict__ Mac = X.mac;
-    BCtx<PR> c;
-    c.Pin = (const typename PR::S*)X.pin;
-    c.M = X.mprev;
-    c.Rprev = (const T*)X.rprev;
-    c.uin1 = (const T*)X.uin1;
-    c.uin2 = (const T*)X.uin2;
-    c.G = &G;
-    c.P = &P;
-    c.ps = G.ps;
-    c.g = g;
-    decode(G, c.g, c.b, c.i, c.j, c.k);
-    const long long ps = G.ps;
-
-    T v[19];
-    closed_pull<PR, FACES>(c, cls, fld, v);
-    T r = sum19(v);
-    T ux = T(0), uy = T(0), uz = T(0);
-    if (fld == 0) {
-        // the outlet row's density is pinned to rho_out (Tmixer.cpp:9575-9582)
-        if (c.b == 1 && c.j == 1) r = T(P.rho_out);
-        T sxm, sym, szm;
-        momentum(v, sxm, sym, szm);
-        ux = sxm / r;
-        uy = sym / r;
-        uz = szm / r;
-    }
-    ux = __shfl_sync(mask, ux, lead);
-    uy = __shfl_sync(mask, uy, lead);
-    uz = __shfl_sync(mask, uz, lead);
-    const T rho = __shfl_sync(mask, r, lead);
-    const T ca = __shfl_sync(mask, r, lead + 1);
-    const T cb = __shfl_sync(mask, r, lead + 2);
-    const T cc = __shfl_sync(mask, r, lead + 3);
-    T poly[19];
-    PR::poly(ux, uy, uz, poly);
-    const T rt = fld == 0 ? T(0) : T(P.rateconst) * ca * cb;
-    collide_store<PR>(Pout, ps, c.g, fld, v, r, poly, P, rt);
-
-    Rcur[fld * ps + c.g] = r;
-    if (PR::kMoments) {
-        if (fld == 0) X.mcur[2 * (long long)c.g] = make_float4((float)rho, (float)ca, (float)cb, (float)cc);
-        if (fld == 1)
-            X.mcur[2 * (long long)c.g + 1] =
-                make_float4((float)ux, (float)uy, (float)uz, omt_term((float)ux, (float)uy, (float)uz));
-    }
-    if (write_macro) {
-        Mac[(fld == 0 ? 0 : 3 + fld) * ps + c.g] = r;
-        if (fld == 0) {
-            Mac[ps + c.g] = ux;
-            Mac[2 * ps + c.g] = uy;
-            Mac[3 * ps + c.g] = uz;
-        }
-    }
-}
 
 // Direction 4K + lane of a group of four lanes (K a compile-time constant,
 // lane a run-time value): its lattice vector and weight, selected from the
@@ -1945,21 +1773,6 @@ __device__ __forceinline__ void boundary_lane_lp(const StepPtrs& X, const Geom& 
     }
 }
 
-// Lane fld of boundary node g in the form's scheme: directions split across
-// the lanes for the interleaved forms (buf: the node's 76 values of shared
-// memory); one field per lane for FP64, whose SoA planes give the direction
-// split no saving and whose larger code then stalls on instruction fetch
-// (65.5 us against 59.6 us for the W=32 faces).
-template <class PR, bool FACES>
-__device__ __forceinline__ void boundary_any(const StepPtrs& X, const Geom& G, const Phys& P, int write_macro, int g,
-                                             int cls, int fld, unsigned mask, int lead, typename PR::T* buf)
-{
-    if constexpr (PR::kOnePass)
-        boundary_lane_lp<PR, FACES>(X, G, P, write_macro, g, cls, fld, mask, lead, buf);
-    else
-        boundary_lane<PR, FACES>(X, G, P, write_macro, g, cls, fld, mask, lead);
-}
-
 // One launch over a node list: thread 4t + fld is lane fld of node t.
 template <class PR, bool FACES>
 __device__ __forceinline__ void boundary_node(const StepPtrs& X, const int* __restrict__ bnode,
@@ -1971,19 +1784,8 @@ __device__ __forceinline__ void boundary_node(const StepPtrs& X, const int* __re
     // the four lanes of a node share one warp; whole nodes drop out together
     const unsigned mask = __ballot_sync(0xffffffffu, t < nb);
     if (t >= nb) return;
-    boundary_any<PR, FACES>(X, G, P, write_macro, bnode[t], bcls[t], fld, mask, (threadIdx.x & 31) & ~3,
+    boundary_lane_lp<PR, FACES>(X, G, P, write_macro, bnode[t], bcls[t], fld, mask, (threadIdx.x & 31) & ~3,
                             buf[threadIdx.x >> 2]);
-}
-
-// One interior node in the form's bulk scheme: one pass over the 76 values
-// for the interleaved layouts, field by field for FP64.
-template <class PR>
-__device__ __forceinline__ void bulk_any(const StepPtrs& X, const Geom& G, const Phys& P, int write_macro, int g)
-{
-    if constexpr (PR::kOnePass)
-        bulk_node_lp<PR>(X, G, P, write_macro, g);
-    else
-        bulk_node<PR>(X, G, P, write_macro, g);
 }
 
 // Kernel definitions for one precision policy; NAME is the kernel-name suffix.
@@ -1998,7 +1800,7 @@ __device__ __forceinline__ void bulk_any(const StepPtrs& X, const Geom& G, const
     __global__ void __launch_bounds__(256, 2) k_bulk_##NAME(StepPtrs X, Geom G, Phys P, int write_macro)        \
     {                                                                                                           \
         for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < G.nnodes; g += gridDim.x * blockDim.x)          \
-            bulk_any<PR>(X, G, P, write_macro, g);                                                              \
+            bulk_node_lp<PR>(X, G, P, write_macro, g);                                                              \
     }
 
 // A batched kernel's block works on one mixer at a time (a sweep tile, 32
@@ -2067,13 +1869,13 @@ __device__ __forceinline__ void load_desc(StepDesc& dst, const MixerDesc* __rest
     __global__ void __launch_bounds__(kBoundaryThreads) k_bfaces_##NAME(                                       \
         StepPtrs X, const int* bnode, const unsigned char* bcls, int nb, Geom G, Phys P, int write_macro)       \
     {                                                                                                           \
-        __shared__ PR::T buf[PR::kOnePass ? kBoundaryThreads / 4 : 1][76];                                      \
+        __shared__ PR::T buf[kBoundaryThreads / 4][76];                                                         \
         boundary_node<PR, true>(X, bnode, bcls, nb, G, P, write_macro, buf, blockIdx.x);                        \
     }                                                                                                           \
     __global__ void __launch_bounds__(kBoundaryThreads) k_bedges_##NAME(                                       \
         StepPtrs X, const int* bnode, const unsigned char* bcls, int nb, Geom G, Phys P, int write_macro)       \
     {                                                                                                           \
-        __shared__ PR::T buf[PR::kOnePass ? kBoundaryThreads / 4 : 1][76];                                      \
+        __shared__ PR::T buf[kBoundaryThreads / 4][76];                                                         \
         boundary_node<PR, false>(X, bnode, bcls, nb, G, P, write_macro, buf, blockIdx.x);                       \
     }
 
@@ -2087,22 +1889,22 @@ __device__ __forceinline__ void load_desc(StepDesc& dst, const MixerDesc* __rest
         for (int b = blockIdx.x; b < nblk; b += gridDim.x) {                                                    \
             const int4 cb = blocks[b];                                                                          \
             const MixerDesc& d = D[cb.x];                                                                       \
-            for (int t = threadIdx.x; t < cb.z; t += NT) bulk_any<PR>(d.X[parity], d.G, d.P, write_macro, cb.y + t); \
+            for (int t = threadIdx.x; t < cb.z; t += NT) bulk_node_lp<PR>(d.X[parity], d.G, d.P, write_macro, cb.y + t); \
         }                                                                                                       \
     }
 // The batched boundary kernels hold the shared descriptor's values in
 // registers; their register counts are held to those of the global-descriptor
-// build (72 and 80 for the interleaved forms' faces and edges, 128 for FP64),
-// which kept them at 7, 6 and 4 blocks per SM: the 4-mixer FP16 sweep step
+// build (72 and 80 for faces and edges),
+// which kept them at 7 and 6 blocks per SM: the 4-mixer FP16 sweep step
 // took 511-517 us capped against 528-533 us uncapped.
 #define TMX_BOUNDARY_BATCH(PR, NAME, KIND, FACES, WHICH)                                                          \
-    __global__ void __launch_bounds__(kBoundaryThreads, PR::kOnePass ? (FACES ? 7 : 6) : 4)                    \
+    __global__ void __launch_bounds__(kBoundaryThreads, FACES ? 7 : 6)                    \
         k_##KIND##_batch_##NAME(                                                                                \
         const MixerDesc* __restrict__ D, const int2* __restrict__ list, const int* __restrict__ counts,         \
         int parity, int write_macro)                                                                            \
     {                                                                                                           \
         const int n = counts[WHICH];                                                                            \
-        __shared__ PR::T buf[PR::kOnePass ? kBoundaryThreads / 4 : 1][76];                                      \
+        __shared__ PR::T buf[kBoundaryThreads / 4][76];                                                         \
         __shared__ StepDesc d;                                                                                  \
         for (int base = blockIdx.x * blockDim.x; base < 4 * n; base += gridDim.x * blockDim.x) {                \
             const int t = (base + threadIdx.x) >> 2, fld = threadIdx.x & 3;                                     \
@@ -2114,7 +1916,7 @@ __device__ __forceinline__ void load_desc(StepDesc& dst, const MixerDesc* __rest
             const bool live = e.x >= 0;                                                                         \
             const unsigned mask = __ballot_sync(0xffffffffu, live);                                             \
             if (live)                                                                                           \
-                boundary_any<PR, FACES>(d.X, d.G, d.P, write_macro, e.x, e.y & 255, fld, mask,                  \
+                boundary_lane_lp<PR, FACES>(d.X, d.G, d.P, write_macro, e.x, e.y & 255, fld, mask,                  \
                                         (threadIdx.x & 31) & ~3, buf[threadIdx.x >> 2]);                        \
         }                                                                                                       \
     }

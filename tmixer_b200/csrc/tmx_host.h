@@ -42,7 +42,6 @@ struct StepKernels {
     void (*run[2])(tmx::StepPtrs, Geom, Phys, int, const int4*, int, const int*, const unsigned char*, int, int*, int, int*);
     int sbytes, tbytes;
     bool moments;  // the form stores per-node FP32 moments next to the populations
-    bool serial;   // the bulk kernel runs after the boundary kernels, not beside them
 };
 extern const StepKernels kForms[3];
 

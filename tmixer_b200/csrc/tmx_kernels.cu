@@ -42,7 +42,35 @@ __device__ __forceinline__ void run_step(const StepPtrs& X, const Geom& G, const
     }
 TMX_DEFINE_RUN(128)
 TMX_DEFINE_RUN(256)
-TMX_DEFINE_BATCH_KERNELS(F64, f64)
+
+// The FP64 step of a batch: the runs and edges of every mixer in one launch;
+// counts[4] runs, counts[2] edge entries, counts[5 + parity] hands out the runs.
+// what: 1 the runs, 2 the edges, 3 both.
+__global__ void __launch_bounds__(kRunBatchThreads, 512 / kRunBatchThreads) k_run_batch_f64(
+    const MixerDesc* __restrict__ D, const int4* __restrict__ runs, const int2* __restrict__ edges,
+    int* __restrict__ counts, int parity, int write_macro, int what, int* error)
+{
+    constexpr int NT = kRunBatchThreads;
+    extern __shared__ __align__(16) unsigned char run_smem[];
+    RunShared<NT>& S = *(RunShared<NT>*)run_smem;
+    const int warp = threadIdx.x >> 5, nb = gridDim.x;
+    const int nruns = what & 1 ? counts[4] : 0, ne = what & 2 ? counts[2] : 0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) counts[5 + (1 - parity)] = 0;  // the next step's
+    run_loop<NT>(
+        [&](const int4& t) {
+            const MixerDesc& d = D[run_mixer(t)];
+            return run_view(d.X[parity], d.G, d.P);
+        },
+        runs, nruns, blockIdx.x, nb, counts + 5 + parity, write_macro, S, error, [&] {
+            const int at = (int)(blockIdx.x + nb - nruns % nb) % nb;
+            for (int e = at * (NT / 32) + warp; e < ne; e += nb * (NT / 32)) {
+                const int2 t = edges[e];
+                if (t.x < 0) continue;
+                const MixerDesc& d = D[t.y >> 8];
+                run_edge(d.X[parity], d.G, d.P, write_macro, t.x, t.y & 255, S.edge[warp]);
+            }
+        });
+}
 
 // ---------------------------------------------------------------------------
 // mixing quality (Tmixer.cpp:10161-10409): per row, per species, the sums of

@@ -76,8 +76,9 @@ struct MixerDesc {
 //   faces / edges   boundary-node lists of {node, mixer * 256 + class}, 
 //           four threads per node, persistent grid; each mixer's part
 //           starts at a multiple of kListAlign, padded with node -1.
-// counts[0..2] = number of cell blocks, face nodes, edge nodes (device
-// memory, so that captured graphs stay valid when the batch changes).
+// counts[0..4] = number of cell blocks, face nodes, edge nodes, sweep tiles,
+// runs (device memory, so that captured graphs stay valid when the batch
+// changes); counts[5..6] are the FP64 form's run counters.
 #define TMX_DECLARE_BATCH_KERNELS(NAME)                                                                           \
     __global__ void k_bulk_batch128_##NAME(const MixerDesc* D, const int4* blocks, const int* counts, int parity, \
                                            int write_macro);                                                      \
@@ -90,7 +91,11 @@ struct MixerDesc {
     __global__ void k_bedges_batch_##NAME(const MixerDesc* D, const int2* list, const int* counts, int parity,    \
                                           int write_macro);
 
-TMX_DECLARE_BATCH_KERNELS(f64)
+constexpr int kCounts = 7;
+// The FP64 form's batched step (runs as k_run128_f64's, of every mixer).
+constexpr int kRunBatchThreads = 128;
+__global__ void k_run_batch_f64(const MixerDesc* D, const int4* runs, const int2* edges, int* counts, int parity,
+                                int write_macro, int what, int* error);
 TMX_DECLARE_BATCH_KERNELS(f32)
 TMX_DECLARE_BATCH_KERNELS(f16)
 
