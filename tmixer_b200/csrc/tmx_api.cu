@@ -396,6 +396,17 @@ int boundary_list(const Geom& G, std::vector<int>& nodes, std::vector<unsigned c
     return TMX_OK;
 }
 
+int box_to_host(const Geom& G, int box, const double* dev, double* scratch, cudaStream_t stream, double* host_out)
+{
+    const int nx = G.nx[box], ny = G.ny[box], nz = G.nz;
+    const long long tiles = (long long)((nx + 31) / 32) * ((nz + 31) / 32) * ny;
+    tmx::k_box_ijk<<<(int)std::min(tiles, 148LL * 8), 256, 0, stream>>>(dev, nx, ny, nz, scratch);
+    TMX_CK(cudaGetLastError());
+    TMX_CK(cudaMemcpyAsync(host_out, scratch, (size_t)nx * ny * nz * sizeof(double), cudaMemcpyDeviceToHost, stream));
+    TMX_CK(cudaStreamSynchronize(stream));
+    return TMX_OK;
+}
+
 // The flags lie in one page of the process, mapped when the first is taken
 // (mapping memory takes about a millisecond, a handle's creation two); beyond
 // its 1024 a flag is mapped by itself.
@@ -1050,33 +1061,15 @@ int tmx_case_of(const tmx_handle* h, tmx_case* out)
     return TMX_OK;
 }
 
-// Copy n = nx*ny*nz doubles of one box from the device (x fastest) into host
-// memory in the reference's [i][j][k] order (k fastest).
-static int box_to_host(tmx_handle* h, int box, const double* dev, double* host_out, std::vector<double>& stage)
-{
-    const Geom& G = h->G;
-    const int nx = G.nx[box], ny = G.ny[box], nz = G.nz;
-    const size_t n = (size_t)nx * ny * nz;
-    stage.resize(n);
-    TMX_CK(cudaMemcpyAsync(stage.data(), dev + G.base[box], n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    TMX_CK(cudaStreamSynchronize(h->stream));
-    if (const int rc = settled(h)) return rc;
-    for (int k = 0; k < nz; k++)
-        for (int j = 0; j < ny; j++) {
-            const double* src = stage.data() + ((size_t)k * ny + j) * nx;
-            for (int i = 0; i < nx; i++) host_out[((size_t)i * ny + j) * nz + k] = src[i];
-        }
-    return TMX_OK;
-}
-
 int tmx_fields(tmx_handle* h, int box, int field, double* host_out)
 {
     if (!h || !host_out) return fail(TMX_E_INVALID, "null argument");
     if (box < 0 || box > 1 || field < 0 || field > 6) return fail(TMX_E_INVALID, "box %d / field %d out of range", box, field);
     if (!h->inited) return fail(TMX_E_STATE, "tmx_fields before tmx_init");
     TMX_CK(cudaSetDevice(h->device));
-    std::vector<double> stage;
-    return box_to_host(h, box, h->mac + (size_t)field * h->G.ps, host_out, stage);
+    const int rc = box_to_host(h->G, box, h->mac + (size_t)field * h->G.ps + h->G.base[box],
+                               (double*)h->pop[1 - h->cur], h->stream, host_out);
+    return rc ? rc : settled(h);
 }
 
 int tmx_populations(tmx_handle* h, int box, int fld, double* host_out)
@@ -1087,14 +1080,13 @@ int tmx_populations(tmx_handle* h, int box, int fld, double* host_out)
     TMX_CK(cudaSetDevice(h->device));
     const Geom& G = h->G;
     const size_t n = (size_t)G.nx[box] * G.ny[box] * G.nz;
-    std::vector<double> stage;
     if (h->sbytes == 8) {
         for (int q = 0; q < 19; q++) {
-            const double* src = (const double*)h->pop[h->cur] + (size_t)(fld * 19 + q) * G.ps;
-            int rc = box_to_host(h, box, src, host_out + q * n, stage);
+            const double* src = (const double*)h->pop[h->cur] + (size_t)(fld * 19 + q) * G.ps + G.base[box];
+            int rc = box_to_host(G, box, src, (double*)h->pop[1 - h->cur], h->stream, host_out + q * n);
             if (rc) return rc;
         }
-        return TMX_OK;
+        return settled(h);
     }
     // reduced precision: widen on the host; the FP16 form adds back feq of
     // the writing node's moments exactly as the kernels do (tmx_engine.cuh)

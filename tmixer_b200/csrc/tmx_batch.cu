@@ -860,17 +860,10 @@ int tmx_batch_fields(tmx_batch* b, int slot, int box, int field, double* host_ou
     TMX_CK(cudaSetDevice(b->device));
     const Slot& s = b->slots[slot];
     const Geom& G = s.G;
-    const int nx = G.nx[box], ny = G.ny[box], nz = G.nz;
-    const size_t n = (size_t)nx * ny * nz;
-    std::vector<double> stage(n);
-    TMX_CK(cudaStreamSynchronize(b->stream));
-    if (const int rc = settled(b)) return rc;
-    TMX_CK(cudaMemcpy(stage.data(), s.mac + (size_t)field * G.ps + G.base[box], n * sizeof(double),
-                      cudaMemcpyDeviceToHost));
-    for (int k = 0; k < nz; k++)
-        for (int j = 0; j < ny; j++)
-            for (int i = 0; i < nx; i++) host_out[((size_t)i * ny + j) * nz + k] = stage[((size_t)k * ny + j) * nx + i];
-    return TMX_OK;
+    // scratch: the population buffer that the next step writes
+    const int q = 1 - (b->parity ^ s.parity0);
+    const int rc = box_to_host(G, box, s.mac + (size_t)field * G.ps + G.base[box], (double*)s.pop[q], b->stream, host_out);
+    return rc ? rc : settled(b);
 }
 
 int tmx_batch_info(const tmx_batch* b, long long out[8])

@@ -179,6 +179,12 @@ inline void step_runs(const Geom& G, int mixer, int nt, std::vector<int4>& out)
     out.insert(out.end(), rest.begin(), rest.end());
 }
 
+// One field of a box from the device (first node dev, x fastest) to the host in
+// the reference's [i][j][k] order, by way of scratch: device memory of
+// a box's doubles that nothing else uses meanwhile (the population buffer that
+// the next step writes).  Waits for the stream.
+int box_to_host(const Geom& G, int box, const double* dev, double* scratch, cudaStream_t stream, double* host_out);
+
 // An int that kernels set when they give up (mapped host memory, 0 to begin
 // with), and its return; null when there is no memory.
 int* error_flag_take();

@@ -122,6 +122,9 @@ __global__ void k_outlet_im_batch(const MixerDesc* D, const int* slots, int n, d
 // written, over the batch's cell-block list (counts[0] blocks).
 __global__ void k_nonfinite_batch(const MixerDesc* D, const int4* blocks, const int* counts, int* flags);
 
+// One field of a box (src: its first node, x fastest) in [i][j][k] order.
+__global__ void k_box_ijk(const double* src, int nx, int ny, int nz, double* dst);
+
 __global__ void k_mixing_rows(const double* __restrict__ Mac, Geom G, double* __restrict__ stats);
 __global__ void k_sums(const double* __restrict__ Mac, Geom G, double* __restrict__ partial);
 // The inlet duct series of the reduced-precision forms, computed on the device.
