@@ -1135,7 +1135,7 @@ int tmx_mixing(tmx_handle* h, double* rows_out, double* outlet_im)
     TMX_CK(cudaSetDevice(h->device));
     const Geom& G = h->G;
     const int nrow = G.mny + G.iny;
-    tmx::k_mixing_rows<<<nrow, 32, 0, h->stream>>>(h->mac, G, h->stats);
+    tmx::k_mixing_rows<<<nrow, 3 * tmx::kRowPart, 0, h->stream>>>(h->mac, G, h->stats);
     TMX_CK(cudaGetLastError());
     std::vector<double> st((size_t)nrow * 9);
     TMX_CK(cudaMemcpyAsync(st.data(), h->stats, st.size() * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
@@ -1197,7 +1197,7 @@ int tmx_mixing_static(tmx_handle* h, double* rows_out, double* outlet_im)
                     cudaGetErrorString(g_mix_err[d]));
     double* stats = g_mix_ptr[d];
     double* rows = stats + (size_t)tmx::kMixStaticRows * 9;
-    tmx::k_mixing_rows<<<nrow, 32, 0, h->stream>>>(h->mac, G, stats);
+    tmx::k_mixing_rows<<<nrow, 3 * tmx::kRowPart, 0, h->stream>>>(h->mac, G, stats);
     tmx::k_mixing_finish<<<1, 96, 0, h->stream>>>(stats, G, rows);
     TMX_CK(cudaGetLastError());
     TMX_CK(cudaMemcpyAsync(rows_out, rows, (size_t)nrow * 7 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
@@ -1252,7 +1252,7 @@ int tmx_pressure_power(tmx_handle* h, double* pressure_rows, double* pressure_x,
         h->bytes += (long long)nout * sizeof(double);
     }
     const int items = 1 + nrow + G.inx + npow;
-    tmx::k_pressure_power<<<(items + 127) / 128, 128, 0, h->stream>>>(h->mac, G, h->c.tau, h->diag);
+    tmx::k_pressure_power<<<items, tmx::kRowPart, 0, h->stream>>>(h->mac, G, h->c.tau, h->diag);
     TMX_CK(cudaGetLastError());
     std::vector<double> o((size_t)nout);
     TMX_CK(cudaMemcpyAsync(o.data(), h->diag, o.size() * sizeof(double), cudaMemcpyDeviceToHost, h->stream));

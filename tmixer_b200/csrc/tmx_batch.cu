@@ -814,7 +814,7 @@ int tmx_batch_outlet_im(tmx_batch* b, const int* slots, int n, double* im_out)
         b->cap_im = n;
     }
     TMX_CK(cudaMemcpyAsync(b->d_slots, slots, (size_t)n * sizeof(int), cudaMemcpyHostToDevice, b->stream));
-    tmx::k_outlet_im_batch<<<n, 32, 0, b->stream>>>(b->d_desc, b->d_slots, n, b->d_im);
+    tmx::k_outlet_im_batch<<<n, 3 * tmx::kRowPart, 0, b->stream>>>(b->d_desc, b->d_slots, n, b->d_im);
     TMX_CK(cudaGetLastError());
     TMX_CK(cudaMemcpyAsync(im_out, b->d_im, (size_t)n * 3 * sizeof(double), cudaMemcpyDeviceToHost, b->stream));
     TMX_CK(cudaStreamSynchronize(b->stream));

@@ -74,73 +74,100 @@ __global__ void __launch_bounds__(kRunBatchThreads, 512 / kRunBatchThreads) k_ru
 
 // ---------------------------------------------------------------------------
 // mixing quality (Tmixer.cpp:10161-10409): per row, per species, the sums of
-// the reference in its order (k inner, i outer), then per-row maxima.  One
-// thread block per row; thread s handles species s.  Rows: mixing 1..mny,
-// then inlet 1..iny over x = ia..ib.
+// the reference in its order (k inner, i outer), then per-row maxima.  Rows:
+// mixing 1..mny, then inlet 1..iny over x = ia..ib.  One block per row, kRowPart
+// threads per species: a thread sums a column over k, the part's first thread
+// the columns in order.  (One thread per species took 130 us for the W=32
+// mixer, waiting for a value at a time; now 12 us.)
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void row_stats(const double* __restrict__ Mac, const Geom& G, int row, int s, double& avg,
-                                          double& var, double& mx)
+struct RowShared {
+    double col[3][kRowPart], mx[3][kRowPart], out[3][3];
+};
+// avg, var and max of the three species of a row in S.out[s] (for all threads)
+__device__ __forceinline__ void row_stats(const double* __restrict__ Mac, const Geom& G, int row, RowShared& S)
 {
     const int b = row < G.mny ? 1 : 0;
     const int j = b == 1 ? row + 1 : row - G.mny + 1;
     const int i0 = b == 1 ? 1 : G.ia, i1 = b == 1 ? G.mnx : G.ib;
+    const int s = threadIdx.x / kRowPart, t = threadIdx.x % kRowPart;
     const double* cfield = Mac + (long long)(4 + s) * G.ps;
-    double sumx = 0.0;
-    mx = __longlong_as_double(0xfff0000000000000ULL);  // -inf
-    for (int i = i0; i <= i1; i++) {
-        double sumz = 0.0;
-        for (int k = 1; k <= G.nz; k++) {
-            const double v = cfield[node_index(G, b, i, j, k)];
-            sumz += v;
-            mx = fmax(mx, v);
+    const long long plane = (long long)box_nx(G, b) * box_ny(G, b);
+    double mx = __longlong_as_double(0xfff0000000000000ULL);  // -inf
+    double avg = 0.0;
+#pragma unroll 1
+    for (int pass = 0; pass < 2; pass++) {
+        double sumx = 0.0;
+        for (int c0 = i0; c0 <= i1; c0 += kRowPart) {
+            const int i = c0 + t;
+            if (i <= i1) {
+                const double* c = cfield + node_index(G, b, i, j, 1);
+                double sumz = 0.0;
+                if (pass == 0) {
+#pragma unroll 8
+                    for (int k = 0; k < G.nz; k++) {
+                        const double v = c[k * plane];
+                        sumz += v;
+                        mx = fmax(mx, v);
+                    }
+                } else {
+#pragma unroll 8
+                    for (int k = 0; k < G.nz; k++) {
+                        const double d = c[k * plane] - avg;
+                        sumz += d * d;
+                    }
+                }
+                S.col[s][t] = sumz;
+            }
+            __syncthreads();
+            if (t == 0) {
+                const int n = min(kRowPart, i1 - c0 + 1);
+#pragma unroll 8
+                for (int c = 0; c < n; c++) sumx += S.col[s][c];
+            }
+            __syncthreads();
         }
-        sumx += sumz;
-    }
-    avg = (sumx / (1.0 * G.nz * G.mnx));
-    sumx = 0.0;
-    for (int i = i0; i <= i1; i++) {
-        double sumz = 0.0;
-        for (int k = 1; k <= G.nz; k++) {
-            const double d = cfield[node_index(G, b, i, j, k)] - avg;
-            sumz += d * d;
+        if (pass == 0) {
+            S.mx[s][t] = mx;
+            if (t == 0) S.out[s][0] = (sumx / (1.0 * G.nz * G.mnx));
+        } else if (t == 0) {
+            S.out[s][1] = (1.0 / (1.0 * G.nz * G.mnx)) * sumx;
         }
-        sumx += sumz;
+        __syncthreads();
+        avg = S.out[s][0];
     }
-    var = (1.0 / (1.0 * G.nz * G.mnx)) * sumx;
+    for (int o = kRowPart / 2; o > 0; o >>= 1) {
+        if (t < o) S.mx[s][t] = fmax(S.mx[s][t], S.mx[s][t + o]);
+        __syncthreads();
+    }
+    if (t == 0) S.out[s][2] = S.mx[s][0];
+    __syncthreads();
 }
 
-__global__ void k_mixing_rows(const double* __restrict__ Mac, Geom G, double* __restrict__ stats)
+__global__ void __launch_bounds__(3 * kRowPart) k_mixing_rows(const double* __restrict__ Mac, Geom G,
+                                                              double* __restrict__ stats)
 {
-    const int row = blockIdx.x;
-    const int s = threadIdx.x;
-    if (s >= 3) return;
-    double avg, var, mx;
-    row_stats(Mac, G, row, s, avg, var, mx);
-    stats[row * 9 + s] = avg;
-    stats[row * 9 + 3 + s] = var;
-    stats[row * 9 + 6 + s] = mx;
+    __shared__ RowShared S;
+    row_stats(Mac, G, blockIdx.x, S);
+    if (threadIdx.x < 9) stats[blockIdx.x * 9 + threadIdx.x] = S.out[threadIdx.x % 3][threadIdx.x / 3];
 }
 
 // Outlet row (mixing row 1, the first row of the reference's order) of batch
 // mixers: its running maximum is max(0, the row's maximum).  One block per
-// entry, thread s handles species s.
-__global__ void k_outlet_im_batch(const MixerDesc* __restrict__ D, const int* __restrict__ slots, int n,
-                                  double* __restrict__ out)
+// entry.
+__global__ void __launch_bounds__(3 * kRowPart) k_outlet_im_batch(const MixerDesc* __restrict__ D,
+                                                                  const int* __restrict__ slots, int n,
+                                                                  double* __restrict__ out)
 {
+    __shared__ RowShared S;
     const int e = blockIdx.x, s = threadIdx.x;
-    __shared__ double avgs[3];
     if (e >= n) return;
     const MixerDesc& d = D[slots[e]];
-    double avg = 0.0, var = 0.0, m = 0.0;
-    if (s < 3) {
-        row_stats(d.X[0].mac, d.G, 0, s, avg, var, m);
-        avgs[s] = avg;
-    }
-    __syncthreads();
+    row_stats(d.X[0].mac, d.G, 0, S);
     if (s >= 3) return;
+    const double avg = S.out[s][0], var = S.out[s][1], m = S.out[s][2];
     double mx = 0.0;
     if (mx < m) mx = m;
-    const bool ok = avgs[0] > 0 && avgs[1] > 0 && avgs[2] > 0;
+    const bool ok = S.out[0][0] > 0 && S.out[1][0] > 0 && S.out[2][0] > 0;
     out[3 * e + s] = ok ? 1.0 - sqrt(var / (avg * (mx - avg))) : 0.0;
 }
 
@@ -240,86 +267,89 @@ __global__ void k_mixing_finish(const double* __restrict__ stats, Geom G, double
 
 // ---------------------------------------------------------------------------
 // Pressure and specific power (the numbers of write_Pressure_Power,
-// Tmixer.cpp:9866-10027), one thread per output item, each a sequential sum
-// in the reference's order.  out: [0] the pressure of inlet row iny over the
-// opening (p_top), [1 .. nrow] the row pressures (mixing rows 1..mny, inlet
-// rows 1..iny over x = ia..ib), then inx cross-section pressures of the inlet
-// box, then for each mixing row j = 2..mny-1 four rates: cross-section and
+// Tmixer.cpp:9866-10027), one block per output item, each a sum in the
+// reference's order: a thread takes one turn of the outer loop with its inner
+// loop, the first threads add up the turns.  (One thread per item took 2.1 ms
+// for the W=32 mixer and 11 ms at W=64.)  out: [0] the pressure of inlet row iny
+// over the opening (p_top), [1 .. nrow] the row pressures (mixing rows 1..mny,
+// inlet rows 1..iny over x = ia..ib), then inx cross-section pressures of the
+// inlet box, then for each mixing row j = 2..mny-1 four rates: cross-section and
 // total as the reference computes them (its x loop assigns rather than adds,
 // so only column mnx-1 enters the sums over k) and the same two summed over
 // every column.  Pressures are mean density / 3; rates use
 // vis = (2 tau - 1) / 6 and the central differences of the velocity.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ double mean_row_rho(const double* __restrict__ rho, const Geom& G, int b, int j, int i0,
-                                               int i1)
+__global__ void __launch_bounds__(kRowPart) k_pressure_power(const double* __restrict__ Mac, Geom G, double tau,
+                                                             double* __restrict__ out)
 {
-    double sumx = 0.0;
-    for (int i = i0; i <= i1; i++) {
-        double sumz = 0.0;
-        for (int k = 1; k <= G.nz; k++) sumz += rho[node_index(G, b, i, j, k)];
-        sumx += sumz;
-    }
-    return (sumx / (1.0 * G.nz * G.mnx)) / 3.0;
-}
-
-__global__ void k_pressure_power(const double* __restrict__ Mac, Geom G, double tau, double* __restrict__ out)
-{
-    const int nrow = G.mny + G.iny, nitems = 1 + nrow + G.inx + (G.mny - 2);
+    __shared__ double part[4][kRowPart];
+    const int nrow = G.mny + G.iny, t = threadIdx.x, item = blockIdx.x;
     const double* rho = Mac;
     const double *ux = Mac + G.ps, *uy = Mac + 2 * G.ps, *uz = Mac + 3 * G.ps;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nitems; t += gridDim.x * blockDim.x) {
-        if (t == 0) {
-            out[0] = mean_row_rho(rho, G, 0, G.iny, G.ia, G.ib);
-        } else if (t <= nrow) {
-            const int r = t - 1;
-            out[t] = r < G.mny ? mean_row_rho(rho, G, 1, r + 1, 1, G.mnx)
-                               : mean_row_rho(rho, G, 0, r - G.mny + 1, G.ia, G.ib);
-        } else if (t <= nrow + G.inx) {
-            const int i = t - nrow;
-            double sumy = 0.0;
-            for (int j = 1; j <= G.iny; j++) {
+    const long long plane[2] = {(long long)G.inx * G.iny, (long long)G.mnx * G.mny};
+    double sum = 0.0;  // thread m < 4: the sum of part m
+    if (item <= nrow + G.inx) {
+        // mean density of a row over its columns, or of the inlet's cross-section
+        // x = i over its rows
+        const bool cross = item > nrow;
+        const int r = item - 1, i = item - nrow;
+        const int b = !cross && item > 0 && r < G.mny ? 1 : 0;
+        const int j = item == 0 ? G.iny : (b ? r + 1 : r - G.mny + 1);
+        const int o0 = cross ? 1 : (b ? 1 : G.ia), o1 = cross ? G.iny : (b ? G.mnx : G.ib);
+        for (int c0 = o0; c0 <= o1; c0 += kRowPart) {
+            const int o = c0 + t;
+            if (o <= o1) {
+                const double* c = rho + (cross ? node_index(G, 0, i, o, 1) : node_index(G, b, o, j, 1));
                 double sumz = 0.0;
-                for (int k = 1; k <= G.nz; k++) sumz += rho[node_index(G, 0, i, j, k)];
-                sumy += sumz;
+#pragma unroll 8
+                for (int k = 0; k < G.nz; k++) sumz += c[k * plane[b]];
+                part[0][t] = sumz;
             }
-            out[t] = (sumy / (1.0 * G.nz * G.iny)) / 3.0;
-        } else {
-            const int j = t - nrow - G.inx + 1;  // 2 .. mny-1
-            const double vis = ((2.0 * tau - 1.0) / 6.0) * (1.0 * 1.0 * 1.0);
-            double sumz = 0.0, sumtotalz = 0.0, allz = 0.0, alltotalz = 0.0;
-            for (int k = 2; k < G.nz; k++) {
-                double sx = 0.0, stx = 0.0, allx = 0.0, alltx = 0.0;
-                for (int i = 2; i < G.mnx; i++) {
-#define TMX_M(a, ii, jj, kk) a[node_index(G, 1, ii, jj, kk)]
-                    const double delux = (TMX_M(ux, i + 1, j, k) - TMX_M(ux, i - 1, j, k)) / 2.0;
-                    const double delvy = (TMX_M(uy, i, j + 1, k) - TMX_M(uy, i, j - 1, k)) / 2.0;
-                    const double delwz = (TMX_M(uz, i, j, k + 1) - TMX_M(uz, i, j, k - 1)) / 2.0;
-                    const double deluy = (TMX_M(ux, i, j + 1, k) - TMX_M(ux, i, j - 1, k)) / 2.0;
-                    const double delvx = (TMX_M(uy, i + 1, j, k) - TMX_M(uy, i - 1, j, k)) / 2.0;
-                    const double deluz = (TMX_M(ux, i, j, k + 1) - TMX_M(ux, i, j, k - 1)) / 2.0;
-                    const double delwx = (TMX_M(uz, i + 1, j, k) - TMX_M(uz, i - 1, j, k)) / 2.0;
-                    const double delvz = (TMX_M(uy, i, j, k + 1) - TMX_M(uy, i, j, k - 1)) / 2.0;
-                    const double delwy = (TMX_M(uz, i, j + 1, k) - TMX_M(uz, i, j - 1, k)) / 2.0;
-#undef TMX_M
-                    const double a = deluz + delwx, bxy = delvx + deluy, c = delvz + delwy;
-                    sx = delux * delux + delwz * delwz + 0.5 * (a * a);
-                    stx = delux * delux + delvy * delvy + delwz * delwz + 0.5 * (bxy * bxy) + 0.5 * (a * a) +
-                          0.5 * (c * c);
-                    allx += sx;
-                    alltx += stx;
-                }
-                sumz += sx;
-                sumtotalz += stx;
-                allz += allx;
-                alltotalz += alltx;
-            }
-            const double n = 1.0 * (G.nz - 2) * (G.mnx - 2);
-            double* o = out + 1 + nrow + G.inx + 4 * (j - 2);
-            o[0] = 2.0 * vis * (sumz / n);
-            o[1] = 2.0 * vis * (sumtotalz / n);
-            o[2] = 2.0 * vis * (allz / n);
-            o[3] = 2.0 * vis * (alltotalz / n);
+            __syncthreads();
+            if (t == 0)
+                for (int c = 0; c < min(kRowPart, o1 - c0 + 1); c++) sum += part[0][c];
+            __syncthreads();
         }
+        if (t == 0) out[item] = (sum / (1.0 * G.nz * (cross ? G.iny : G.mnx))) / 3.0;
+        return;
+    }
+    const int j = item - nrow - G.inx + 1;  // 2 .. mny-1
+    for (int k0 = 2; k0 < G.nz; k0 += kRowPart) {
+        const int k = k0 + t;
+        if (k < G.nz) {
+            double sx = 0.0, stx = 0.0, allx = 0.0, alltx = 0.0;
+            for (int i = 2; i < G.mnx; i++) {
+#define TMX_M(a, ii, jj, kk) a[node_index(G, 1, ii, jj, kk)]
+                const double delux = (TMX_M(ux, i + 1, j, k) - TMX_M(ux, i - 1, j, k)) / 2.0;
+                const double delvy = (TMX_M(uy, i, j + 1, k) - TMX_M(uy, i, j - 1, k)) / 2.0;
+                const double delwz = (TMX_M(uz, i, j, k + 1) - TMX_M(uz, i, j, k - 1)) / 2.0;
+                const double deluy = (TMX_M(ux, i, j + 1, k) - TMX_M(ux, i, j - 1, k)) / 2.0;
+                const double delvx = (TMX_M(uy, i + 1, j, k) - TMX_M(uy, i - 1, j, k)) / 2.0;
+                const double deluz = (TMX_M(ux, i, j, k + 1) - TMX_M(ux, i, j, k - 1)) / 2.0;
+                const double delwx = (TMX_M(uz, i + 1, j, k) - TMX_M(uz, i - 1, j, k)) / 2.0;
+                const double delvz = (TMX_M(uy, i, j, k + 1) - TMX_M(uy, i, j, k - 1)) / 2.0;
+                const double delwy = (TMX_M(uz, i, j + 1, k) - TMX_M(uz, i, j - 1, k)) / 2.0;
+#undef TMX_M
+                const double a = deluz + delwx, bxy = delvx + deluy, c = delvz + delwy;
+                sx = delux * delux + delwz * delwz + 0.5 * (a * a);
+                stx = delux * delux + delvy * delvy + delwz * delwz + 0.5 * (bxy * bxy) + 0.5 * (a * a) + 0.5 * (c * c);
+                allx += sx;
+                alltx += stx;
+            }
+            part[0][t] = sx;
+            part[1][t] = stx;
+            part[2][t] = allx;
+            part[3][t] = alltx;
+        }
+        __syncthreads();
+        if (t < 4)
+            for (int c = 0; c < min(kRowPart, G.nz - k0); c++) sum += part[t][c];
+        __syncthreads();
+    }
+    if (t < 4) {
+        const double vis = ((2.0 * tau - 1.0) / 6.0) * (1.0 * 1.0 * 1.0);
+        const double n = 1.0 * (G.nz - 2) * (G.mnx - 2);
+        out[1 + nrow + G.inx + 4 * (j - 2) + t] = 2.0 * vis * (sum / n);
     }
 }
 

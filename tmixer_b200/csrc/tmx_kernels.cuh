@@ -112,6 +112,10 @@ TMX_DECLARE_SWEEP(8)
 TMX_DECLARE_SWEEP(4)
 constexpr int sweep_smem_host(int ty) { return 2 * 4 * (ty + 2) * 34 * 16; }
 
+// Threads per species of the row kernels (blocks of 3 kRowPart; the pressure and
+// power kernel has kRowPart).
+constexpr int kRowPart = 128;
+
 // Outlet mixing quality of batch mixers: for entry e, mixer slots[e], the
 // I_A, I_B, I_C of mixing row 1 (the first row of tmx_mixing) into
 // out[3e..3e+2], with the arithmetic of k_mixing_rows and its finish.
