@@ -99,6 +99,11 @@ def interior_nodes(s) -> int:
     return inlet + mixing
 
 
+def row_ends(s) -> int:
+    """The inlet and x wall face nodes, the ends of the interior rows."""
+    return 2 * ((s.iny - 2) + (s.mny - 1)) * (s.nz - 2)
+
+
 def face_nodes(s) -> int:
     """The inlet, outlet and wall face nodes (no edges and corners)."""
     z, ib = s.nz - 2, s.ia + s.mnx - 1
@@ -394,10 +399,11 @@ def run_ours(args, dist: Dist) -> dict | None:
         bulk_ms, bnd_ms = tb / kr, tbd / kr
         bpl = FORM_BYTES[form]
         # nodes the interior kernel updates: the interior ones, with the sweep
-        # shape the z wall faces too (one per interior column at each end), in
-        # the FP64 form every face
+        # shape the z wall faces too (one per interior column at each end) and
+        # the ends of the rows, in the FP64 form every face
         bulk_nodes = counts["interior"] + (face_nodes(sp) if form == "fp64" else
-                                           2 * counts["interior"] // (sp.nz - 2) if form == "fp16" else 0)
+                                           2 * counts["interior"] // (sp.nz - 2) + row_ends(sp)
+                                           if form == "fp16" else 0)
         bulk_bytes = bulk_nodes * bpl
         achieved = bulk_bytes / (bulk_ms * 1e-3) / 1e9
         return dict(counts=counts, ms_max=ms_max, clk=clk, bulk_ms=bulk_ms, bnd_ms=bnd_ms, bulk_bytes=bulk_bytes,
@@ -412,7 +418,7 @@ def run_ours(args, dist: Dist) -> dict | None:
     traffic = prof.get("dram_bytes_per_launch") if prof and prof.get("nodes") == nodes else None
     roofline = {"bound": "hbm", "achieved": main["achieved"], "peak": peaks["hbm_gbs"], "unit": "GB/s",
                 "frac": main["achieved"] / peaks["hbm_gbs"], "traffic": traffic,
-                "kernel": ("k_sweep4_f16 (interior nodes and z wall faces, %d per launch)" % main["bulk_nodes"]
+                "kernel": ("k_sweep4_f16 (interior nodes, row ends and z wall faces, %d per launch)" % main["bulk_nodes"]
                            if args.form == "fp16" else
                            "k_run128_f64 (interior and face nodes, %d per launch)" % main["bulk_nodes"]
                            if args.form == "fp64" else
@@ -572,9 +578,10 @@ def run_batched(args, dist: Dist, fp64_mlups: float, peaks: dict) -> dict:
         im = B.outlet_im()
         B_shape = B.shape()
     # nodes the interior kernel updates: the interior ones, and with a sweep
-    # shape the z wall faces (one at each end of every interior column)
+    # shape the z wall faces (one at each end of every interior column) and the
+    # ends of the rows
     swept = B_shape["kernel"] != "flat"
-    upd = sum(interior_nodes(s) * (s.nz / (s.nz - 2) if swept else 1) for s in specs)
+    upd = sum(interior_nodes(s) * s.nz / (s.nz - 2) + row_ends(s) if swept else interior_nodes(s) for s in specs)
     int_gbs = upd * FORM_BYTES["fp16"] / (t_int / kt * 1e-3) / 1e9
     int_pc = pattern_ceiling(T.TMX_FP16, upd, int_gbs, dist.local_rank)
     mlups = nodes * args.batched_steps / (ms * 1e-3) / 1e6

@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 
 import tmixer_b200 as T
-from tests.cases import GOLDEN_CASES, ORACLE_CASES, to_spec
+from tests.cases import GOLDEN_CASES, ORACLE_CASES, ref_like, to_spec
 
 pytestmark = pytest.mark.gpu
 
@@ -35,13 +35,23 @@ def _same(a, b):
     return all(np.array_equal(x.view(np.uint64), y.view(np.uint64)) for x, y in zip(a, b))
 
 
-CASES = [("w24", None), ("tiny_species", None), ("wide_opening", None), ("odd_ia", None), ("w8", None)]
+CASES = [("w24", None), ("tiny_species", None), ("wide_opening", None), ("odd_ia", None), ("w8", None),
+         ("col33", None), ("col3", None)]
+
+# boxes whose last column would be alone in its tile (65 and 33 columns: an x
+# wall's species come from its neighbour in the same warp), and a mixing box
+# whose two x walls share their neighbour
+EXTRA = {
+    "col33": dict(ref_like(65, 6, 5, 33, 7, tau=0.65, k=2.0, rho0=1.5, rho_out=1.4, umean=0.05,
+                           cin=[[0.9, 0.2], [0.1, 1.1], [0.05, 0.02]]), ia=9),
+    "col3": ref_like(9, 5, 4, 3, 5, umean=0.03, cin=[[1.0, 0.25], [0.3, 1.0], [0.1, 0.05]]),
+}
 
 
 def _spec(name):
     if name.startswith("w") and name[1:].isdigit():
         return T.w_layout(int(name[1:]), u_max=0.05, tau_f=0.6, tau_c=0.6, k=1e-3, rho=1.0, precision=T.TMX_FP16)
-    s = _case(name)
+    s = to_spec(EXTRA[name]) if name in EXTRA else _case(name)
     s.precision = T.TMX_FP16
     return s
 

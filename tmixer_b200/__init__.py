@@ -406,7 +406,7 @@ class Solver:
         """Launch shape of the interior kernel (tmx_set_shape): SHAPE_FLAT, or
         for the FP16 form a sweep shape (SHAPE_SWEEP8, SHAPE_SWEEP4) with zchunk
         planes per tile.  Every shape gives the same bits.  Default: SHAPE_SWEEP4
-        with 8 planes for the FP16 form, SHAPE_FLAT for the others."""
+        with 3 to 8 planes by size for the FP16 form, SHAPE_FLAT for the others."""
         _check(lib().tmx_set_shape(self._h, int(kind), int(zchunk)))
         return self
 

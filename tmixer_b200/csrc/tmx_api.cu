@@ -75,9 +75,9 @@ struct tmx_handle {
     cudaStream_t aux = nullptr, aux2 = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr, join2 = nullptr;
     int nface = 0;  // the first nface boundary nodes are face classes
-    // the last nzwall faces are the z wall faces, which the sweep kernels
-    // update (boundary_list)
-    int nzwall = 0;
+    // the last nswept faces are those that the sweep kernels update
+    // (boundary_list)
+    int nswept = 0;
     // FP64 form: the run list and grid of k_run_f64, its two run counters
     int4* runs = nullptr;
     int nruns = 0, run_slots = 0, run_nt = 256;
@@ -337,16 +337,16 @@ void inlet_profile(const tmx_case& c, std::vector<double>& U1, std::vector<doubl
 }
 
 int boundary_list(const Geom& G, std::vector<int>& nodes, std::vector<unsigned char>& cls, int& nface,
-                  std::vector<int>* class_count, int* nzwall)
+                  std::vector<int>* class_count, int* nswept)
 {
     struct Entry {
         int cls, node;
-        bool zwall;
+        bool swept;
     };
     std::vector<Entry> all;
     all.reserve((size_t)boundary_count(G));
     if (class_count) class_count->assign(tmx::K_NCLASSES, 0);
-    bool zsep = nzwall != nullptr;
+    bool zsep = nswept != nullptr;
     long long zcount = 0, interior2 = 0;
     for (int b = 0; b < 2; b++)
         for (int i = 1; i <= G.nx[b]; i++)
@@ -361,26 +361,27 @@ int boundary_list(const Geom& G, std::vector<int>& nodes, std::vector<unsigned c
                     const bool zw = c == tmx::K_FACE_Z1 || c == tmx::K_FACE_ZT;
                     if (zw) {
                         // the interior node of the column the sweep kernels
-                        // update this wall node with (sweep_zwall)
+                        // update this wall node with (zwall_node)
                         const int kw = c == tmx::K_FACE_Z1 ? 1 : G.nz, kn = c == tmx::K_FACE_Z1 ? 2 : G.nz - 1;
                         if (k != kw || G.nz < 3 || tmx::is_boundary(G, b, i, j, kn)) zsep = false;
                         zcount++;
                     }
-                    all.push_back({c, tmx::node_index(G, b, i, j, k), zw});
+                    const bool end = c == tmx::K_INLET1 || c == tmx::K_INLET2 || c == tmx::K_FACE_MX1 || c == tmx::K_FACE_MXT;
+                    all.push_back({c, tmx::node_index(G, b, i, j, k), zw || end});
                 }
             }
     // every z wall node above or below an interior node, and every interior
     // node of planes 2 and nz - 1 under or over one
     if (zcount != 2 * interior2) zsep = false;
-    if (nzwall && !zsep && interior2 > 0)
+    if (nswept && !zsep && interior2 > 0)
         return fail(TMX_E_INVALID, "internal: the z wall faces do not pair with the interior nodes of planes 2 and %d",
                     G.nz - 1);
-    // faces first (with zsep the z wall faces last among them), then edges
+    // faces first (with zsep the swept ones last among them), then edges
     // and corners; by class, then node
     std::vector<std::pair<int, int>> bl;
     bl.reserve(all.size());
     for (const Entry& e : all)
-        bl.emplace_back((tmx::is_face_class(e.cls) ? (zsep && e.zwall ? 128 : 0) : 256) + e.cls, e.node);
+        bl.emplace_back((tmx::is_face_class(e.cls) ? (zsep && e.swept ? 128 : 0) : 256) + e.cls, e.node);
     std::sort(bl.begin(), bl.end());
     nodes.resize(bl.size());
     cls.resize(bl.size());
@@ -392,7 +393,7 @@ int boundary_list(const Geom& G, std::vector<int>& nodes, std::vector<unsigned c
         if (bl[t].first < 256) nface++;
         if (bl[t].first >= 128 && bl[t].first < 256) nzw++;
     }
-    if (nzwall) *nzwall = nzw;
+    if (nswept) *nswept = nzw;
     return TMX_OK;
 }
 
@@ -550,9 +551,8 @@ int enqueue_step(tmx_handle* h, int cur, int write_macro, cudaEvent_t* ev)
     if (ev) TMX_CK(cudaEventRecord(ev[2], h->aux));
     const int nf = h->nface, ne = h->nb - h->nface;
     const int bt = tmx::kBoundaryThreadsHost, nl = tmx::kBoundaryLanesHost;  // nl threads per face
-    // with a sweep shape the interior kernel updates the z wall faces, the
-    // last nzwall of the face range (zwall_node)
-    const int nfk = sweep_shape(h->shape) ? nf - h->nzwall : nf;
+    // with a sweep shape the interior kernel updates the last nswept faces
+    const int nfk = sweep_shape(h->shape) ? nf - h->nswept : nf;
     if (nfk > 0)
         h->K->faces<<<(nl * nfk + bt - 1) / bt, bt, 0, h->aux>>>(X, h->bnode, h->bcls, nfk, G, h->P, write_macro);
     if (ne > 0)
@@ -798,7 +798,7 @@ int tmx_create(const tmx_case* c, int device, tmx_handle** out)
     // boundary node list, faces first, sorted by class then node index
     std::vector<int> nodes;
     std::vector<unsigned char> cls;
-    rc = boundary_list(G, nodes, cls, h->nface, &h->class_count, &h->nzwall);
+    rc = boundary_list(G, nodes, cls, h->nface, &h->class_count, &h->nswept);
     if (rc) {
         delete h;
         return rc;
@@ -861,10 +861,15 @@ int tmx_create(const tmx_case* c, int device, tmx_handle** out)
         cudaGetLastError();
         h->run_slots = sms * std::max(1, per);
     }
-    // the FP16 form's interior as 32 x 4 sweep tiles of 8 planes (the same
-    // bits as the flat kernel, faster: W=32 step 61 us against 69 us)
+    // the FP16 form's interior as 32 x 4 sweep tiles (the same bits as the flat
+    // kernel, faster)
     if (h->K->moments) {
-        const int rc = tmx_set_shape(h, TMX_SHAPE_SWEEP4, 8);
+        const SweepShape* sh = sweep_shape(TMX_SHAPE_SWEEP4);
+        int per = 4;
+        if (sweep_allow_smem() == cudaSuccess)
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)sh->single, sh->threads(), sh->smem());
+        cudaGetLastError();
+        const int rc = tmx_set_shape(h, TMX_SHAPE_SWEEP4, sweep_planes(h->G, sms * std::max(1, per)));
         if (rc) {
             const std::string msg = last_error();
             tmx_destroy(h);

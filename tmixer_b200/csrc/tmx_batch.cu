@@ -96,7 +96,7 @@ struct Slot {
     std::vector<int> nodes;
     std::vector<unsigned char> cls;
     int nface = 0;
-    int nzwall = 0;  // z wall faces last among the faces (boundary_list)
+    int nswept = 0;  // faces that the sweep kernels update, last among them (boundary_list)
     int parity0 = 0;  // batch parity at admission
     long long steps = 0;
 };
@@ -307,10 +307,9 @@ int rebuild(tmx_batch* b)
             blocks.push_back(make_int4((int)m, g0, std::min(b->cells, s.G.nnodes - g0), 0));
         if (fp64) step_runs(s.G, (int)m, tmx::kRunBatchThreads, runs);
         if (b->sweep) sweep_tiles(s.G, (int)m, sweep_shape(b->sweep)->ty, b->zchunk, tiles);
-        // with a sweep shape the interior kernel updates the z wall faces,
-        // the last nzwall of the face range (zwall_node)
+        // with a sweep shape the interior kernel updates the last nswept faces
         // (and the FP64 form's runs every face)
-        const int nfk = fp64 ? 0 : (b->sweep ? s.nface - s.nzwall : s.nface);
+        const int nfk = fp64 ? 0 : (b->sweep ? s.nface - s.nswept : s.nface);
         for (size_t t = 0; t < s.nodes.size(); t++) {
             const int2 e = make_int2(s.nodes[t], (int)m * 256 + s.cls[t]);
             if ((int)t < s.nface) {
@@ -551,6 +550,10 @@ int tmx_batch_create(int precision, long long budget_bytes, int device, tmx_batc
     b->K = &kForms[precision];
     b->B = &kBatchForms[precision];
     cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, device);
+    if (b->K->moments) {
+        b->sweep = TMX_SHAPE_SWEEP4;
+        b->zchunk = kBatchPlanes;
+    }
     const long long budget = align_up(budget_bytes);
     cudaError_t e = cudaMalloc((void**)&b->arena_base, (size_t)budget);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
@@ -628,7 +631,7 @@ int admit(tmx_batch* b, const tmx_case* c, const void* buf, long long size, int*
     if (off < 0)
         return fail(TMX_E_NOMEM, "batch budget: %lld bytes needed, %lld free (largest range %lld)", cv.total,
                     b->arena.free_bytes(), b->arena.largest());
-    rc = boundary_list(s.G, s.nodes, s.cls, s.nface, nullptr, &s.nzwall);
+    rc = boundary_list(s.G, s.nodes, s.cls, s.nface, nullptr, &s.nswept);
     if (rc) {
         b->arena.release(off, cv.total);
         return rc;

@@ -589,9 +589,30 @@ struct PopGlobal {
 // one pass, which the FP32 register budget affords (the FP64 form loads field
 // by field).  The arithmetic does not depend on where the records and the
 // stored populations (pop) come from.
-template <class PR, class Rec, class Pop>
+//
+// With XF the node may be an x face (xf.cls; the sweep kernels): the flow is
+// closed, and the species come from the neighbour lane xf.from, whose node is
+// the interior neighbour (the mixing box's walls), or are closed (the inlets).
+struct XFace {
+    int cls;        // the node's class, -1: interior
+    int from;       // the lane of the node whose species are taken
+    unsigned mask;  // the lanes that are here
+    bool walls;     // (warp-uniform) some lane is an x wall of the mixing box
+};
+template <class PR>
+struct BCtx;
+template <class PR>
+__device__ __forceinline__ void closure_face(const BCtx<PR>& c, int cls, int fld, typename PR::T (&v)[19]);
+template <class T>
+__device__ __forceinline__ void wall_flow_closure(int cls, T rout, T (&v)[19]);
+template <class PR>
+__device__ __forceinline__ void xface_inlet(const StepPtrs& X, const Geom& G, const Phys& P, int cls, int j, int k,
+                                            float2 (&p01)[19], float2 (&p23)[19]);
+
+template <class PR, bool XF = false, class Rec, class Pop>
 __device__ __forceinline__ void lp_interior(const StepPtrs& X, const Geom& G, const Phys& P, int write_macro, int g,
-                                            int b, int i, int j, int k, const Rec& rec, const Pop& pop)
+                                            int b, int i, int j, int k, const Rec& rec, const Pop& pop,
+                                            const XFace xf = XFace{-1, 0, 0u, false})
 {
     using T = typename PR::T;
     typename PR::S* __restrict__ Pout = (typename PR::S*)X.pout;
@@ -607,6 +628,28 @@ __device__ __forceinline__ void lp_interior(const StepPtrs& X, const Geom& G, co
         float4 mf = make_float4(0.f, 0.f, 0.f, 0.f), ms = mf;
         if constexpr (PR::kMoments) rec(q, s, mf, ms);
         PR::decode_raw(pop(q, s), EX(q), EY(q), EZ(q), (float)wq(q), mf, ms, p01[q], p23[q]);
+    }
+    if constexpr (XF) {
+        if (xf.walls) {
+#pragma unroll
+            for (int q = 0; q < 19; q++) {
+                p01[q].y = __shfl_sync(xf.mask, p01[q].y, xf.from);
+                p23[q].x = __shfl_sync(xf.mask, p23[q].x, xf.from);
+                p23[q].y = __shfl_sync(xf.mask, p23[q].y, xf.from);
+            }
+        }
+        if (xf.cls >= 0) {
+            if (b) {
+                T v[19];
+#pragma unroll
+                for (int q = 0; q < 19; q++) v[q] = p01[q].x;
+                wall_flow_closure(xf.cls, T(0), v);
+#pragma unroll
+                for (int q = 0; q < 19; q++) p01[q].x = v[q];
+            } else {
+                xface_inlet<PR>(X, G, P, xf.cls, j, k, p01, p23);
+            }
+        }
     }
     // sums in index order, two fields at a time
     float2 s01 = p01[0], s23 = p23[0];
@@ -631,7 +674,7 @@ __device__ __forceinline__ void lp_interior(const StepPtrs& X, const Geom& G, co
 #pragma unroll
     for (int q = 0; q < 19; q++)
         PR::collide_store(Pout, q, ps, g, p01[q], p23[q], r01, r23, poly[q], c1a, c1b, c2a, c2b, (float)wq(q) * rt);
-    if (b == 0 && j == 2 && (i == G.ia || i == G.ib)) {
+    if ((b == 0 && j == 2 && (i == G.ia || i == G.ib)) || (XF && xf.cls >= 0)) {
         T* Rcur = (T*)X.rcur;
         Rcur[g] = rho;
         Rcur[ps + g] = ca;
@@ -801,8 +844,11 @@ __device__ __forceinline__ int tile_rec_node(const Geom& G, int b, int x, int y,
     return -1;
 }
 
-// One tile {mixer * 2 + box, x0 | y0 << 16, z0 | z1 << 16} (0-based x0, y0;
-// interior planes z0 .. z1-1, 2 <= z0 < z1 <= nz).  A and B hold the two
+// One tile {mixer * 2 + box | planes << 20, x0, y0, z0} (0-based columns from x0,
+// sweep_end, and y0; the interior planes z0 .. z1-1, 2 <= z0 < z1 <= nz).
+// A row's ends are the inlets or the mixing box's x walls, updated with it (as
+// face nodes of a list their 8-byte values were read a sector each, and the
+// partly written sectors read back: most of the face kernel's time).  A and B hold the two
 // halves of 4 * (TY + 2) * 34 records.  Every thread of the block runs the
 // same iterations (the barriers are uniform).  The tiles of the first chunk
 // (z0 = 2) also update the z = 1 wall face nodes of their columns, those of
@@ -814,10 +860,20 @@ __device__ __forceinline__ void sweep_tile(const StepPtrs& X, const Geom& G, con
 {
     constexpr int RW = kSweepX + 2, PLANE = (TY + 2) * RW, NT = kSweepX * TY;
     const int b = t.x & 1;
-    const int x0 = t.y & 0xffff, y0 = t.y >> 16, z0 = t.z & 0xffff, z1 = t.z >> 16;
+    const int x0 = t.y, y0 = t.z, z0 = t.w, z1 = z0 + (t.x >> 20);
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const int nx = box_nx(G, b), ny = box_ny(G, b);
+    const int nx = box_nx(G, b), ny = box_ny(G, b), x1 = sweep_end(x0, nx);
     const int x = x0 + tx, y = y0 + ty;
+    // the rows of interior nodes, ends and all (of the opening's row the middle)
+    const bool opening = b == 0 && y == 0;
+    const bool row = y < ny && (b ? y > 0 : y < ny - 1);
+    const bool act = row && x < x1 && (!opening || (x >= G.ia && x < G.ib - 1));
+    const bool end = !opening && (x == 0 || x == nx - 1);
+    XFace xf;
+    xf.cls = !end ? -1 : (b ? (x == 0 ? K_FACE_MX1 : K_FACE_MXT) : (x == 0 ? K_INLET1 : K_INLET2));
+    xf.from = tx + (end && b ? (x == 0 ? 1 : -1) : 0);
+    xf.walls = b && (x0 == 0 || x1 == nx);
+    xf.mask = __ballot_sync(0xffffffffu, act);
     const float4* __restrict__ M = X.mprev;
     auto stage = [&](int kk) {
         const int slot = (kk & 3) * PLANE;
@@ -841,14 +897,14 @@ __device__ __forceinline__ void sweep_tile(const StepPtrs& X, const Geom& G, con
         // any more (the barrier at the end of the previous iteration)
         if (k + 2 < z1 + 1) stage(k + 2);
         cp_async_commit();
-        if (x < nx && y < ny && !is_boundary(G, b, x + 1, y + 1, k)) {
+        if (act) {
             const int g = box_base(G, b) + ((k - 1) * ny + y) * nx + x;
-            lp_interior<PR>(X, G, P, write_macro, g, b, x + 1, y + 1, k, RecShared<TY>{A, B, tx, ty, k},
-                            PopGlobal<PR>{(const typename PR::S*)X.pin, G.ps});
-            if (k == 2)
+            lp_interior<PR, true>(X, G, P, write_macro, g, b, x + 1, y + 1, k, RecShared<TY>{A, B, tx, ty, k},
+                                  PopGlobal<PR>{(const typename PR::S*)X.pin, G.ps}, xf);
+            if (k == 2 && xf.cls < 0)
                 zwall_node<PR>(X, G, P, write_macro, b, x + 1, y + 1, 1, 2, g - nx * ny, g,
                                RecShared<TY>{A, B, tx, ty, 1}, RecShared<TY>{A, B, tx, ty, 2});
-            if (k == G.nz - 1)
+            if (k == G.nz - 1 && xf.cls < 0)
                 zwall_node<PR>(X, G, P, write_macro, b, x + 1, y + 1, G.nz, k, g + nx * ny, g,
                                RecShared<TY>{A, B, tx, ty, G.nz}, RecShared<TY>{A, B, tx, ty, k});
         }
@@ -1105,6 +1161,30 @@ __device__ __forceinline__ void closure_face(const BCtx<PR>& c, int cls, int fld
         if (flow) wall_flow_closure(cls, T(c.P->rho_out), v);
         break;
     default: break;
+    }
+}
+
+// The four fields of an inlet node in lp_interior's pairs.
+template <class PR>
+__device__ __forceinline__ void xface_inlet(const StepPtrs& X, const Geom& G, const Phys& P, int cls, int j, int k,
+                                            float2 (&p01)[19], float2 (&p23)[19])
+{
+    using T = typename PR::T;
+    BCtx<PR> c{};
+    c.uin1 = (const T*)X.uin1;
+    c.uin2 = (const T*)X.uin2;
+    c.G = &G;
+    c.P = &P;
+    c.j = j;
+    c.k = k;
+    T v[19];
+#pragma unroll
+    for (int fld = 0; fld < 4; fld++) {
+#pragma unroll
+        for (int q = 0; q < 19; q++) v[q] = fld == 0 ? p01[q].x : (fld == 1 ? p01[q].y : (fld == 2 ? p23[q].x : p23[q].y));
+        closure_face(c, cls, fld, v);
+#pragma unroll
+        for (int q = 0; q < 19; q++) (fld == 0 ? p01[q].x : (fld == 1 ? p01[q].y : (fld == 2 ? p23[q].x : p23[q].y))) = v[q];
     }
 }
 
@@ -1854,7 +1934,7 @@ __device__ __forceinline__ void load_desc(StepDesc& dst, const MixerDesc* __rest
         for (int t = blockIdx.x; t < n; t += gridDim.x) {                                                       \
             const int4 tl = tiles[t];                                                                           \
             __syncthreads();                                                                                    \
-            load_desc(d, D, tl.x >> 1, parity);                                                                 \
+            load_desc(d, D, (tl.x & 0xfffff) >> 1, parity);                                                                 \
             __syncthreads();                                                                                    \
             sweep_tile<PR, TY>(d.X, d.G, d.P, write_macro, tl, A, B);                                           \
         }                                                                                                       \

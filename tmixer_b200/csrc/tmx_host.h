@@ -57,14 +57,15 @@ long long boundary_count(const Geom& G);
 // Class of a boundary node (tmx_classes.h), -1 for a node no case covers.
 int classify(const Geom& G, int b, int i, int j, int k);
 // Boundary nodes sorted faces first, then by class, then by node index; the
-// first nface entries are face classes.  With nzwall the z wall faces
-// (K_FACE_Z1, K_FACE_ZT) come last among the faces and *nzwall counts them:
-// each lies above or below an interior node and each interior node of planes
-// 2 and nz - 1 has one (checked; an internal error otherwise), and the sweep
-// kernels update them (zwall_node).  Without interior nodes (nz < 3) they
-// stay in place and *nzwall is 0.  Returns TMX_OK or a failure code.
+// first nface entries are face classes.  With nswept the faces that the sweep
+// kernels update come last among them and *nswept counts them: the ends of the
+// interior rows (the inlets, the mixing box's x walls) and the z wall faces
+// (K_FACE_Z1, K_FACE_ZT), of which each lies above or below an interior node
+// and each interior node of planes 2 and nz - 1 has one (checked; an internal
+// error otherwise).  Without interior nodes (nz < 3) they stay in place and
+// *nswept is 0.  Returns TMX_OK or a failure code.
 int boundary_list(const Geom& G, std::vector<int>& nodes, std::vector<unsigned char>& cls, int& nface,
-                  std::vector<int>* class_count, int* nzwall);
+                  std::vector<int>* class_count, int* nswept);
 // Inlet profiles Uin1, Uin2 ((iny+3) x (nz+3)) as the reference computes them:
 // the duct series (which depends on iny and nz only) and its mean, then the
 // scaling to umean and the shifts.
@@ -115,18 +116,17 @@ inline cudaError_t sweep_allow_smem()
 }
 
 // Tiles of the sweep kernels (tmx_engine.cuh sweep_tile) for one mixer:
-// {mixer * 2 + box, x0 | y0 << 16, z0 | z1 << 16, 0}, 32 x ty nodes of a box
-// (0-based x0, y0) over the interior planes z0 .. z1-1 (zchunk at most),
-// z-chunks outermost.
+// {mixer * 2 + box | planes << 20, x0, y0, z0}, the columns from x0 (sweep_end)
+// by ty rows of a box (0-based x0, y0) over zchunk interior planes from z0 (2000
+// at most), z-chunks outermost.
 inline void sweep_tiles(const Geom& G, int mixer, int ty, int zchunk, std::vector<int4>& out)
 {
-    for (int z0 = 2; z0 <= G.nz - 1; z0 += zchunk) {
-        const int z1 = z0 + zchunk < G.nz ? z0 + zchunk : G.nz;
+    zchunk = zchunk < 2000 ? zchunk : 2000;
+    for (int z0 = 2; z0 <= G.nz - 1; z0 += zchunk)
         for (int b = 0; b < 2; b++)
             for (int y0 = 0; y0 < G.ny[b]; y0 += ty)
-                for (int x0 = 0; x0 < G.nx[b]; x0 += 32)
-                    out.push_back(make_int4(mixer * 2 + b, x0 | (y0 << 16), z0 | (z1 << 16), 0));
-    }
+                for (int x0 = 0; x0 < G.nx[b]; x0 = tmx::sweep_end(x0, G.nx[b]))
+                    out.push_back(make_int4((mixer * 2 + b) | std::min(zchunk, G.nz - z0) << 20, x0, y0, z0));
 }
 
 // Threads per block, and so nodes per run, of the FP64 step: 256, whose 2 KB
@@ -189,6 +189,25 @@ int box_to_host(const Geom& G, int box, const double* dev, double* scratch, cuda
 // with), and its return; null when there is no memory.
 int* error_flag_take();
 void error_flag_give(int* flag);
+
+// Planes per 32 x 4 tile of a new FP16 handle: the fewest from 3 whose tiles the
+// GPU holds at once (slots blocks), 8 where none does.  A tile goes through its
+// planes one after another, so a small mixer wants short tiles (W=8 step 19.5 us
+// by 3 planes, 29.8 us by 8; W=24 31.8 by 4, 39.3 by 8), and a second, partly
+// filled wave costs a whole one (W=32 75.5 us by 6 planes, 60.3 by 8).
+inline int sweep_planes(const Geom& G, int slots)
+{
+    for (int z = 3; z < 8; z++) {
+        std::vector<int4> t;
+        sweep_tiles(G, 0, 4, z, t);
+        if ((int)t.size() <= slots) return z;
+    }
+    return 8;
+}
+// ... and of a new FP16 batch, whose mixers are not known yet (8 mixers of
+// 544,000 nodes: 123 us by the flat kernel, 85 by 4 planes, 95 by 8; 4 mixers of
+// 4.3M nodes: 585, 409, 401 us)
+constexpr int kBatchPlanes = 4;
 
 // Checkpoint layout (tmx_checkpoint, tmx_batch_checkpoint): this header, then
 // the sections in the order of `bytes`: the population buffer the next step

@@ -100,9 +100,15 @@ TMX_DECLARE_BATCH_KERNELS(f32)
 TMX_DECLARE_BATCH_KERNELS(f16)
 
 // The FP16 form's interior by tiles of 32 x TY nodes swept through z
-// (tmx_engine.cuh sweep_tile): tiles[t] = {mixer * 2 + box, x0 | y0 << 16,
-// z0 | z1 << 16}; the single-mixer kernels take mixer 0, the batched ones read
+// (tmx_engine.cuh sweep_tile): tiles[t] = {mixer * 2 + box | planes << 20,
+// x0, y0, z0}; the single-mixer kernels take mixer 0, the batched ones read
 // the tile count from counts[3].  Dynamic shared memory: sweep_smem_host(TY).
+// The end of a tile's columns: 32 on, but never the box's last column alone (an
+// x wall's species come from its neighbour in the same warp).
+__host__ __device__ constexpr int sweep_end(int x0, int nx)
+{
+    return x0 + 32 >= nx ? nx : (x0 + 32 == nx - 1 ? x0 + 31 : x0 + 32);
+}
 #define TMX_DECLARE_SWEEP(SUFFIX)                                                                               \
     __global__ void k_sweep##SUFFIX##_f16(StepPtrs X, Geom G, Phys P, int write_macro, const int4* tiles,     \
                                           int ntiles);                                                        \
