@@ -400,10 +400,9 @@ def run_ours(args, dist: Dist) -> dict | None:
         bpl = FORM_BYTES[form]
         # nodes the interior kernel updates: the interior ones, with the sweep
         # shape the z wall faces too (one per interior column at each end) and
-        # the ends of the rows, in the FP64 form every face
-        bulk_nodes = counts["interior"] + (face_nodes(sp) if form == "fp64" else
-                                           2 * counts["interior"] // (sp.nz - 2) + row_ends(sp)
-                                           if form == "fp16" else 0)
+        # the ends of the rows, in the FP64 and FP32 forms every face
+        bulk_nodes = counts["interior"] + (2 * counts["interior"] // (sp.nz - 2) + row_ends(sp)
+                                           if form == "fp16" else face_nodes(sp))
         bulk_bytes = bulk_nodes * bpl
         achieved = bulk_bytes / (bulk_ms * 1e-3) / 1e9
         return dict(counts=counts, ms_max=ms_max, clk=clk, bulk_ms=bulk_ms, bnd_ms=bnd_ms, bulk_bytes=bulk_bytes,
@@ -420,9 +419,8 @@ def run_ours(args, dist: Dist) -> dict | None:
                 "frac": main["achieved"] / peaks["hbm_gbs"], "traffic": traffic,
                 "kernel": ("k_sweep4_f16 (interior nodes, row ends and z wall faces, %d per launch)" % main["bulk_nodes"]
                            if args.form == "fp16" else
-                           "k_run128_f64 (interior and face nodes, %d per launch)" % main["bulk_nodes"]
-                           if args.form == "fp64" else
-                           "k_bulk_%s (interior nodes, %d per launch)" % (args.form, counts["interior"])),
+                           "k_run128_%s (interior and face nodes, %d per launch)" % (
+                               {"fp64": "f64", "fp32": "f32"}[args.form], main["bulk_nodes"])),
                 "peak_source": peaks["source"],
                 "algorithmic_bytes_per_lup": FORM_BYTES[args.form],
                 "algorithmic_bytes_per_launch": main["bulk_bytes"],
@@ -510,7 +508,7 @@ def run_ours(args, dist: Dist) -> dict | None:
             "data": "synthetic",
             "form": form_text[args.form], "config": config_dict(workload_params(), dist.world),
             "roofline": roofline, "cpu_baseline": cpu, "e2e": e2e, "clocks": clk,
-            "gpu_launches": (1 if args.form == "fp64" else 3) * args.steps, "forms": forms,
+            "gpu_launches": (3 if args.form == "fp16" else 1) * args.steps, "forms": forms,
             "reference_case": refcase, "batched": batched,
             "served": served}
 

@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "../../tmixer_b200/csrc/tmx_host.h"
+#include "../../tmixer_b200/csrc/tmx_run32.cuh"
 #include "../../tmixer_b200/csrc/tmx_run64.cuh"
 
 using namespace tmx;
@@ -32,6 +33,21 @@ static int check(const Geom& G, int nt)
                 const long long at = p * G.ps + first[fld][q];
                 if (at < 0 || at % 2 || count[fld][q] % 2 || count[fld][q] > nt + 4 || at + count[fld][q] > 76 * G.ps)
                     return std::printf("window %lld + %d\n", at, count[fld][q]), 1;
+            }
+        // the FP32 form's windows: the value that thread e reads is at e + 1 (+ xs)
+        for (int c = 0; c < 2; c++)
+            for (int q = 0; q < 19; q++) {
+                const int off = run_offset(R, c, EX(q), EY(q), EZ(q));
+                int f = 0, n = 0;
+                if (!run_pulls(R, c, EY(q), EZ(q))) continue;
+                run32_window(R.g0, R.n, off, q, G.ps, f, n);
+                const long long at = q * G.ps + f;
+                if (at < 0 || n > nt + 2 || at + n > 19 * G.ps || f + 1 != R.g0 + off)
+                    return std::printf("FP32 window %lld + %d\n", at, n), 1;
+                for (int e = 0; e < R.n; e++) {
+                    const RunNode N = run_node(G, R, e);
+                    if (N.act && e + 1 + (c ? N.xs : 0) >= n) return std::printf("FP32 window too short\n"), 1;
+                }
             }
         for (int e = 0; e < nt; e++) {
             const RunNode N = run_node(G, R, e);

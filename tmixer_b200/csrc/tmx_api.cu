@@ -78,7 +78,8 @@ struct tmx_handle {
     // the last nswept faces are those that the sweep kernels update
     // (boundary_list)
     int nswept = 0;
-    // FP64 form: the run list and grid of k_run_f64, its two run counters
+    // FP64 and FP32 forms: the run list and grid of the run kernel, its two run
+    // counters
     int4* runs = nullptr;
     int nruns = 0, run_slots = 0, run_nt = 256;
     int* counters = nullptr;
@@ -95,9 +96,12 @@ struct tmx_handle {
 };
 
 const StepKernels tmx_host::kForms[3] = {
-    {tmx::k_init_f64, nullptr, nullptr, nullptr, {tmx::k_run128_f64, tmx::k_run256_f64}, 8, 8, false},
-    {tmx::k_init_f32, tmx::k_bulk_f32, tmx::k_bfaces_f32, tmx::k_bedges_f32, {nullptr, nullptr}, 4, 4, false},
-    {tmx::k_init_f16, tmx::k_bulk_f16, tmx::k_bfaces_f16, tmx::k_bedges_f16, {nullptr, nullptr}, 2, 4, true},
+    {tmx::k_init_f64, nullptr, nullptr, nullptr, {tmx::k_run128_f64, tmx::k_run256_f64}, tmx::run_smem_host, 8, 8,
+     false},
+    {tmx::k_init_f32, nullptr, nullptr, nullptr, {tmx::k_run128_f32, tmx::k_run128_f32}, tmx::run32_smem_host, 4, 4,
+     false},
+    {tmx::k_init_f16, tmx::k_bulk_f16, tmx::k_bfaces_f16, tmx::k_bedges_f16, {nullptr, nullptr}, nullptr, 2, 4,
+     true},
 };
 
 namespace tmx_host {
@@ -499,7 +503,7 @@ void free_all(tmx_handle* h)
     h->stream = nullptr;
 }
 
-// The FP64 step from buffer `cur`: one launch.  With ev (4 events) the edges
+// The FP64 or FP32 step from buffer `cur`: one launch.  With ev (4 events) the edges
 // and the runs are launched one after the other, so that each event pair times
 // its part alone.
 int enqueue_run(tmx_handle* h, const tmx::StepPtrs& X, int cur, int write_macro, cudaEvent_t* ev)
@@ -508,7 +512,7 @@ int enqueue_run(tmx_handle* h, const tmx::StepPtrs& X, int cur, int write_macro,
     auto launch = [&](int nruns, int nedges) {
         const int per = h->run_nt / 32;  // a warp per edge node
         const int blocks = std::max(1, std::min(h->run_slots, (nedges + per - 1) / per + nruns));
-        h->K->run[h->run_nt > 128]<<<blocks, h->run_nt, tmx::run_smem_host(h->run_nt), h->stream>>>(
+        h->K->run[h->run_nt > 128]<<<blocks, h->run_nt, h->K->run_smem(h->run_nt), h->stream>>>(
             X, h->G, h->P, write_macro, h->runs, nruns, h->bnode + h->nface, h->bcls + h->nface, nedges, h->counters,
             cur, h->error);
     };
@@ -528,7 +532,7 @@ int enqueue_run(tmx_handle* h, const tmx::StepPtrs& X, int cur, int write_macro,
 
 // Queue one step from buffer `cur`: the face and the edge kernel on the two
 // auxiliary streams, forked from and joined back into the main stream, and the
-// bulk kernel on the main stream (FP64: enqueue_run).  With ev (4 events) each
+// bulk kernel on the main stream (FP64 and FP32: enqueue_run).  With ev (4 events) each
 // part is bracketed by its own pair of events.  The state and density buffers
 // flip together every step, so one parity index selects both.
 int enqueue_step(tmx_handle* h, int cur, int write_macro, cudaEvent_t* ev)
@@ -590,7 +594,7 @@ int enqueue_step(tmx_handle* h, int cur, int write_macro, cudaEvent_t* ev)
 int settled(const tmx_handle* h)
 {
     if (h->error && *(volatile int*)h->error)
-        return fail(TMX_E_CUDA, "a step of the FP64 form gave up waiting for its copies: the state is not valid");
+        return fail(TMX_E_CUDA, "a step gave up waiting for its copies: the state is not valid");
     return TMX_OK;
 }
 
@@ -832,7 +836,7 @@ int tmx_create(const tmx_case* c, int device, tmx_handle** out)
     if (e == cudaSuccess && h->nb) e = cudaMemcpy(h->bcls, cls.data(), cls.size(), cudaMemcpyHostToDevice);
     std::vector<int4> runs;
     if (h->K->run[0]) {
-        h->run_nt = run_threads(G.nnodes);
+        h->run_nt = run_threads(c->precision, G.nnodes);
         step_runs(G, 0, h->run_nt, runs);
         h->nruns = (int)runs.size();
         if (e == cudaSuccess) e = alloc((void**)&h->runs, std::max<size_t>(1, runs.size()) * sizeof(int4));
@@ -853,7 +857,7 @@ int tmx_create(const tmx_case* c, int device, tmx_handle** out)
     h->bulk_blocks = std::max(1, std::min((G.nnodes + 255) / 256, sms * 8));
     if (h->K->run[0]) {
         const void* k = (const void*)h->K->run[h->run_nt > 128];
-        const int smem = tmx::run_smem_host(h->run_nt);
+        const int smem = h->K->run_smem(h->run_nt);
         cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         int per = 1;

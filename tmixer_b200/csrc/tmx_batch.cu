@@ -46,18 +46,19 @@ using namespace tmx_host;
 namespace {
 
 using BulkBatchFn = void (*)(const MixerDesc*, const int4*, const int*, int, int);
+using RunBatchFn = void (*)(const MixerDesc*, const int4*, const int2*, int*, int, int, int, int*);
 using BoundaryBatchFn = void (*)(const MixerDesc*, const int2*, const int*, int, int);
 
 struct BatchKernels {
     BulkBatchFn bulk[3];  // 128, 256, 512 threads per block
     BoundaryBatchFn faces, edges;
+    RunBatchFn run;  // the whole step (FP64 and FP32; the pointers above are null)
 };
 const BatchKernels kBatchForms[3] = {
-    {{nullptr, nullptr, nullptr}, nullptr, nullptr},  // FP64: k_run_batch_f64
-    {{tmx::k_bulk_batch128_f32, tmx::k_bulk_batch256_f32, tmx::k_bulk_batch512_f32}, tmx::k_bfaces_batch_f32,
-     tmx::k_bedges_batch_f32},
+    {{nullptr, nullptr, nullptr}, nullptr, nullptr, tmx::k_run_batch_f64},
+    {{nullptr, nullptr, nullptr}, nullptr, nullptr, tmx::k_run_batch_f32},
     {{tmx::k_bulk_batch128_f16, tmx::k_bulk_batch256_f16, tmx::k_bulk_batch512_f16}, tmx::k_bfaces_batch_f16,
-     tmx::k_bedges_batch_f16},
+     tmx::k_bedges_batch_f16, nullptr},
 };
 constexpr int kBulkThreads[3] = {128, 256, 512};
 constexpr int kCellChoices[4] = {1024, 2048, 4096, 8192};
@@ -205,9 +206,9 @@ struct tmx_batch {
     int2* d_edges = nullptr;
     int cap_edges = 0;
     int* d_counts = nullptr;  // kCounts ints (tmx_kernels.cuh)
-    int4* d_runs = nullptr;   // FP64 form: runs of every mixer
+    int4* d_runs = nullptr;   // FP64 and FP32 forms: runs of every mixer
     int cap_runs = 0;
-    int* error = nullptr;     // FP64 form: set by a step whose copies did not arrive (error_flag_take)
+    int* error = nullptr;     // ... set by a step whose copies did not arrive (error_flag_take)
     int* d_slots = nullptr;
     double* d_im = nullptr;
     int* d_flags = nullptr;  // per-slot health flags (tmx_batch_health)
@@ -295,7 +296,7 @@ int rebuild(tmx_batch* b)
 {
     std::vector<MixerDesc> desc(b->slots.size());
     std::vector<int4> blocks, tiles, runs;
-    const bool fp64 = b->precision == TMX_FP64;
+    const bool by_runs = b->B->run != nullptr;
     std::vector<int2> faces, edges;
     int nactive = 0;
     for (size_t m = 0; m < b->slots.size(); m++) {
@@ -305,11 +306,11 @@ int rebuild(tmx_batch* b)
         desc[m] = desc_of(b, s);
         for (int g0 = 0; g0 < s.G.nnodes; g0 += b->cells)
             blocks.push_back(make_int4((int)m, g0, std::min(b->cells, s.G.nnodes - g0), 0));
-        if (fp64) step_runs(s.G, (int)m, tmx::kRunBatchThreads, runs);
+        if (by_runs) step_runs(s.G, (int)m, tmx::kRunBatchThreads, runs);
         if (b->sweep) sweep_tiles(s.G, (int)m, sweep_shape(b->sweep)->ty, b->zchunk, tiles);
         // with a sweep shape the interior kernel updates the last nswept faces
-        // (and the FP64 form's runs every face)
-        const int nfk = fp64 ? 0 : (b->sweep ? s.nface - s.nswept : s.nface);
+        // (and the runs every face)
+        const int nfk = by_runs ? 0 : (b->sweep ? s.nface - s.nswept : s.nface);
         for (size_t t = 0; t < s.nodes.size(); t++) {
             const int2 e = make_int2(s.nodes[t], (int)m * 256 + s.cls[t]);
             if ((int)t < s.nface) {
@@ -365,11 +366,10 @@ int rebuild(tmx_batch* b)
 // alone (tmx_batch_step_timed).
 int enqueue(tmx_batch* b, int parity, int write_macro, cudaEvent_t* ev = nullptr)
 {
-    if (b->precision == TMX_FP64) {
+    if (b->B->run) {
         auto launch = [&](int what) {
-            tmx::k_run_batch_f64<<<b->grid_run, tmx::kRunBatchThreads, tmx::run_smem_host(tmx::kRunBatchThreads),
-                                   b->stream>>>(b->d_desc, b->d_runs, b->d_edges, b->d_counts, parity, write_macro,
-                                                what, b->error);
+            b->B->run<<<b->grid_run, tmx::kRunBatchThreads, b->K->run_smem(tmx::kRunBatchThreads), b->stream>>>(
+                b->d_desc, b->d_runs, b->d_edges, b->d_counts, parity, write_macro, what, b->error);
         };
         if (ev) {
             TMX_CK(cudaEventRecord(ev[2], b->stream));
@@ -445,10 +445,10 @@ int step_one(tmx_batch* b, int write_macro)
 
 void set_grids(tmx_batch* b)
 {
-    if (b->precision == TMX_FP64) {
+    if (b->B->run) {
         // one launch of as many blocks as fit; bound_bps only shows in the shape
-        const void* k = (const void*)tmx::k_run_batch_f64;
-        const int smem = tmx::run_smem_host(tmx::kRunBatchThreads);
+        const void* k = (const void*)b->B->run;
+        const int smem = b->K->run_smem(tmx::kRunBatchThreads);
         cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         int per = 1;
@@ -513,7 +513,7 @@ int init_slot(tmx_batch* b, Slot& s)
 int settled(const tmx_batch* b)
 {
     if (b->error && *(volatile int*)b->error)
-        return fail(TMX_E_CUDA, "a step of the FP64 batch gave up waiting for its copies: the state is not valid");
+        return fail(TMX_E_CUDA, "a step of the batch gave up waiting for its copies: the state is not valid");
     return TMX_OK;
 }
 
@@ -564,7 +564,7 @@ int tmx_batch_create(int precision, long long budget_bytes, int device, tmx_batc
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->join2, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaMalloc((void**)&b->d_counts, tmx::kCounts * sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(b->d_counts, 0, tmx::kCounts * sizeof(int));
-    if (e == cudaSuccess && precision == TMX_FP64 && !(b->error = error_flag_take())) e = cudaErrorMemoryAllocation;
+    if (e == cudaSuccess && b->B->run && !(b->error = error_flag_take())) e = cudaErrorMemoryAllocation;
     if (e != cudaSuccess) {
         cudaGetLastError();
         tmx_batch_destroy(b);
@@ -978,9 +978,9 @@ int tmx_batch_tune(tmx_batch* b, int steps_per_trial, int* threads_out, int* cel
         cudaEventElapsedTime(&ms, t0, t1);
         ms_step = ms / steps_per_trial;
     };
-    // the FP64 form has one kernel: its shape stays as it is
-    if (b->precision == TMX_FP64) trial(best);
-    for (int v = 0; v < 3 && rc == TMX_OK && b->precision != TMX_FP64; v++)
+    // the FP64 and FP32 forms have one kernel: their shape stays as it is
+    if (b->B->run) trial(best);
+    for (int v = 0; v < 3 && rc == TMX_OK && !b->B->run; v++)
         for (int ci = 0; ci < 4 && rc == TMX_OK; ci++) {
             const int cells = kCellChoices[ci];
             if (cells < kBulkThreads[v]) continue;
@@ -1015,7 +1015,7 @@ int tmx_batch_tune(tmx_batch* b, int steps_per_trial, int* threads_out, int* cel
     if (rc == TMX_OK) rc = tmx_batch_set_shape(b, kBulkThreads[bv], bc);
     if (rc == TMX_OK && bs) rc = tmx_batch_set_sweep(b, bs, bz);
     const int bchoices[4] = {1, 2, 4, 0};
-    for (int after = 0; after < (b->precision == TMX_FP64 ? 0 : 2) && rc == TMX_OK; after++)
+    for (int after = 0; after < (b->B->run ? 0 : 2) && rc == TMX_OK; after++)
         for (int i = 0; i < 4 && rc == TMX_OK; i++) {
             if (bchoices[i] >= b->bound_fit) continue;  // the same grid as 0
             rc = tmx_batch_set_boundary(b, bchoices[i], after);

@@ -583,6 +583,65 @@ struct PopGlobal {
     long long ps;
     __device__ __forceinline__ typename PR::Raw operator()(int q, int s) const { return PR::load_raw(Pin, ps, q, s); }
 };
+// Moments, equilibrium, collision and stores of node g from its closed
+// populations, the four fields as the pairs (flow, A), (B, C).  outlet: the density
+// is pinned to rho_out (Tmixer.cpp:9575-9582); densities: write them for the
+// closures that read them next step.
+template <class PR>
+__device__ __forceinline__ void lp_finish(const StepPtrs& X, const Geom& G, const Phys& P, int write_macro, int g,
+                                          const float2 (&p01)[19], const float2 (&p23)[19], bool outlet,
+                                          bool densities)
+{
+    using T = typename PR::T;
+    typename PR::S* __restrict__ Pout = (typename PR::S*)X.pout;
+    const long long ps = G.ps;
+    // sums in index order, two fields at a time
+    float2 s01 = p01[0], s23 = p23[0];
+#pragma unroll
+    for (int q = 1; q < 19; q++) {
+        s01 = __fadd2_rn(s01, p01[q]);
+        s23 = __fadd2_rn(s23, p23[q]);
+    }
+    const T rho = outlet ? T(P.rho_out) : s01.x, ca = s01.y, cb = s23.x, cc = s23.y;
+    T f[19];
+#pragma unroll
+    for (int q = 0; q < 19; q++) f[q] = p01[q].x;
+    T sxm, sym, szm;
+    momentum(f, sxm, sym, szm);
+    const T ux = sxm / rho, uy = sym / rho, uz = szm / rho;
+    T poly[19];
+    PR::poly(ux, uy, uz, poly);
+    const T rt = T(P.rateconst) * ca * cb;
+    const float2 r01 = make_float2(rho, ca), r23 = make_float2(cb, cc);
+    const float2 c1a = make_float2((float)P.c1[0], (float)P.c1[1]), c1b = make_float2((float)P.c1[2], (float)P.c1[3]);
+    const float2 c2a = make_float2((float)P.c2[0], (float)P.c2[1]), c2b = make_float2((float)P.c2[2], (float)P.c2[3]);
+#pragma unroll
+    for (int q = 0; q < 19; q++)
+        PR::collide_store(Pout, q, ps, g, p01[q], p23[q], r01, r23, poly[q], c1a, c1b, c2a, c2b, (float)wq(q) * rt);
+    if (densities) {
+        T* Rcur = (T*)X.rcur;
+        Rcur[g] = rho;
+        Rcur[ps + g] = ca;
+        Rcur[2 * ps + g] = cb;
+        Rcur[3 * ps + g] = cc;
+    }
+    if (PR::kMoments) {
+        X.mcur[2 * (long long)g] = make_float4((float)rho, (float)ca, (float)cb, (float)cc);
+        X.mcur[2 * (long long)g + 1] =
+            make_float4((float)ux, (float)uy, (float)uz, omt_term((float)ux, (float)uy, (float)uz));
+    }
+    if (write_macro) {
+        double* Mac = X.mac;
+        Mac[g] = rho;
+        Mac[ps + g] = ux;
+        Mac[2 * ps + g] = uy;
+        Mac[3 * ps + g] = uz;
+        Mac[4 * ps + g] = ca;
+        Mac[5 * ps + g] = cb;
+        Mac[6 * ps + g] = cc;
+    }
+}
+
 // One interior node (b, i, j, k) = g for the reduced-precision forms (FP32
 // arithmetic): every source index and (FP16 form) every writer's record
 // (from rec) is fetched once per direction and all 76 populations decoded in
@@ -615,8 +674,6 @@ __device__ __forceinline__ void lp_interior(const StepPtrs& X, const Geom& G, co
                                             const XFace xf = XFace{-1, 0, 0u, false})
 {
     using T = typename PR::T;
-    typename PR::S* __restrict__ Pout = (typename PR::S*)X.pout;
-    const long long ps = G.ps;
     const int sy = box_nx(G, b), sz = box_nx(G, b) * box_ny(G, b);
     const int iface = (b == 0 && j == 1) ? 1 : ((b == 1 && j == G.mny) ? 2 : 0);
 
@@ -651,51 +708,8 @@ __device__ __forceinline__ void lp_interior(const StepPtrs& X, const Geom& G, co
             }
         }
     }
-    // sums in index order, two fields at a time
-    float2 s01 = p01[0], s23 = p23[0];
-#pragma unroll
-    for (int q = 1; q < 19; q++) {
-        s01 = __fadd2_rn(s01, p01[q]);
-        s23 = __fadd2_rn(s23, p23[q]);
-    }
-    const T rho = s01.x, ca = s01.y, cb = s23.x, cc = s23.y;
-    T f[19];
-#pragma unroll
-    for (int q = 0; q < 19; q++) f[q] = p01[q].x;
-    T sxm, sym, szm;
-    momentum(f, sxm, sym, szm);
-    const T ux = sxm / rho, uy = sym / rho, uz = szm / rho;
-    T poly[19];
-    PR::poly(ux, uy, uz, poly);
-    const T rt = T(P.rateconst) * ca * cb;
-    const float2 r01 = make_float2(rho, ca), r23 = make_float2(cb, cc);
-    const float2 c1a = make_float2((float)P.c1[0], (float)P.c1[1]), c1b = make_float2((float)P.c1[2], (float)P.c1[3]);
-    const float2 c2a = make_float2((float)P.c2[0], (float)P.c2[1]), c2b = make_float2((float)P.c2[2], (float)P.c2[3]);
-#pragma unroll
-    for (int q = 0; q < 19; q++)
-        PR::collide_store(Pout, q, ps, g, p01[q], p23[q], r01, r23, poly[q], c1a, c1b, c2a, c2b, (float)wq(q) * rt);
-    if ((b == 0 && j == 2 && (i == G.ia || i == G.ib)) || (XF && xf.cls >= 0)) {
-        T* Rcur = (T*)X.rcur;
-        Rcur[g] = rho;
-        Rcur[ps + g] = ca;
-        Rcur[2 * ps + g] = cb;
-        Rcur[3 * ps + g] = cc;
-    }
-    if (PR::kMoments) {
-        X.mcur[2 * (long long)g] = make_float4((float)rho, (float)ca, (float)cb, (float)cc);
-        X.mcur[2 * (long long)g + 1] =
-            make_float4((float)ux, (float)uy, (float)uz, omt_term((float)ux, (float)uy, (float)uz));
-    }
-    if (write_macro) {
-        double* Mac = X.mac;
-        Mac[g] = rho;
-        Mac[ps + g] = ux;
-        Mac[2 * ps + g] = uy;
-        Mac[3 * ps + g] = uz;
-        Mac[4 * ps + g] = ca;
-        Mac[5 * ps + g] = cb;
-        Mac[6 * ps + g] = cc;
-    }
+    lp_finish<PR>(X, G, P, write_macro, g, p01, p23, false,
+                  (b == 0 && j == 2 && (i == G.ia || i == G.ib)) || (XF && xf.cls >= 0));
 }
 
 

@@ -37,9 +37,10 @@ struct StepKernels {
     // the face and edge lists as two launches (forms whose bulk runs beside them)
     void (*faces)(tmx::StepPtrs, const int*, const unsigned char*, int, Geom, Phys, int);
     void (*edges)(tmx::StepPtrs, const int*, const unsigned char*, int, Geom, Phys, int);
-    // the whole step in one launch, by runs of up to 128 or 256 nodes (FP64; the
-    // pointers above are null)
+    // the whole step in one launch, by runs of up to 128 or 256 nodes (FP64 and
+    // FP32; the pointers above are null)
     void (*run[2])(tmx::StepPtrs, Geom, Phys, int, const int4*, int, const int*, const unsigned char*, int, int*, int, int*);
+    int (*run_smem)(int nt);  // its dynamic shared memory
     int sbytes, tbytes;
     bool moments;  // the form stores per-node FP32 moments next to the populations
 };
@@ -129,15 +130,15 @@ inline void sweep_tiles(const Geom& G, int mixer, int ty, int zchunk, std::vecto
                     out.push_back(make_int4((mixer * 2 + b) | std::min(zchunk, G.nz - z0) << 20, x0, y0, z0));
 }
 
-// Threads per block, and so nodes per run, of the FP64 step: 256, whose 2 KB
+// Threads per block, and so nodes per run, of the FP64 step (FP32: 128): 256, whose 2 KB
 // copies get the most from DRAM, or 128 where the finer runs fill the SMs more
 // evenly (step by 128 / 256: 65,536 nodes 23.7 / 30.5 us, 524,288 nodes 116.4 /
 // 118.4 us, 1.8M nodes 358.7 / 357.7 us, 4.9M nodes 969 / 956 us).
-inline int run_threads(long long nodes)
+inline int run_threads(int precision, long long nodes)
 {
-    return nodes < 2000000 ? 128 : 256;
+    return precision != TMX_FP64 || nodes < 2000000 ? 128 : 256;
 }
-// Runs of the FP64 step (tmx_kernels.cuh) for one mixer, of up to nt nodes:
+// Runs of the FP64 and FP32 steps (tmx_kernels.cuh) for one mixer, of up to nt nodes:
 // every node but the edges and corners, plane by plane; the long runs first,
 // then the short ones (which even out the end of the launch).
 inline void step_runs(const Geom& G, int mixer, int nt, std::vector<int4>& out)

@@ -39,27 +39,28 @@ constexpr int kListAlign = kBoundaryThreadsHost / kBoundaryLanesHost;
                                     Phys P, int write_macro);
 
 TMX_DECLARE_INIT_KERNEL(f64)
-TMX_DECLARE_STEP_KERNELS(f32)
+TMX_DECLARE_INIT_KERNEL(f32)
 TMX_DECLARE_STEP_KERNELS(f16)
-TMX_DECLARE_BOUNDARY_KERNELS(f32)
 TMX_DECLARE_BOUNDARY_KERNELS(f16)
 
-// Runs of the FP64 step (tmx_run64.cuh): {first node, nodes | kind << 9 |
+// Runs of the FP64 and FP32 steps (tmx_run64.cuh, tmx_run32.cuh): {first node, nodes | kind << 9 |
 // box << 12 | iface << 13 | mixer << 15, x of the first node, z}, up to
 // NT consecutive nodes of one plane of a box, NT the kernel's threads (128 or
 // 256; run_threads in tmx_host.h).  iface: the row whose ey = 1 (1) or ey = -1
 // (2) sources lie in the other box.
 enum RunKind { kRunRows = 0, kRunZ1, kRunZT, kRunYT, kRunY1 };
+constexpr int run32_smem_host(int nt) { return 19 * (nt + 2) * 16 + nt / 32 * 400 + 544; }  // RunShared32
 constexpr int run_smem_host(int nt) { return 2 * 19 * (nt + 4) * 8 + nt / 32 * 800 + 400; }  // RunShared
 // The runs, and the edge and corner nodes enode[0..ne); counters[parity] hands
 // out the runs, counters[1 - parity] is cleared for the next step.
-#define TMX_DECLARE_RUN(NT)                                                                                     \
-    __global__ void k_run##NT##_f64(const __grid_constant__ StepPtrs X, const __grid_constant__ Geom G,         \
+#define TMX_DECLARE_RUN(NT, NAME)                                                                               \
+    __global__ void k_run##NT##_##NAME(const __grid_constant__ StepPtrs X, const __grid_constant__ Geom G,         \
                                     const __grid_constant__ Phys P, int write_macro, const int4* runs,          \
                                     int nruns, const int* enode, const unsigned char* ecls, int ne,             \
                                     int* counters, int parity, int* error);
-TMX_DECLARE_RUN(128)
-TMX_DECLARE_RUN(256)
+TMX_DECLARE_RUN(128, f64)
+TMX_DECLARE_RUN(256, f64)
+TMX_DECLARE_RUN(128, f32)
 
 // One mixer of a batch: its buffers for either parity of the batch's step
 // counter, its geometry and its physics constants (device memory, read by
@@ -78,7 +79,7 @@ struct MixerDesc {
 //           starts at a multiple of kListAlign, padded with node -1.
 // counts[0..4] = number of cell blocks, face nodes, edge nodes, sweep tiles,
 // runs (device memory, so that captured graphs stay valid when the batch
-// changes); counts[5..6] are the FP64 form's run counters.
+// changes); counts[5..6] are the run counters.
 #define TMX_DECLARE_BATCH_KERNELS(NAME)                                                                           \
     __global__ void k_bulk_batch128_##NAME(const MixerDesc* D, const int4* blocks, const int* counts, int parity, \
                                            int write_macro);                                                      \
@@ -92,11 +93,12 @@ struct MixerDesc {
                                           int write_macro);
 
 constexpr int kCounts = 7;
-// The FP64 form's batched step (runs as k_run128_f64's, of every mixer).
+// The FP64 and FP32 forms' batched steps (runs as k_run128_*'s, of every mixer).
 constexpr int kRunBatchThreads = 128;
 __global__ void k_run_batch_f64(const MixerDesc* D, const int4* runs, const int2* edges, int* counts, int parity,
                                 int write_macro, int what, int* error);
-TMX_DECLARE_BATCH_KERNELS(f32)
+__global__ void k_run_batch_f32(const MixerDesc* D, const int4* runs, const int2* edges, int* counts, int parity,
+                                int write_macro, int what, int* error);
 TMX_DECLARE_BATCH_KERNELS(f16)
 
 // The FP16 form's interior by tiles of 32 x TY nodes swept through z
