@@ -909,14 +909,10 @@ int tmx_set_shape(tmx_handle* h, int kind, int zchunk)
                             cudaGetErrorString(e));
             }
         }
-        int per = 1, sms = 148;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)sh->single, sh->threads(), sh->smem());
-        cudaGetLastError();
         cudaFree(h->tiles);
         h->tiles = d;
         h->ntiles = (int)t.size();
-        h->sweep_blocks = std::max(1, std::min(h->ntiles, sms * std::max(1, per)));
+        h->sweep_blocks = std::max(1, h->ntiles);
     }
     h->shape = kind;
     h->zchunk = zchunk;

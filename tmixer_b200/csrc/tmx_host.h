@@ -87,7 +87,7 @@ void inlet_scale(const tmx_case& c, const std::vector<double>& raw, double avera
 struct SweepShape {
     int kind, ty;
     void (*single)(tmx::StepPtrs, Geom, Phys, int, const int4*, int);
-    void (*batch)(const tmx::MixerDesc*, const int4*, const int*, int, int);
+    void (*batch)(const tmx::MixerDesc*, const int4*, int*, int, int);
     int threads() const { return 32 * ty; }
     int smem() const { return tmx::sweep_smem_host(ty); }
 };

@@ -79,7 +79,8 @@ struct MixerDesc {
 //           starts at a multiple of kListAlign, padded with node -1.
 // counts[0..4] = number of cell blocks, face nodes, edge nodes, sweep tiles,
 // runs (device memory, so that captured graphs stay valid when the batch
-// changes); counts[5..6] are the run counters.
+// changes); counts[5..6] hand out the runs or tiles of a step of either parity,
+// each cleared by the step before.
 #define TMX_DECLARE_BATCH_KERNELS(NAME)                                                                           \
     __global__ void k_bulk_batch128_##NAME(const MixerDesc* D, const int4* blocks, const int* counts, int parity, \
                                            int write_macro);                                                      \
@@ -104,7 +105,8 @@ TMX_DECLARE_BATCH_KERNELS(f16)
 // The FP16 form's interior by tiles of 32 x TY nodes swept through z
 // (tmx_engine.cuh sweep_tile): tiles[t] = {mixer * 2 + box | planes << 20,
 // x0, y0, z0}; the single-mixer kernels take mixer 0, the batched ones read
-// the tile count from counts[3].  Dynamic shared memory: sweep_smem_host(TY).
+// the tile count from counts[3] and hand the tiles out by counts[5 + parity].
+// Dynamic shared memory: sweep_smem_host(TY).
 // The end of a tile's columns: 32 on, but never the box's last column alone (an
 // x wall's species come from its neighbour in the same warp).
 __host__ __device__ constexpr int sweep_end(int x0, int nx)
@@ -114,7 +116,7 @@ __host__ __device__ constexpr int sweep_end(int x0, int nx)
 #define TMX_DECLARE_SWEEP(SUFFIX)                                                                               \
     __global__ void k_sweep##SUFFIX##_f16(StepPtrs X, Geom G, Phys P, int write_macro, const int4* tiles,     \
                                           int ntiles);                                                        \
-    __global__ void k_sweep_batch##SUFFIX##_f16(const MixerDesc* D, const int4* tiles, const int* counts,     \
+    __global__ void k_sweep_batch##SUFFIX##_f16(const MixerDesc* D, const int4* tiles, int* counts,           \
                                                 int parity, int write_macro);
 TMX_DECLARE_SWEEP(8)
 TMX_DECLARE_SWEEP(4)
