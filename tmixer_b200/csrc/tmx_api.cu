@@ -86,6 +86,8 @@ struct tmx_handle {
     int* error = nullptr;  // mapped host memory: set by a kernel whose copies did not arrive
     // one captured step per (state buffer, macroscopic output) combination
     cudaGraphExec_t graph[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
+    // ... and kGraphSteps of them by state buffer
+    cudaGraphExec_t graph_many[2] = {nullptr, nullptr};
     int sbytes = 8, tbytes = 8;  // storage / arithmetic bytes per value of the form
     const struct StepKernels* K = nullptr;
     // interior kernel shape (tmx_set_shape): TMX_SHAPE_*, planes per tile,
@@ -458,6 +460,17 @@ void error_flag_give(int* flag)
 
 namespace {
 
+void drop_graphs(tmx_handle* h)
+{
+    cudaGraphExec_t* all[6] = {&h->graph[0][0], &h->graph[0][1],   &h->graph[1][0],
+                               &h->graph[1][1], &h->graph_many[0], &h->graph_many[1]};
+    for (cudaGraphExec_t* g : all)
+        if (*g) {
+            cudaGraphExecDestroy(*g);
+            *g = nullptr;
+        }
+}
+
 void free_all(tmx_handle* h)
 {
     for (int s = 0; s < 2; s++) {
@@ -468,12 +481,7 @@ void free_all(tmx_handle* h)
         h->pop[s] = h->rho[s] = h->uin_d[s] = nullptr;
         h->mom[s] = nullptr;
     }
-    for (int a = 0; a < 2; a++)
-        for (int m = 0; m < 2; m++)
-            if (h->graph[a][m]) {
-                cudaGraphExecDestroy(h->graph[a][m]);
-                h->graph[a][m] = nullptr;
-            }
+    drop_graphs(h);
     if (h->fork) cudaEventDestroy(h->fork);
     if (h->join) cudaEventDestroy(h->join);
     if (h->join2) cudaEventDestroy(h->join2);
@@ -505,26 +513,26 @@ void free_all(tmx_handle* h)
 
 // The FP64 or FP32 step from buffer `cur`: one launch.  With ev (4 events) the edges
 // and the runs are launched one after the other, so that each event pair times
-// its part alone.
-int enqueue_run(tmx_handle* h, const tmx::StepPtrs& X, int cur, int write_macro, cudaEvent_t* ev)
+// its part alone.  overlap: launched behind another step of the same graph.
+int enqueue_run(tmx_handle* h, const tmx::StepPtrs& X, int cur, int write_macro, cudaEvent_t* ev, bool overlap)
 {
     const int ne = h->nb - h->nface, nr = h->nruns;
-    auto launch = [&](int nruns, int nedges) {
+    auto launch = [&](int nruns, int nedges) -> cudaError_t {
         const int per = h->run_nt / 32;  // a warp per edge node
         const int blocks = std::max(1, std::min(h->run_slots, (nedges + per - 1) / per + nruns));
-        h->K->run[h->run_nt > 128]<<<blocks, h->run_nt, h->K->run_smem(h->run_nt), h->stream>>>(
-            X, h->G, h->P, write_macro, h->runs, nruns, h->bnode + h->nface, h->bcls + h->nface, nedges, h->counters,
-            cur, h->error);
+        return launch_step(h->K->run[h->run_nt > 128], blocks, h->run_nt, h->K->run_smem(h->run_nt), h->stream, overlap,
+                           X, h->G, h->P, write_macro, h->runs, nruns, h->bnode + h->nface, h->bcls + h->nface, nedges,
+                           h->counters, cur, h->error);
     };
     if (ev) {
         TMX_CK(cudaEventRecord(ev[2], h->stream));
-        launch(0, ne);
+        TMX_CK(launch(0, ne));
         TMX_CK(cudaEventRecord(ev[3], h->stream));
         TMX_CK(cudaEventRecord(ev[0], h->stream));
-        launch(nr, 0);
+        TMX_CK(launch(nr, 0));
         TMX_CK(cudaEventRecord(ev[1], h->stream));
     } else {
-        launch(nr, ne);
+        TMX_CK(launch(nr, ne));
     }
     TMX_CK(cudaGetLastError());
     return TMX_OK;
@@ -535,7 +543,7 @@ int enqueue_run(tmx_handle* h, const tmx::StepPtrs& X, int cur, int write_macro,
 // bulk kernel on the main stream (FP64 and FP32: enqueue_run).  With ev (4 events) each
 // part is bracketed by its own pair of events.  The state and density buffers
 // flip together every step, so one parity index selects both.
-int enqueue_step(tmx_handle* h, int cur, int write_macro, cudaEvent_t* ev)
+int enqueue_step(tmx_handle* h, int cur, int write_macro, cudaEvent_t* ev, bool overlap = false)
 {
     const Geom& G = h->G;
     tmx::StepPtrs X;
@@ -548,7 +556,7 @@ int enqueue_step(tmx_handle* h, int cur, int write_macro, cudaEvent_t* ev)
     X.mcur = h->mom[1 - cur];
     X.uin1 = h->uin_d[0];
     X.uin2 = h->uin_d[1];
-    if (h->K->run[0]) return enqueue_run(h, X, cur, write_macro, ev);
+    if (h->K->run[0]) return enqueue_run(h, X, cur, write_macro, ev, overlap);
     TMX_CK(cudaEventRecord(h->fork, h->stream));
     TMX_CK(cudaStreamWaitEvent(h->aux, h->fork, 0));
     TMX_CK(cudaStreamWaitEvent(h->aux2, h->fork, 0));
@@ -598,23 +606,24 @@ int settled(const tmx_handle* h)
     return TMX_OK;
 }
 
-int advance(tmx_handle* h)
+int advance(tmx_handle* h, int steps = 1)
 {
-    h->cur = 1 - h->cur;
+    if (steps & 1) h->cur = 1 - h->cur;
     h->rcur = h->cur;
-    h->steps++;
+    h->steps += steps;
     return TMX_OK;
 }
 
-// One step through a captured graph (built on first use for this parity and
-// output flag).
-int graph_step(tmx_handle* h, int write_macro)
+// n steps (one, or kGraphSteps without macroscopic output) through a captured
+// graph, built on first use for this parity.
+int graph_steps(tmx_handle* h, int n, int write_macro)
 {
-    cudaGraphExec_t& ex = h->graph[h->cur][write_macro];
+    cudaGraphExec_t& ex = n > 1 ? h->graph_many[h->cur] : h->graph[h->cur][write_macro];
     if (!ex) {
         cudaGraph_t gr = nullptr;
         TMX_CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-        int rc = enqueue_step(h, h->cur, write_macro, nullptr);
+        int rc = TMX_OK;
+        for (int s = 0; s < n && rc == TMX_OK; s++) rc = enqueue_step(h, h->cur ^ (s & 1), write_macro, nullptr, s > 0);
         cudaError_t e = cudaStreamEndCapture(h->stream, &gr);
         if (rc) {
             if (gr) cudaGraphDestroy(gr);
@@ -626,7 +635,7 @@ int graph_step(tmx_handle* h, int write_macro)
         TMX_CK(e);
     }
     TMX_CK(cudaGraphLaunch(ex, h->stream));
-    return advance(h);
+    return advance(h, n);
 }
 
 int timed_step(tmx_handle* h, int write_macro, cudaEvent_t* ev)
@@ -916,12 +925,7 @@ int tmx_set_shape(tmx_handle* h, int kind, int zchunk)
     }
     h->shape = kind;
     h->zchunk = zchunk;
-    for (auto& row : h->graph)
-        for (auto& g : row)
-            if (g) {
-                cudaGraphExecDestroy(g);
-                g = nullptr;
-            }
+    drop_graphs(h);
     return TMX_OK;
 }
 
@@ -963,9 +967,11 @@ int tmx_step(tmx_handle* h, int nsteps)
     if (!h->inited) return fail(TMX_E_STATE, "tmx_step before tmx_init");
     if (nsteps < 0) return fail(TMX_E_INVALID, "negative step count");
     TMX_CK(cudaSetDevice(h->device));
-    for (int s = 0; s < nsteps; s++) {
-        int rc = graph_step(h, s == nsteps - 1);
+    for (int left = nsteps; left > 0;) {
+        const int n = left > kGraphSteps ? kGraphSteps : 1;
+        const int rc = graph_steps(h, n, left == 1);
         if (rc) return rc;
+        left -= n;
     }
     return TMX_OK;
 }

@@ -232,6 +232,7 @@ struct tmx_batch {
     int grid_faces = 0, grid_edges = 0, grid_run = 0;
     int nblocks = 0, nfaces = 0, nedges = 0, ntiles = 0, nactive = 0;
     cudaGraphExec_t graph[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
+    cudaGraphExec_t graph_many[2] = {nullptr, nullptr};  // kGraphSteps steps
 };
 
 namespace {
@@ -244,6 +245,11 @@ void drop_graphs(tmx_batch* b)
                 cudaGraphExecDestroy(g);
                 g = nullptr;
             }
+    for (auto& g : b->graph_many)
+        if (g) {
+            cudaGraphExecDestroy(g);
+            g = nullptr;
+        }
 }
 
 template <class E>
@@ -364,22 +370,23 @@ int rebuild(tmx_batch* b)
 // and end, boundary start and end) the interior kernel runs after the
 // boundary kernels in every form, so that each event pair times its kernels
 // alone (tmx_batch_step_timed).
-int enqueue(tmx_batch* b, int parity, int write_macro, cudaEvent_t* ev = nullptr)
+int enqueue(tmx_batch* b, int parity, int write_macro, cudaEvent_t* ev = nullptr, bool overlap = false)
 {
     if (b->B->run) {
         auto launch = [&](int what) {
-            b->B->run<<<b->grid_run, tmx::kRunBatchThreads, b->K->run_smem(tmx::kRunBatchThreads), b->stream>>>(
-                b->d_desc, b->d_runs, b->d_edges, b->d_counts, parity, write_macro, what, b->error);
+            return launch_step(b->B->run, b->grid_run, tmx::kRunBatchThreads, b->K->run_smem(tmx::kRunBatchThreads),
+                               b->stream, overlap, b->d_desc, b->d_runs, b->d_edges, b->d_counts, parity, write_macro,
+                               what, b->error);
         };
         if (ev) {
             TMX_CK(cudaEventRecord(ev[2], b->stream));
-            launch(2);
+            TMX_CK(launch(2));
             TMX_CK(cudaEventRecord(ev[3], b->stream));
             TMX_CK(cudaEventRecord(ev[0], b->stream));
-            launch(1);
+            TMX_CK(launch(1));
             TMX_CK(cudaEventRecord(ev[1], b->stream));
         } else {
-            launch(3);
+            TMX_CK(launch(3));
         }
         TMX_CK(cudaGetLastError());
         return TMX_OK;
@@ -418,15 +425,18 @@ int enqueue(tmx_batch* b, int parity, int write_macro, cudaEvent_t* ev = nullptr
     return TMX_OK;
 }
 
-int step_one(tmx_batch* b, int write_macro)
+// n steps (one, or kGraphSteps without macroscopic output) through a captured
+// graph, built on first use for this parity.
+int graph_steps(tmx_batch* b, int n, int write_macro)
 {
     const int p = b->parity;
-    cudaGraphExec_t& ge = b->graph[p][write_macro];
+    cudaGraphExec_t& ge = n > 1 ? b->graph_many[p] : b->graph[p][write_macro];
     if (!ge) {
         cudaGraph_t g = nullptr;
         cudaStreamCaptureMode mode = cudaStreamCaptureModeThreadLocal;
         TMX_CK(cudaStreamBeginCapture(b->stream, mode));
-        int rc = enqueue(b, p, write_macro);
+        int rc = TMX_OK;
+        for (int s = 0; s < n && rc == TMX_OK; s++) rc = enqueue(b, p ^ (s & 1), write_macro, nullptr, s > 0);
         cudaError_t e = cudaStreamEndCapture(b->stream, &g);
         if (rc) {
             if (g) cudaGraphDestroy(g);
@@ -438,8 +448,8 @@ int step_one(tmx_batch* b, int write_macro)
         TMX_CK(e);
     }
     TMX_CK(cudaGraphLaunch(ge, b->stream));
-    b->parity ^= 1;
-    b->steps++;
+    b->parity ^= n & 1;
+    b->steps += n;
     return TMX_OK;
 }
 
@@ -758,9 +768,11 @@ int tmx_batch_step(tmx_batch* b, int nsteps, int write_macro_last)
         int rc = rebuild(b);
         if (rc) return rc;
     }
-    for (int s = 0; s < nsteps; s++) {
-        int rc = step_one(b, (s == nsteps - 1 && write_macro_last) ? 1 : 0);
+    for (int left = nsteps; left > 0;) {
+        const int n = left > kGraphSteps ? kGraphSteps : 1;
+        const int rc = graph_steps(b, n, left == 1 && write_macro_last ? 1 : 0);
         if (rc) return rc;
+        left -= n;
     }
     for (auto& s : b->slots)
         if (s.used) s.steps += nsteps;

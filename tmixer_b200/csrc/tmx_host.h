@@ -130,6 +130,30 @@ inline void sweep_tiles(const Geom& G, int mixer, int ty, int zchunk, std::vecto
                     out.push_back(make_int4((mixer * 2 + b) | std::min(zchunk, G.nz - z0) << 20, x0, y0, z0));
 }
 
+// Steps of one captured graph where many are asked for (an even number: the
+// buffers are back in place).  A graph of its own per step costs a small mixer a
+// microsecond or two between steps.
+constexpr int kGraphSteps = 16;
+
+// Launch a step's kernel; overlap: as soon as the step before it in the stream
+// leaves room, which the kernel waits for by itself (step_wait).
+template <class... P, class... A>
+cudaError_t launch_step(void (*kernel)(P...), int blocks, int threads, int smem, cudaStream_t stream, bool overlap,
+                        A... args)
+{
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3((unsigned)blocks);
+    c.blockDim = dim3((unsigned)threads);
+    c.dynamicSmemBytes = (size_t)smem;
+    c.stream = stream;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &at;
+    c.numAttrs = overlap ? 1 : 0;
+    return cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+
 // Threads per block, and so nodes per run, of the FP64 step (FP32: 128): 256, whose 2 KB
 // copies get the most from DRAM, or 128 where the finer runs fill the SMs more
 // evenly (step by 128 / 256: 65,536 nodes 23.7 / 30.5 us, 524,288 nodes 116.4 /

@@ -23,9 +23,13 @@ __global__ void __launch_bounds__(128, 4) k_run128_f32(
     extern __shared__ __align__(16) unsigned char run_smem[];
     RunShared32<NT>& S = *(RunShared32<NT>*)run_smem;
     const int warp = threadIdx.x >> 5, nb = gridDim.x;
-    if (blockIdx.x == 0 && threadIdx.x == 0) counters[1 - parity] = 0;  // the next step's
+    const auto ready = [&] {
+        step_wait();
+        if (blockIdx.x == 0 && threadIdx.x == 0) counters[1 - parity] = 0;  // the next step's
+    };
+    step_begin();
     run32_loop<NT>([&](const int4&) { return RunView32{&X, &G, &P}; }, runs, nruns, blockIdx.x, nb, counters + parity,
-                   write_macro, S, error, [&] {
+                   write_macro, S, error, ready, [&] {
                        const int at = (int)(blockIdx.x + nb - nruns % nb) % nb;
                        for (int e = at * (NT / 32) + warp; e < ne; e += nb * (NT / 32))
                            run32_edge(X, G, P, write_macro, enode[e], ecls[e], S.edge[warp]);
@@ -42,13 +46,17 @@ __global__ void __launch_bounds__(kRunBatchThreads, 512 / kRunBatchThreads) k_ru
     RunShared32<NT>& S = *(RunShared32<NT>*)run_smem;
     const int warp = threadIdx.x >> 5, nb = gridDim.x;
     const int nruns = what & 1 ? counts[4] : 0, ne = what & 2 ? counts[2] : 0;
-    if (blockIdx.x == 0 && threadIdx.x == 0) counts[5 + (1 - parity)] = 0;  // the next step's
+    const auto ready = [&] {
+        step_wait();
+        if (blockIdx.x == 0 && threadIdx.x == 0) counts[5 + (1 - parity)] = 0;  // the next step's
+    };
+    step_begin();
     run32_loop<NT>(
         [&](const int4& t) {
             const MixerDesc& d = D[run_mixer(t)];
             return RunView32{&d.X[parity], &d.G, &d.P};
         },
-        runs, nruns, blockIdx.x, nb, counts + 5 + parity, write_macro, S, error, [&] {
+        runs, nruns, blockIdx.x, nb, counts + 5 + parity, write_macro, S, error, ready, [&] {
             const int at = (int)(blockIdx.x + nb - nruns % nb) % nb;
             for (int e = at * (NT / 32) + warp; e < ne; e += nb * (NT / 32)) {
                 const int2 t = edges[e];

@@ -97,16 +97,17 @@ __device__ __noinline__ void run32_edge(const StepPtrs& X, const Geom& G, const 
 
 // The runs of one block: two by its number, then by the launch's counter.
 // get(t) gives the buffers, geometry and constants of run t's mixer.  error: set
-// when a copy does not arrive.  meanwhile(): what the warps do while the first
-// run's copies are on their way.
-template <int NT, class Get, class Mean>
+// when a copy does not arrive.  ready(): waits for the step before; meanwhile():
+// what the warps do while the first run's copies are on their way.
+template <int NT, class Get, class Ready, class Mean>
 __device__ __forceinline__ void run32_loop(const Get& get, const int4* __restrict__ runs, int nruns, int first,
                                            int nblocks, int* __restrict__ counter, int write_macro,
-                                           RunShared32<NT>& S, int* error, const Mean& meanwhile)
+                                           RunShared32<NT>& S, int* error, const Ready& ready, const Mean& meanwhile)
 {
     const int t = threadIdx.x, warp = t >> 5;
     constexpr int kWarps = NT / 32;
     if (first >= nruns) {  // (the whole block)
+        ready();
         meanwhile();
         return;
     }
@@ -119,13 +120,13 @@ __device__ __forceinline__ void run32_loop(const Get& get, const int4* __restric
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    if (warp == 0) {
-        const RunView32 M = get(S.run[0]);
-        run32_prepare(S, 0, *M.G);
-        __syncwarp();
-        run32_fill(S, 0, M, 0);
-    }
+    if (warp == 0) run32_prepare(S, 0, *get(S.run[0]).G);
     if (warp == kWarps - 1 && (S.run[1].y & 511)) run32_prepare(S, 1, *get(S.run[1]).G);
+    ready();
+    if (warp == 0) {
+        __syncwarp();
+        run32_fill(S, 0, get(S.run[0]), 0);
+    }
     meanwhile();
     unsigned phase = 0;
     int ord = 0;

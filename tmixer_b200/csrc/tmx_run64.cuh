@@ -199,16 +199,17 @@ __device__ __noinline__ void run_edge(const StepPtrs& X, const Geom& G, const Ph
 
 // The runs of one block: the first by its number, then by the launch's counter.
 // get(t) gives the buffers, geometry and constants of run t's mixer.  error: set
-// when a copy does not arrive.  meanwhile(): what the warps do while the first
-// run's copies are on their way.
-template <int NT, class Get, class Mean>
+// when a copy does not arrive.  ready(): waits for the step before; meanwhile():
+// what the warps do while the first run's copies are on their way.
+template <int NT, class Get, class Ready, class Mean>
 __device__ __forceinline__ void run_loop(const Get& get, const int4* __restrict__ runs, int nruns, int first,
                                          int nblocks, int* __restrict__ counter, int write_macro, RunShared<NT>& S,
-                                         int* error, const Mean& meanwhile)
+                                         int* error, const Ready& ready, const Mean& meanwhile)
 {
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     constexpr int kWarps = NT / 32;
     if (first >= nruns) {  // (the whole block)
+        ready();
         meanwhile();
         return;
     }
@@ -221,9 +222,10 @@ __device__ __forceinline__ void run_loop(const Get& get, const int4* __restrict_
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
+    if (warp == 0) run_prepare(S, 0, *get(S.run[0]).G);
+    ready();
     if (warp == 0) {
         const RunView M = get(S.run[0]);
-        run_prepare(S, 0, *M.G);
         __syncwarp();
         run_fill(S, 0, 0, M, 0);
         run_fill(S, 1, 0, M, 1);
