@@ -508,7 +508,7 @@ def run_ours(args, dist: Dist) -> dict | None:
             "data": "synthetic",
             "form": form_text[args.form], "config": config_dict(workload_params(), dist.world),
             "roofline": roofline, "cpu_baseline": cpu, "e2e": e2e, "clocks": clk,
-            "gpu_launches": (3 if args.form == "fp16" else 1) * args.steps, "forms": forms,
+            "gpu_launches": (2 if args.form == "fp16" else 1) * args.steps, "forms": forms,
             "reference_case": refcase, "batched": batched,
             "served": served}
 

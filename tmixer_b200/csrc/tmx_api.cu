@@ -94,7 +94,7 @@ struct tmx_handle {
     // and the sweep kernels' tile list and grid
     int shape = TMX_SHAPE_FLAT, zchunk = 8;
     int4* tiles = nullptr;
-    int ntiles = 0, sweep_blocks = 0;
+    int ntiles = 0, sweep_slots = 0;  // tiles, and blocks of their kernel that the GPU holds at once
 };
 
 const StepKernels tmx_host::kForms[3] = {
@@ -538,11 +538,39 @@ int enqueue_run(tmx_handle* h, const tmx::StepPtrs& X, int cur, int write_macro,
     return TMX_OK;
 }
 
+// The FP16 step with the wall rows in the tiles' launch.  Where its blocks with
+// the edges' fill half of the GPU at most the edges are in it too (1,000 to 22,000
+// nodes 13.1 to 16.7 us a step against 16.4 to 18.3 in three kernels); else the edge
+// kernel runs beside it (edges by warps of the tile kernel hold up the tiles that
+// share an SM with them; in it / beside: 43,904 nodes 20.6 / 15.6 us, 65,536 19.7 /
+// 18.1, 221,184 33.3 / 27.4).
+int enqueue_sweep(tmx_handle* h, const SweepShape* sh, const tmx::StepPtrs& X, int write_macro, bool overlap)
+{
+    // the wall rows are the faces that the tiles leave, the first of the list
+    const int nw = h->nface - h->nswept, ne = h->nb - h->nface, nt = sh->threads();
+    const int wb = (nw + nt - 1) / nt, eb = (ne + nt / 32 - 1) / (nt / 32);
+    const bool one = 2 * (h->ntiles + wb + eb) <= h->sweep_slots;
+    const bool beside = !one && ne > 0;
+    if (beside) {
+        const int bt = tmx::kBoundaryThreadsHost, nl = tmx::kBoundaryLanesHost;
+        TMX_CK(cudaEventRecord(h->fork, h->stream));
+        TMX_CK(cudaStreamWaitEvent(h->aux2, h->fork, 0));
+        h->K->edges<<<(nl * ne + bt - 1) / bt, bt, 0, h->aux2>>>(X, h->bnode + h->nface, h->bcls + h->nface, ne, h->G,
+                                                                 h->P, write_macro);
+        TMX_CK(cudaEventRecord(h->join2, h->aux2));
+    }
+    TMX_CK(launch_step(sh->single, h->ntiles + wb + (one ? eb : 0), nt, sh->smem(), h->stream, one && overlap, X, h->G,
+                       h->P, write_macro, h->tiles, h->ntiles, h->bnode, h->bcls, nw, h->nface, one ? ne : 0));
+    if (beside) TMX_CK(cudaStreamWaitEvent(h->stream, h->join2, 0));
+    TMX_CK(cudaGetLastError());
+    return TMX_OK;
+}
+
 // Queue one step from buffer `cur`: the face and the edge kernel on the two
 // auxiliary streams, forked from and joined back into the main stream, and the
-// bulk kernel on the main stream (FP64 and FP32: enqueue_run).  With ev (4 events) each
-// part is bracketed by its own pair of events.  The state and density buffers
-// flip together every step, so one parity index selects both.
+// bulk kernel on the main stream (FP64 and FP32: enqueue_run).  With ev (4
+// events) each part is bracketed by its own pair of events.  The state and density
+// buffers flip together every step, so one parity index selects both.
 int enqueue_step(tmx_handle* h, int cur, int write_macro, cudaEvent_t* ev, bool overlap = false)
 {
     const Geom& G = h->G;
@@ -557,14 +585,19 @@ int enqueue_step(tmx_handle* h, int cur, int write_macro, cudaEvent_t* ev, bool 
     X.uin1 = h->uin_d[0];
     X.uin2 = h->uin_d[1];
     if (h->K->run[0]) return enqueue_run(h, X, cur, write_macro, ev, overlap);
+    // FP16 by up to four rounds of tiles: the wall rows with them.  Beyond, and for
+    // the timed parts, a face kernel: tiles without the walls' and edges' code beside
+    // them run faster (together / apart: 524,288 nodes 55.2 / 56.4 us, 1.8M 149.4 /
+    // 150.6, 4.2M 318.6 / 317.7, 4.9M 428 / 421).
+    const SweepShape* sh = sweep_shape(h->shape);
+    if (sh && !ev && h->ntiles <= 4 * h->sweep_slots) return enqueue_sweep(h, sh, X, write_macro, overlap);
     TMX_CK(cudaEventRecord(h->fork, h->stream));
     TMX_CK(cudaStreamWaitEvent(h->aux, h->fork, 0));
     TMX_CK(cudaStreamWaitEvent(h->aux2, h->fork, 0));
     if (ev) TMX_CK(cudaEventRecord(ev[2], h->aux));
     const int nf = h->nface, ne = h->nb - h->nface;
     const int bt = tmx::kBoundaryThreadsHost, nl = tmx::kBoundaryLanesHost;  // nl threads per face
-    // with a sweep shape the interior kernel updates the last nswept faces
-    const int nfk = sweep_shape(h->shape) ? nf - h->nswept : nf;
+    const int nfk = sh ? nf - h->nswept : nf;  // a sweep shape's tiles update the last nswept faces
     if (nfk > 0)
         h->K->faces<<<(nl * nfk + bt - 1) / bt, bt, 0, h->aux>>>(X, h->bnode, h->bcls, nfk, G, h->P, write_macro);
     if (ne > 0)
@@ -584,9 +617,8 @@ int enqueue_step(tmx_handle* h, int cur, int write_macro, cudaEvent_t* ev, bool 
         TMX_CK(cudaStreamWaitEvent(h->stream, h->join2, 0));
     }
     if (ev) TMX_CK(cudaEventRecord(ev[0], h->stream));
-    if (const SweepShape* sh = sweep_shape(h->shape))
-        sh->single<<<h->sweep_blocks, sh->threads(), sh->smem(), h->stream>>>(X, G, h->P, write_macro, h->tiles,
-                                                                             h->ntiles);
+    if (sh)
+        sh->tiles<<<h->ntiles, sh->threads(), sh->smem(), h->stream>>>(X, G, h->P, write_macro, h->tiles, h->ntiles);
     else
         h->K->bulk<<<h->bulk_blocks, 256, 0, h->stream>>>(X, G, h->P, write_macro);
     if (ev) TMX_CK(cudaEventRecord(ev[1], h->stream));
@@ -921,7 +953,11 @@ int tmx_set_shape(tmx_handle* h, int kind, int zchunk)
         cudaFree(h->tiles);
         h->tiles = d;
         h->ntiles = (int)t.size();
-        h->sweep_blocks = std::max(1, h->ntiles);
+        int per = 1, sms = 148;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)sh->single, sh->threads(), sh->smem());
+        cudaGetLastError();
+        h->sweep_slots = sms * std::max(1, per);
     }
     h->shape = kind;
     h->zchunk = zchunk;

@@ -396,7 +396,9 @@ int enqueue(tmx_batch* b, int parity, int write_macro, cudaEvent_t* ev = nullptr
     TMX_CK(cudaStreamWaitEvent(b->aux2, b->fork, 0));
     if (ev) TMX_CK(cudaEventRecord(ev[2], b->aux));
     const int bt = tmx::kBoundaryThreadsHost;
-    b->B->faces<<<b->grid_faces, bt, 0, b->aux>>>(b->d_desc, b->d_faces, b->d_counts, parity, write_macro);
+    // (a sweep shape's kernel takes the faces that its tiles leave)
+    if (!b->sweep)
+        b->B->faces<<<b->grid_faces, bt, 0, b->aux>>>(b->d_desc, b->d_faces, b->d_counts, parity, write_macro);
     b->B->edges<<<b->grid_edges, bt, 0, b->aux2>>>(b->d_desc, b->d_edges, b->d_counts, parity, write_macro);
     TMX_CK(cudaEventRecord(b->join2, b->aux2));
     if (ev) {
@@ -412,7 +414,8 @@ int enqueue(tmx_batch* b, int parity, int write_macro, cudaEvent_t* ev = nullptr
     if (ev) TMX_CK(cudaEventRecord(ev[0], b->stream));
     if (const SweepShape* sh = b->sweep ? sweep_shape(b->sweep) : nullptr)
         sh->batch<<<b->grid_sweep[b->sweep], sh->threads(), sh->smem(), b->stream>>>(b->d_desc, b->d_tiles,
-                                                                                    b->d_counts, parity, write_macro);
+                                                                                    b->d_faces, b->d_counts, parity,
+                                                                                    write_macro);
     else
         b->B->bulk[b->variant]<<<b->grid_bulk[b->variant], kBulkThreads[b->variant], 0, b->stream>>>(
             b->d_desc, b->d_blocks, b->d_counts, parity, write_macro);

@@ -1924,13 +1924,74 @@ __device__ __forceinline__ void load_desc(StepDesc& dst, const MixerDesc* __rest
     for (int e = threadIdx.x; e < nw; e += blockDim.x) d[e] = e < nx ? __ldg(sx + e) : __ldg(sg + (e - nx));
 }
 
-// The FP16 form's interior as tiles (sweep_tile): 32 x 8 threads (two blocks
-// per SM) or 32 x 4 (four).  A single mixer launches a block per tile, a batch a
-// persistent grid whose blocks take the next tile from a counter: tiles differ
-// (wall planes, ragged columns, blocks that the boundary kernels delay), and in
-// a fixed share of them the last block was 8% late (64 mixers, the interior
-// alone: 3.23 -> 2.95 ms; W=64 321 -> 299 us).  Dynamic shared
-// memory: sweep_smem_host(TY).
+// Steps that follow each other in one graph overlap (programmatic dependent
+// launch): a step lets the next one's blocks start as soon as its own leave
+// room, and they set up what no step changes (the run kernels' barriers, the first
+// run's entry and offsets) before they wait for this one to end.
+__device__ __forceinline__ void step_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void step_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// One face node of a y wall row or of the outlet row (K_FACE_YT, K_FACE_Y1,
+// K_OUTLET) by one thread, the reduced-precision forms' operations in
+// boundary_lane_lp's order: the flow pulled and closed, the species the interior
+// neighbour's pulls.  The rows are contiguous, so a warp's accesses are too.
+template <class PR>
+__device__ __forceinline__ void wall_row_node(const StepPtrs& X, const Geom& G, const Phys& P, int write_macro, int g,
+                                              int cls)
+{
+    using T = typename PR::T;
+    const long long ps = G.ps;
+    const int b = g >= G.base[1], nx = box_nx(G, b), sz = nx * box_ny(G, b);
+    const int dy = cls == K_FACE_YT ? -1 : 1, gn = g + dy * nx;
+    const PopGlobal<PR> pop{(const typename PR::S*)X.pin, ps};
+    const RecGlobal rec{X.mprev};
+    float2 p01[19], p23[19];
+#pragma unroll
+    for (int q = 0; q < 19; q++) {
+        float4 mf = make_float4(0.f, 0.f, 0.f, 0.f), ms = mf;
+        float2 v01;
+        const int off = EX(q) + EY(q) * nx + EZ(q) * sz;
+        if constexpr (PR::kMoments) rec(q, gn - off, mf, ms);
+        PR::decode_raw(pop(q, gn - off), EX(q), EY(q), EZ(q), (float)wq(q), mf, ms, p01[q], p23[q]);
+        p01[q].x = T(0);
+        if (EY(q) != dy) {
+            float2 v23;
+            if constexpr (PR::kMoments) rec(q, g - off, mf, ms);
+            PR::decode_raw(pop(q, g - off), EX(q), EY(q), EZ(q), (float)wq(q), mf, ms, v01, v23);
+            p01[q].x = v01.x;
+        }
+    }
+    T v[19];
+#pragma unroll
+    for (int q = 0; q < 19; q++) v[q] = p01[q].x;
+    wall_flow_closure(cls, T(P.rho_out), v);
+#pragma unroll
+    for (int q = 0; q < 19; q++) p01[q].x = v[q];
+    lp_finish<PR>(X, G, P, write_macro, g, p01, p23, cls == K_OUTLET, true);
+}
+// (out of line, like the edges: their registers are not the tiles' concern)
+template <class PR>
+__device__ __noinline__ void sweep_wall(const StepPtrs& X, const Geom& G, const Phys& P, int write_macro, int g, int cls)
+{
+    wall_row_node<PR>(X, G, P, write_macro, g, cls);
+}
+template <class PR>
+__device__ __noinline__ void sweep_edge(const StepPtrs& X, const Geom& G, const Phys& P, int write_macro, int g, int cls,
+                                        typename PR::T* buf)
+{
+    edge_node<PR>(X, G, P, write_macro, g, cls, buf);
+}
+
+// The FP16 form's step by tiles (sweep_tile): 32 x 8 threads (two blocks per SM)
+// or 32 x 4 (four).  Single mixer: a block per tile (k_sweep), and in one launch
+// with them (k_sweepw) blocks of a thread per wall row node (bnode[0..nw)) and of
+// a warp per edge node (bnode[e0..e0 + ne)), which fill the end of the launch.
+// Batch: a persistent grid whose blocks take the next tile, then the next
+// kSweepWalls entries of the wall rows, from a counter (the edges are a kernel
+// beside it).  Blocks differ (wall planes, ragged
+// columns), and in a fixed share of the tiles the last block was 8% late (64
+// mixers, the interior alone: 3.23 -> 2.95 ms; W=64 321 -> 299 us).  Dynamic
+// shared memory: sweep_smem_host(TY).
 #define TMX_SWEEP_KERNEL(PR, NAME, TY, MINB)                                                                      \
     __global__ void __launch_bounds__(kSweepX * TY, MINB) k_sweep##TY##_##NAME(                                  \
         StepPtrs X, Geom G, Phys P, int write_macro, const int4* __restrict__ tiles, int ntiles)                 \
@@ -1940,25 +2001,57 @@ __device__ __forceinline__ void load_desc(StepDesc& dst, const MixerDesc* __rest
         float4* B = A + 4 * (TY + 2) * (kSweepX + 2);                                                           \
         for (int t = blockIdx.x; t < ntiles; t += gridDim.x) sweep_tile<PR, TY>(X, G, P, write_macro, tiles[t], A, B); \
     }                                                                                                           \
+    __global__ void __launch_bounds__(kSweepX * TY, MINB) k_sweepw##TY##_##NAME(                                 \
+        const __grid_constant__ StepPtrs X, const __grid_constant__ Geom G, const __grid_constant__ Phys P,      \
+        int write_macro, const int4* __restrict__ tiles, int ntiles, const int* __restrict__ bnode,              \
+        const unsigned char* __restrict__ bcls, int nw, int e0, int ne)                                          \
+    {                                                                                                           \
+        extern __shared__ float4 sweep_smem[];                                                                  \
+        constexpr int NT = kSweepX * TY;                                                                        \
+        float4* A = sweep_smem;                                                                                 \
+        float4* B = A + 4 * (TY + 2) * (kSweepX + 2);                                                           \
+        step_begin();                                                                                           \
+        step_wait();                                                                                            \
+        const int t = blockIdx.x, w = t - ntiles, e = w - (nw + NT - 1) / NT;                                   \
+        if (w < 0) {                                                                                            \
+            sweep_tile<PR, TY>(X, G, P, write_macro, tiles[t], A, B);                                           \
+        } else if (e < 0) {                                                                                     \
+            const int at = w * NT + threadIdx.x;                                                                \
+            if (at < nw) sweep_wall<PR>(X, G, P, write_macro, bnode[at], bcls[at]);                             \
+        } else {                                                                                                \
+            const int wp = threadIdx.x >> 5, at = e * (NT / 32) + wp;                                           \
+            if (at < ne)                                                                                        \
+                sweep_edge<PR>(X, G, P, write_macro, bnode[e0 + at], bcls[e0 + at], (PR::T*)A + wp * kEdgeBuf); \
+        }                                                                                                       \
+    }                                                                                                           \
     __global__ void __launch_bounds__(kSweepX * TY, MINB) k_sweep_batch##TY##_##NAME(                            \
-        const MixerDesc* __restrict__ D, const int4* __restrict__ tiles, int* __restrict__ counts,               \
-        int parity, int write_macro)                                                                            \
+        const MixerDesc* __restrict__ D, const int4* __restrict__ tiles, const int2* __restrict__ walls,         \
+        int* __restrict__ counts, int parity, int write_macro)                                                  \
     {                                                                                                           \
         extern __shared__ float4 sweep_smem[];                                                                  \
         float4* A = sweep_smem;                                                                                 \
         float4* B = A + 4 * (TY + 2) * (kSweepX + 2);                                                           \
         __shared__ StepDesc d;                                                                                  \
         __shared__ int next;                                                                                    \
-        const int n = counts[3];                                                                                \
+        const int n = counts[3], nw = counts[1];                                                                \
         if (blockIdx.x == 0 && threadIdx.x == 0) counts[5 + (1 - parity)] = 0; /* the next step's */             \
-        for (int t = blockIdx.x; t < n; t = next) {                                                             \
-            const int4 tl = tiles[t];                                                                           \
+        for (int t = blockIdx.x; t < n + (nw + kSweepWalls - 1) / kSweepWalls; t = next) {                      \
+            const int at = (t - n) * kSweepWalls, m = t < n ? (tiles[t].x & 0xfffff) >> 1 : walls[at].y >> 8;    \
             __syncthreads();                                                                                    \
             /* the tile after this one, by the launch's counter */                                              \
             if (threadIdx.x == 0) next = gridDim.x + atomicAdd(counts + 5 + parity, 1);                         \
-            load_desc(d, D, (tl.x & 0xfffff) >> 1, parity);                                                                 \
+            load_desc(d, D, m, parity);                                                                         \
             __syncthreads();                                                                                    \
-            sweep_tile<PR, TY>(d.X, d.G, d.P, write_macro, tl, A, B);                                           \
+            if (t < n) {                                                                                        \
+                sweep_tile<PR, TY>(d.X, d.G, d.P, write_macro, tiles[t], A, B);                                 \
+            } else {                                                                                            \
+                for (int e = at + threadIdx.x; e < nw && e < at + kSweepWalls; e += kSweepX * TY) {             \
+                    const int2 v = walls[e];                                                                    \
+                    if (v.x < 0) continue;                                                                      \
+                    const MixerDesc& o = D[v.y >> 8];                                                           \
+                    sweep_wall<PR>(o.X[parity], o.G, o.P, write_macro, v.x, v.y & 255);                         \
+                }                                                                                               \
+            }                                                                                                   \
         }                                                                                                       \
     }
 #define TMX_DEFINE_SWEEP_KERNELS(PR, NAME) \

@@ -86,16 +86,17 @@ void inlet_scale(const tmx_case& c, const std::vector<double>& raw, double avera
 // memory.
 struct SweepShape {
     int kind, ty;
-    void (*single)(tmx::StepPtrs, Geom, Phys, int, const int4*, int);
-    void (*batch)(const tmx::MixerDesc*, const int4*, int*, int, int);
+    void (*tiles)(tmx::StepPtrs, Geom, Phys, int, const int4*, int);
+    void (*single)(tmx::StepPtrs, Geom, Phys, int, const int4*, int, const int*, const unsigned char*, int, int, int);
+    void (*batch)(const tmx::MixerDesc*, const int4*, const int2*, int*, int, int);
     int threads() const { return 32 * ty; }
     int smem() const { return tmx::sweep_smem_host(ty); }
 };
 inline const SweepShape* sweep_shape(int kind)
 {
     static const SweepShape shapes[] = {
-        {TMX_SHAPE_SWEEP8, 8, tmx::k_sweep8_f16, tmx::k_sweep_batch8_f16},
-        {TMX_SHAPE_SWEEP4, 4, tmx::k_sweep4_f16, tmx::k_sweep_batch4_f16},
+        {TMX_SHAPE_SWEEP8, 8, tmx::k_sweep8_f16, tmx::k_sweepw8_f16, tmx::k_sweep_batch8_f16},
+        {TMX_SHAPE_SWEEP4, 4, tmx::k_sweep4_f16, tmx::k_sweepw4_f16, tmx::k_sweep_batch4_f16},
     };
     for (const SweepShape& e : shapes)
         if (e.kind == kind) return &e;
@@ -109,6 +110,8 @@ inline cudaError_t sweep_allow_smem()
         const SweepShape* sh = sweep_shape(kind);
         cudaError_t e = cudaFuncSetAttribute((const void*)sh->single, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              sh->smem());
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute((const void*)sh->tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, sh->smem());
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute((const void*)sh->batch, cudaFuncAttributeMaxDynamicSharedMemorySize, sh->smem());
         if (e != cudaSuccess) return e;

@@ -113,11 +113,16 @@ __host__ __device__ constexpr int sweep_end(int x0, int nx)
 {
     return x0 + 32 >= nx ? nx : (x0 + 32 == nx - 1 ? x0 + 31 : x0 + 32);
 }
+constexpr int kSweepWalls = 256;  // wall row entries that a batch's block takes at a time
 #define TMX_DECLARE_SWEEP(SUFFIX)                                                                               \
     __global__ void k_sweep##SUFFIX##_f16(StepPtrs X, Geom G, Phys P, int write_macro, const int4* tiles,     \
-                                          int ntiles);                                                        \
-    __global__ void k_sweep_batch##SUFFIX##_f16(const MixerDesc* D, const int4* tiles, int* counts,           \
-                                                int parity, int write_macro);
+                                          int ntiles);                                                         \
+    __global__ void k_sweepw##SUFFIX##_f16(const __grid_constant__ StepPtrs X, const __grid_constant__ Geom G, \
+                                          const __grid_constant__ Phys P, int write_macro, const int4* tiles,  \
+                                          int ntiles, const int* bnode, const unsigned char* bcls, int nw,     \
+                                          int e0, int ne);                                                     \
+    __global__ void k_sweep_batch##SUFFIX##_f16(const MixerDesc* D, const int4* tiles, const int2* walls,     \
+                                                int* counts, int parity, int write_macro);
 TMX_DECLARE_SWEEP(8)
 TMX_DECLARE_SWEEP(4)
 constexpr int sweep_smem_host(int ty) { return 2 * 4 * (ty + 2) * 34 * 16; }

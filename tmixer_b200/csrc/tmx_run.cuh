@@ -42,13 +42,6 @@ __device__ __forceinline__ void bulk_load(unsigned dst, const void* src, unsigne
                  : "memory");
 }
 
-// Steps that follow each other in one graph overlap (programmatic dependent
-// launch): a step lets the next one's blocks start as soon as its own leave
-// room, and they set up what no step changes (barriers, the first run's entry and
-// offsets) before they wait for this one to end.
-__device__ __forceinline__ void step_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void step_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 // A run, the same for the whole block: its first node, nodes, kind and box, and
 // the strides of its sources.  Direction q of node h (the node itself for the
 // flow, node + shift for the species) comes from h - ex - ez * sz, for ey = 1
