@@ -3,7 +3,8 @@
 // classification; every direction of every field is pulled from the source of
 // the general rule (pull_src), the species of a copied face from the interior
 // neighbour's, in the copied window's place that the kernel reads; and every
-// window is aligned and inside the population buffer.  Arguments: inx iny nz mnx mny ia, repeated.
+// window is aligned and inside the population buffer.  Also the FP16 form's tiles
+// (check_tiles).  Arguments: inx iny nz mnx mny ia, repeated.
 #include <cstdio>
 #include <cstdlib>
 #include <vector>
@@ -100,6 +101,52 @@ static int check(const Geom& G, int nt)
     return 0;
 }
 
+// The tiles of the FP16 form: every node of the interior rows (the x faces
+// among them, the opening's ends not) in exactly one, the species' source of an x wall
+// in the same group of lanes, and every record of a node's sources staged in the
+// place that the node reads.
+static int check_tiles(const Geom& G, int ty, int planes, bool groups)
+{
+    std::vector<int4> tiles;
+    tmx_host::sweep_tiles(G, 5, ty, planes, groups, tiles);
+    std::vector<char> seen(G.nnodes, 0);
+    const int pitch = sweep_pitch(groups);
+    for (const int4& t : tiles) {
+        const int b = t.x & 1, s = t.x >> 29, z1 = t.w + (t.x >> 20 & 511), w = 32 >> s;
+        const int nx = box_nx(G, b), ny = box_ny(G, b), x1 = sweep_end(t.y, nx, w);
+        if ((t.x & 0xfffff) >> 1 != 5 || (!groups && s)) return std::printf("mixer or groups\n"), 1;
+        if (x1 - t.y < 2 || x1 - t.y > w || t.w < 2 || z1 > G.nz) return std::printf("tile\n"), 1;
+        for (int warp = 0; warp < ty; warp++)
+            for (int lane = 0; lane < 32; lane++) {
+                const SweepLane at = sweep_lane(s, lane, warp, ty);
+                const int x = t.y + at.x, y = t.z + at.y;
+                if (x >= x1 || y >= ny || (b ? y < 1 : y >= ny - 1)) continue;
+                if (b == 0 && y == 0 && (x < G.ia || x >= G.ib - 1)) continue;
+                for (int k = t.w; k < z1; k++)
+                    if (seen[box_base(G, b) + ((k - 1) * ny + y) * nx + x]++) return std::printf("twice\n"), 1;
+                const int from = x == 0 ? lane + 1 : (x == nx - 1 ? lane - 1 : lane);
+                if (from >> (5 - s) != lane >> (5 - s)) return std::printf("wall's neighbour\n"), 1;
+                for (int dx = -1; dx <= 1; dx++)
+                    for (int dy = -1; dy <= 1; dy++) {
+                        const int col = at.col + 1 + dx, row = warp + 1 + dy, c = sweep_group(s, col);
+                        if (col < 0 || col >= pitch || c != lane >> (5 - s) || sweep_column(s, col) != at.x + dx ||
+                            c * ty + row - 1 != at.y + dy)
+                            return std::printf("record\n"), 1;
+                    }
+            }
+    }
+    for (int b = 0; b < 2; b++)
+        for (int k = 2; k < G.nz; k++)
+            for (int y = 0; y < box_ny(G, b); y++)
+                for (int x = 0; x < box_nx(G, b); x++) {
+                    bool in = b ? y > 0 : y < G.iny - 1;
+                    if (b == 0 && y == 0) in = x >= G.ia && x < G.ib - 1;
+                    if (seen[box_base(G, b) + ((k - 1) * box_ny(G, b) + y) * box_nx(G, b) + x] != (in ? 1 : 0))
+                        return std::printf("cover %d %d %d %d\n", b, x, y, k), 1;
+                }
+    return 0;
+}
+
 int main(int argc, char** argv)
 {
     for (int a = 1; a + 5 < argc; a += 6) {
@@ -112,7 +159,9 @@ int main(int argc, char** argv)
         c.ia = atoi(argv[a + 5]);
         Geom G;
         tmx_host::geometry_of(c, G);
-        if (check(G, 128) || check(G, 256)) {
+        int bad = check(G, 128) || check(G, 256);
+        for (int v = 0; v < 12 && !bad; v++) bad = check_tiles(G, v & 1 ? 8 : 4, v < 4 ? 1 : (v < 8 ? 3 : 1000), v & 2);
+        if (bad) {
             std::printf("case %d %d %d %d %d %d\n", c.inx, c.iny, c.nz, c.mnx, c.mny, c.ia);
             return 1;
         }

@@ -67,6 +67,32 @@ def test_sweep_equals_flat(gpu, name):
         assert _same(got, want), (name, shape, zchunk)
 
 
+# boxes whose columns take 32-, 16- and 8-wide tiles of a batch (sweep_tiles):
+# one group and less, each remainder, and a last column that is never alone
+GROUP_BOXES = [(16, 5, 5, 8, 9, 4), (20, 9, 4, 9, 17, 5), (44, 6, 5, 18, 35, 9), (50, 11, 5, 24, 20, 3),
+               (73, 7, 4, 33, 9, 20), (97, 18, 5, 41, 34, 30)]
+
+
+@pytest.mark.parametrize("kind,zchunk", [(T.SHAPE_SWEEP4, 4), (T.SHAPE_SWEEP8, 2), (T.SHAPE_SWEEP4, 1)])
+def test_batch_groups_equal_flat(gpu, kind, zchunk):
+    specs = []
+    for n, (inx, iny, nz, mnx, mny, ia) in enumerate(GROUP_BOXES):
+        s = to_spec(dict(ref_like(inx, iny, nz, mnx, mny, umean=0.02 + 0.01 * n, k=0.5), ia=ia))
+        s.precision = T.TMX_FP16
+        specs.append(s)
+    with T.Batch(T.TMX_FP16, budget=sum(T.Batch.footprint(s) for s in specs) + (1 << 20)) as B:
+        slots = [B.add(s) for s in specs]
+        B.set_sweep(kind, zchunk)
+        B.step(12)
+        for s, m in zip(specs, slots):
+            with T.Solver(s) as one:
+                one.set_shape(T.SHAPE_FLAT, 8)
+                one.init()
+                one.step(12)
+                for b in (0, 1):
+                    assert _same([B.field(m, b, f) for f in T.FIELDS], [one.field(b, f) for f in T.FIELDS])
+
+
 def test_sweep_shape_rejected_outside_fp16(gpu):
     spec = T.w_layout(4, u_max=0.05, tau_f=0.6, tau_c=0.6, k=1e-3, rho=1.0, precision=T.TMX_FP32)
     with T.Solver(spec) as s:

@@ -1,5 +1,5 @@
-"""The FP64 step's run lists against the general pull and class rules, on the
-CPU: native/run_lists.cu over the smallest boxes, the test cases' and random
+"""The run lists of the FP64 and FP32 steps against the general pull and class
+rules, and the cover of the FP16 form's tiles, on the CPU: native/run_lists.cu over the smallest boxes, the test cases' and random
 ones (openings next to the inlets, rows shorter and longer than a warp)."""
 import os
 import random

@@ -559,7 +559,7 @@ int enqueue_sweep(tmx_handle* h, const SweepShape* sh, const tmx::StepPtrs& X, i
                                                                  h->P, write_macro);
         TMX_CK(cudaEventRecord(h->join2, h->aux2));
     }
-    TMX_CK(launch_step(sh->single, h->ntiles + wb + (one ? eb : 0), nt, sh->smem(), h->stream, one && overlap, X, h->G,
+    TMX_CK(launch_step(sh->single, h->ntiles + wb + (one ? eb : 0), nt, sh->smem(false), h->stream, one && overlap, X, h->G,
                        h->P, write_macro, h->tiles, h->ntiles, h->bnode, h->bcls, nw, h->nface, one ? ne : 0));
     if (beside) TMX_CK(cudaStreamWaitEvent(h->stream, h->join2, 0));
     TMX_CK(cudaGetLastError());
@@ -618,7 +618,7 @@ int enqueue_step(tmx_handle* h, int cur, int write_macro, cudaEvent_t* ev, bool 
     }
     if (ev) TMX_CK(cudaEventRecord(ev[0], h->stream));
     if (sh)
-        sh->tiles<<<h->ntiles, sh->threads(), sh->smem(), h->stream>>>(X, G, h->P, write_macro, h->tiles, h->ntiles);
+        sh->tiles<<<h->ntiles, sh->threads(), sh->smem(false), h->stream>>>(X, G, h->P, write_macro, h->tiles, h->ntiles);
     else
         h->K->bulk<<<h->bulk_blocks, 256, 0, h->stream>>>(X, G, h->P, write_macro);
     if (ev) TMX_CK(cudaEventRecord(ev[1], h->stream));
@@ -912,9 +912,10 @@ int tmx_create(const tmx_case* c, int device, tmx_handle** out)
         const SweepShape* sh = sweep_shape(TMX_SHAPE_SWEEP4);
         int per = 4;
         if (sweep_allow_smem() == cudaSuccess)
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)sh->single, sh->threads(), sh->smem());
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)sh->single, sh->threads(), sh->smem(false));
         cudaGetLastError();
-        const int rc = tmx_set_shape(h, TMX_SHAPE_SWEEP4, sweep_planes(h->G, sms * std::max(1, per)));
+        const int nt = sh->threads(), rest = (h->nface - h->nswept + nt - 1) / nt + (h->nb - h->nface + nt / 32 - 1) / (nt / 32);
+        const int rc = tmx_set_shape(h, TMX_SHAPE_SWEEP4, sweep_planes(h->G, sms * std::max(1, per), rest));
         if (rc) {
             const std::string msg = last_error();
             tmx_destroy(h);
@@ -938,7 +939,7 @@ int tmx_set_shape(tmx_handle* h, int kind, int zchunk)
     if (sh) {
         TMX_CK(sweep_allow_smem());
         std::vector<int4> t;
-        sweep_tiles(h->G, 0, sh->ty, zchunk, t);
+        sweep_tiles(h->G, 0, sh->ty, zchunk, false, t);
         int4* d = nullptr;
         if (!t.empty()) {
             cudaError_t e = cudaMalloc((void**)&d, t.size() * sizeof(int4));
@@ -955,7 +956,7 @@ int tmx_set_shape(tmx_handle* h, int kind, int zchunk)
         h->ntiles = (int)t.size();
         int per = 1, sms = 148;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)sh->single, sh->threads(), sh->smem());
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)sh->single, sh->threads(), sh->smem(false));
         cudaGetLastError();
         h->sweep_slots = sms * std::max(1, per);
     }

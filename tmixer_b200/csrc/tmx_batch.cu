@@ -223,6 +223,7 @@ struct tmx_batch {
     int cells = 4096;    // nodes per cell block
     int sweep = 0;       // 0: the flat kernel; else the TMX_SHAPE_SWEEP* shape of the interior
     int zchunk = 8;      // planes per sweep tile
+    bool groups = false; // the sweep tiles have groups (by rebuild)
     int bound_bps = 0;   // boundary kernels' blocks per SM (0: as many as fit)
     int bound_after = 0; // reduced-precision forms: interior kernel after the boundary kernels (1) or beside them
     int bound_fit = 1;   // blocks of the face kernel that fit on an SM
@@ -301,7 +302,7 @@ MixerDesc desc_of(const tmx_batch* b, const Slot& s)
 int rebuild(tmx_batch* b)
 {
     std::vector<MixerDesc> desc(b->slots.size());
-    std::vector<int4> blocks, tiles, runs;
+    std::vector<int4> blocks, tiles, grouped, runs;
     const bool by_runs = b->B->run != nullptr;
     std::vector<int2> faces, edges;
     int nactive = 0;
@@ -313,7 +314,10 @@ int rebuild(tmx_batch* b)
         for (int g0 = 0; g0 < s.G.nnodes; g0 += b->cells)
             blocks.push_back(make_int4((int)m, g0, std::min(b->cells, s.G.nnodes - g0), 0));
         if (by_runs) step_runs(s.G, (int)m, tmx::kRunBatchThreads, runs);
-        if (b->sweep) sweep_tiles(s.G, (int)m, sweep_shape(b->sweep)->ty, b->zchunk, tiles);
+        if (b->sweep) {
+            sweep_tiles(s.G, (int)m, sweep_shape(b->sweep)->ty, b->zchunk, false, tiles);
+            sweep_tiles(s.G, (int)m, sweep_shape(b->sweep)->ty, b->zchunk, true, grouped);
+        }
         // with a sweep shape the interior kernel updates the last nswept faces
         // (and the runs every face)
         const int nfk = by_runs ? 0 : (b->sweep ? s.nface - s.nswept : s.nface);
@@ -331,6 +335,11 @@ int rebuild(tmx_batch* b)
         while (faces.size() % tmx::kListAlign) faces.push_back(pad);
         while (edges.size() % tmx::kListAlign) edges.push_back(pad);
     }
+    // tiles with groups where they are a tenth fewer (tmx_kernels.cuh sweep_pitch)
+    const bool groups = b->sweep && grouped.size() * 10 <= tiles.size() * 9;
+    if (groups) tiles.swap(grouped);
+    if (groups != b->groups) drop_graphs(b);
+    b->groups = groups;
     cudaError_t e = grow(b, b->d_desc, b->cap_desc, (int)std::max<size_t>(1, desc.size()));
     if (e == cudaSuccess) e = grow(b, b->d_blocks, b->cap_blocks, (int)std::max<size_t>(1, blocks.size()));
     if (e == cudaSuccess) e = grow(b, b->d_faces, b->cap_faces, (int)std::max<size_t>(1, faces.size()));
@@ -413,7 +422,7 @@ int enqueue(tmx_batch* b, int parity, int write_macro, cudaEvent_t* ev = nullptr
     }
     if (ev) TMX_CK(cudaEventRecord(ev[0], b->stream));
     if (const SweepShape* sh = b->sweep ? sweep_shape(b->sweep) : nullptr)
-        sh->batch<<<b->grid_sweep[b->sweep], sh->threads(), sh->smem(), b->stream>>>(b->d_desc, b->d_tiles,
+        sh->batch[b->groups]<<<b->grid_sweep[b->sweep], sh->threads(), sh->smem(b->groups), b->stream>>>(b->d_desc, b->d_tiles,
                                                                                     b->d_faces, b->d_counts, parity,
                                                                                     write_macro);
     else
@@ -481,7 +490,7 @@ void set_grids(tmx_batch* b)
         for (int kind = TMX_SHAPE_SWEEP8; kind <= TMX_SHAPE_SWEEP4; kind++) {
             const SweepShape* sh = sweep_shape(kind);
             int per = 1;
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)sh->batch, sh->threads(), sh->smem());
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)sh->batch[1], sh->threads(), sh->smem(true));
             b->grid_sweep[kind] = b->sms * std::max(1, per);
         }
     int pf = 1, pe = 1;

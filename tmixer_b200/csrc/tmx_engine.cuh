@@ -560,16 +560,16 @@ struct RecGlobal {
     }
 };
 // ... or from the shared-memory planes of a sweep tile (sweep_tile): plane
-// slot (k - ez) & 3, row ty + 1 - ey, column tx + 1 - ex of (TY + 2) x 34
+// slot (k - ez) & 3, row ty + 1 - ey, column col + 1 - ex of (TY + 2) x RW
 // records, the two halves of each record in separate arrays.
-template <int TY>
+template <int TY, int RW>
 struct RecShared {
     const float4* A;
     const float4* B;
-    int tx, ty, k;
+    int col, ty, k;
     __device__ __forceinline__ void operator()(int q, int, float4& mf, float4& ms) const
     {
-        const int e = (((k - EZ(q)) & 3) * (TY + 2) + ty + 1 - EY(q)) * 34 + tx + 1 - EX(q);
+        const int e = (((k - EZ(q)) & 3) * (TY + 2) + ty + 1 - EY(q)) * RW + col + 1 - EX(q);
         mf = A[e];
         ms = B[e];
     }
@@ -822,7 +822,7 @@ __device__ __forceinline__ void bulk_node_lp(const StepPtrs& X, const Geom& G, c
 // through the planes z0 .. z1-1, one node per thread per plane.  The writer
 // records its nodes read (the 9 source rows of each node, 19 reads per node in
 // the flat kernel) are staged once per plane in shared memory: a ring of four
-// planes of (TY + 2) x 34 records (the tile and a one-node halo), the next
+// planes of (TY + 2) rows of records (the tile and a one-node halo), the next
 // plane but one copied asynchronously (cp.async) while the current plane is
 // computed.  The populations stream straight from global memory.  Each node's
 // arithmetic is lp_interior's, so the results are the flat kernel's bit for
@@ -858,26 +858,27 @@ __device__ __forceinline__ int tile_rec_node(const Geom& G, int b, int x, int y,
     return -1;
 }
 
-// One tile {mixer * 2 + box | planes << 20, x0, y0, z0} (0-based columns from x0,
-// sweep_end, and y0; the interior planes z0 .. z1-1, 2 <= z0 < z1 <= nz).
+// One tile {mixer * 2 + box | planes << 20 | s << 29, x0, y0, z0} (0-based columns
+// from x0, sweep_end, and y0; the interior planes z0 .. z1-1, 2 <= z0 < z1 <= nz).
 // A row's ends are the inlets or the mixing box's x walls, updated with it (as
 // face nodes of a list their 8-byte values were read a sector each, and the
 // partly written sectors read back: most of the face kernel's time).  A and B hold the two
-// halves of 4 * (TY + 2) * 34 records.  Every thread of the block runs the
+// halves of 4 * (TY + 2) * sweep_pitch records (GROUPS: tiles with s > 0 too).  Every thread of the block runs the
 // same iterations (the barriers are uniform).  The tiles of the first chunk
 // (z0 = 2) also update the z = 1 wall face nodes of their columns, those of
 // the last chunk (z1 = nz) the z = nz ones (zwall_node), the records of
 // both planes being in the ring.
-template <class PR, int TY>
+template <class PR, int TY, bool GROUPS>
 __device__ __forceinline__ void sweep_tile(const StepPtrs& X, const Geom& G, const Phys& P, int write_macro, int4 t,
                                            float4* A, float4* B)
 {
-    constexpr int RW = kSweepX + 2, PLANE = (TY + 2) * RW, NT = kSweepX * TY;
-    const int b = t.x & 1;
-    const int x0 = t.y, y0 = t.z, z0 = t.w, z1 = z0 + (t.x >> 20);
+    constexpr int RW = sweep_pitch(GROUPS), PLANE = (TY + 2) * RW, NT = kSweepX * TY;
+    const int b = t.x & 1, s = GROUPS ? t.x >> 29 : 0;
+    const int x0 = t.y, y0 = t.z, z0 = t.w, z1 = z0 + (GROUPS ? t.x >> 20 & 511 : t.x >> 20);
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const int nx = box_nx(G, b), ny = box_ny(G, b), x1 = sweep_end(x0, nx);
-    const int x = x0 + tx, y = y0 + ty;
+    const int nx = box_nx(G, b), ny = box_ny(G, b), x1 = sweep_end(x0, nx, GROUPS ? kSweepX >> s : kSweepX);
+    const SweepLane at = sweep_lane(s, tx, ty, TY);
+    const int x = x0 + (GROUPS ? at.x : tx), y = y0 + (GROUPS ? at.y : ty);
     // the rows of interior nodes, ends and all (of the opening's row the middle)
     const bool opening = b == 0 && y == 0;
     const bool row = y < ny && (b ? y > 0 : y < ny - 1);
@@ -893,7 +894,13 @@ __device__ __forceinline__ void sweep_tile(const StepPtrs& X, const Geom& G, con
         const int slot = (kk & 3) * PLANE;
         for (int e = threadIdx.x; e < PLANE; e += NT) {
             const int ry = e / RW, rx = e - ry * RW;
-            const int n = tile_rec_node(G, b, x0 + rx - 1, y0 + ry - 1, kk);
+            int n;
+            if constexpr (GROUPS) {
+                const int c = sweep_group(s, rx);
+                n = c < 1 << s ? tile_rec_node(G, b, x0 + sweep_column(s, rx), y0 + c * TY + ry - 1, kk) : -1;
+            } else {
+                n = tile_rec_node(G, b, x0 + rx - 1, y0 + ry - 1, kk);
+            }
             if (n >= 0) {
                 cp_async16(A + slot + e, M + 2 * (long long)n);
                 cp_async16(B + slot + e, M + 2 * (long long)n + 1);
@@ -913,14 +920,14 @@ __device__ __forceinline__ void sweep_tile(const StepPtrs& X, const Geom& G, con
         cp_async_commit();
         if (act) {
             const int g = box_base(G, b) + ((k - 1) * ny + y) * nx + x;
-            lp_interior<PR, true>(X, G, P, write_macro, g, b, x + 1, y + 1, k, RecShared<TY>{A, B, tx, ty, k},
+            lp_interior<PR, true>(X, G, P, write_macro, g, b, x + 1, y + 1, k, RecShared<TY, RW>{A, B, GROUPS ? at.col : tx, ty, k},
                                   PopGlobal<PR>{(const typename PR::S*)X.pin, G.ps}, xf);
             if (k == 2 && xf.cls < 0)
                 zwall_node<PR>(X, G, P, write_macro, b, x + 1, y + 1, 1, 2, g - nx * ny, g,
-                               RecShared<TY>{A, B, tx, ty, 1}, RecShared<TY>{A, B, tx, ty, 2});
+                               RecShared<TY, RW>{A, B, GROUPS ? at.col : tx, ty, 1}, RecShared<TY, RW>{A, B, GROUPS ? at.col : tx, ty, 2});
             if (k == G.nz - 1 && xf.cls < 0)
                 zwall_node<PR>(X, G, P, write_macro, b, x + 1, y + 1, G.nz, k, g + nx * ny, g,
-                               RecShared<TY>{A, B, tx, ty, G.nz}, RecShared<TY>{A, B, tx, ty, k});
+                               RecShared<TY, RW>{A, B, GROUPS ? at.col : tx, ty, G.nz}, RecShared<TY, RW>{A, B, GROUPS ? at.col : tx, ty, k});
         }
         cp_async_wait_all();
         __syncthreads();
@@ -1991,15 +1998,15 @@ __device__ __noinline__ void sweep_edge(const StepPtrs& X, const Geom& G, const 
 // beside it).  Blocks differ (wall planes, ragged
 // columns), and in a fixed share of the tiles the last block was 8% late (64
 // mixers, the interior alone: 3.23 -> 2.95 ms; W=64 321 -> 299 us).  Dynamic
-// shared memory: sweep_smem_host(TY).
+// shared memory: sweep_smem_host.
 #define TMX_SWEEP_KERNEL(PR, NAME, TY, MINB)                                                                      \
     __global__ void __launch_bounds__(kSweepX * TY, MINB) k_sweep##TY##_##NAME(                                  \
         StepPtrs X, Geom G, Phys P, int write_macro, const int4* __restrict__ tiles, int ntiles)                 \
     {                                                                                                           \
         extern __shared__ float4 sweep_smem[];                                                                  \
         float4* A = sweep_smem;                                                                                 \
-        float4* B = A + 4 * (TY + 2) * (kSweepX + 2);                                                           \
-        for (int t = blockIdx.x; t < ntiles; t += gridDim.x) sweep_tile<PR, TY>(X, G, P, write_macro, tiles[t], A, B); \
+        float4* B = A + 4 * (TY + 2) * sweep_pitch(false);                                                          \
+        for (int t = blockIdx.x; t < ntiles; t += gridDim.x) sweep_tile<PR, TY, false>(X, G, P, write_macro, tiles[t], A, B); \
     }                                                                                                           \
     __global__ void __launch_bounds__(kSweepX * TY, MINB) k_sweepw##TY##_##NAME(                                 \
         const __grid_constant__ StepPtrs X, const __grid_constant__ Geom G, const __grid_constant__ Phys P,      \
@@ -2009,12 +2016,12 @@ __device__ __noinline__ void sweep_edge(const StepPtrs& X, const Geom& G, const 
         extern __shared__ float4 sweep_smem[];                                                                  \
         constexpr int NT = kSweepX * TY;                                                                        \
         float4* A = sweep_smem;                                                                                 \
-        float4* B = A + 4 * (TY + 2) * (kSweepX + 2);                                                           \
+        float4* B = A + 4 * (TY + 2) * sweep_pitch(false);                                                          \
         step_begin();                                                                                           \
         step_wait();                                                                                            \
         const int t = blockIdx.x, w = t - ntiles, e = w - (nw + NT - 1) / NT;                                   \
         if (w < 0) {                                                                                            \
-            sweep_tile<PR, TY>(X, G, P, write_macro, tiles[t], A, B);                                           \
+            sweep_tile<PR, TY, false>(X, G, P, write_macro, tiles[t], A, B);                                           \
         } else if (e < 0) {                                                                                     \
             const int at = w * NT + threadIdx.x;                                                                \
             if (at < nw) sweep_wall<PR>(X, G, P, write_macro, bnode[at], bcls[at]);                             \
@@ -2023,14 +2030,16 @@ __device__ __noinline__ void sweep_edge(const StepPtrs& X, const Geom& G, const 
             if (at < ne)                                                                                        \
                 sweep_edge<PR>(X, G, P, write_macro, bnode[e0 + at], bcls[e0 + at], (PR::T*)A + wp * kEdgeBuf); \
         }                                                                                                       \
-    }                                                                                                           \
-    __global__ void __launch_bounds__(kSweepX * TY, MINB) k_sweep_batch##TY##_##NAME(                            \
+    }
+// GROUPS: for tiles with s > 0.
+#define TMX_SWEEP_BATCH_KERNEL(PR, NAME, TY, MINB, SUFFIX, GROUPS)                                               \
+    __global__ void __launch_bounds__(kSweepX * TY, MINB) k_sweep_batch##SUFFIX##_##NAME(                            \
         const MixerDesc* __restrict__ D, const int4* __restrict__ tiles, const int2* __restrict__ walls,         \
         int* __restrict__ counts, int parity, int write_macro)                                                  \
     {                                                                                                           \
         extern __shared__ float4 sweep_smem[];                                                                  \
         float4* A = sweep_smem;                                                                                 \
-        float4* B = A + 4 * (TY + 2) * (kSweepX + 2);                                                           \
+        float4* B = A + 4 * (TY + 2) * sweep_pitch(GROUPS);                                                  \
         __shared__ StepDesc d;                                                                                  \
         __shared__ int next;                                                                                    \
         const int n = counts[3], nw = counts[1];                                                                \
@@ -2043,7 +2052,7 @@ __device__ __noinline__ void sweep_edge(const StepPtrs& X, const Geom& G, const 
             load_desc(d, D, m, parity);                                                                         \
             __syncthreads();                                                                                    \
             if (t < n) {                                                                                        \
-                sweep_tile<PR, TY>(d.X, d.G, d.P, write_macro, tiles[t], A, B);                                 \
+                sweep_tile<PR, TY, GROUPS>(d.X, d.G, d.P, write_macro, tiles[t], A, B);                         \
             } else {                                                                                            \
                 for (int e = at + threadIdx.x; e < nw && e < at + kSweepWalls; e += kSweepX * TY) {             \
                     const int2 v = walls[e];                                                                    \
@@ -2055,8 +2064,12 @@ __device__ __noinline__ void sweep_edge(const StepPtrs& X, const Geom& G, const 
         }                                                                                                       \
     }
 #define TMX_DEFINE_SWEEP_KERNELS(PR, NAME) \
-    TMX_SWEEP_KERNEL(PR, NAME, 8, 2)       \
-    TMX_SWEEP_KERNEL(PR, NAME, 4, 4)
+    TMX_SWEEP_KERNEL(PR, NAME, 8, 2)                    \
+    TMX_SWEEP_KERNEL(PR, NAME, 4, 4)                    \
+    TMX_SWEEP_BATCH_KERNEL(PR, NAME, 8, 2, 8, false)    \
+    TMX_SWEEP_BATCH_KERNEL(PR, NAME, 4, 4, 4, false)    \
+    TMX_SWEEP_BATCH_KERNEL(PR, NAME, 8, 2, 8g, true)    \
+    TMX_SWEEP_BATCH_KERNEL(PR, NAME, 4, 4, 4g, true)
 
 // The face and the edge list as two launches (the FP32 and FP16-storage steps;
 // the FP64 step is k_run_f64).

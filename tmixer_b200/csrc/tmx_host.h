@@ -88,15 +88,15 @@ struct SweepShape {
     int kind, ty;
     void (*tiles)(tmx::StepPtrs, Geom, Phys, int, const int4*, int);
     void (*single)(tmx::StepPtrs, Geom, Phys, int, const int4*, int, const int*, const unsigned char*, int, int, int);
-    void (*batch)(const tmx::MixerDesc*, const int4*, const int2*, int*, int, int);
+    void (*batch[2])(const tmx::MixerDesc*, const int4*, const int2*, int*, int, int);  // [1]: tiles with groups
     int threads() const { return 32 * ty; }
-    int smem() const { return tmx::sweep_smem_host(ty); }
+    int smem(bool groups) const { return tmx::sweep_smem_host(ty, groups); }
 };
 inline const SweepShape* sweep_shape(int kind)
 {
     static const SweepShape shapes[] = {
-        {TMX_SHAPE_SWEEP8, 8, tmx::k_sweep8_f16, tmx::k_sweepw8_f16, tmx::k_sweep_batch8_f16},
-        {TMX_SHAPE_SWEEP4, 4, tmx::k_sweep4_f16, tmx::k_sweepw4_f16, tmx::k_sweep_batch4_f16},
+        {TMX_SHAPE_SWEEP8, 8, tmx::k_sweep8_f16, tmx::k_sweepw8_f16, {tmx::k_sweep_batch8_f16, tmx::k_sweep_batch8g_f16}},
+        {TMX_SHAPE_SWEEP4, 4, tmx::k_sweep4_f16, tmx::k_sweepw4_f16, {tmx::k_sweep_batch4_f16, tmx::k_sweep_batch4g_f16}},
     };
     for (const SweepShape& e : shapes)
         if (e.kind == kind) return &e;
@@ -109,28 +109,51 @@ inline cudaError_t sweep_allow_smem()
     for (int kind = TMX_SHAPE_SWEEP8; kind <= TMX_SHAPE_SWEEP4; kind++) {
         const SweepShape* sh = sweep_shape(kind);
         cudaError_t e = cudaFuncSetAttribute((const void*)sh->single, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             sh->smem());
+                                             sh->smem(false));
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute((const void*)sh->tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, sh->smem());
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute((const void*)sh->batch, cudaFuncAttributeMaxDynamicSharedMemorySize, sh->smem());
+            e = cudaFuncSetAttribute((const void*)sh->tiles, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     sh->smem(false));
+        for (int g = 0; g < 2 && e == cudaSuccess; g++)
+            e = cudaFuncSetAttribute((const void*)sh->batch[g], cudaFuncAttributeMaxDynamicSharedMemorySize, sh->smem(g));
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
 }
 
 // Tiles of the sweep kernels (tmx_engine.cuh sweep_tile) for one mixer:
-// {mixer * 2 + box | planes << 20, x0, y0, z0}, the columns from x0 (sweep_end)
-// by ty rows of a box (0-based x0, y0) over zchunk interior planes from z0 (2000
-// at most), z-chunks outermost.
-inline void sweep_tiles(const Geom& G, int mixer, int ty, int zchunk, std::vector<int4>& out)
+// {mixer * 2 + box | planes << 20 | s << 29, x0, y0, z0}, the columns from x0
+// (sweep_end) by ty << s rows of a box (0-based x0, y0; the rows of interior nodes)
+// over zchunk interior planes from z0 (500 at most), z-chunks outermost.  groups: the widths
+// are those that cover the box with the fewest tiles, the wider of equals
+// (24, 40 and 48 columns by 47, 79 and 95 rows of 4: 9, 25 and 36 tiles a plane where
+// 32 columns each take 24, 40 and 48); else s = 0.
+inline void sweep_tiles(const Geom& G, int mixer, int ty, int zchunk, bool groups, std::vector<int4>& out)
 {
-    zchunk = zchunk < 2000 ? zchunk : 2000;
+    zchunk = zchunk < 500 ? zchunk : 500;
+    std::vector<int> wide[2];  // per box: the s of a tile from column x
+    for (int b = 0; b < 2; b++) {
+        const int nx = G.nx[b], rows = G.ny[b] - 1;
+        std::vector<int> least(nx + 1, 0);
+        wide[b].assign(nx, 0);
+        for (int x = nx - 1; x >= 0; x--)
+            for (int s = 0; s < (groups ? 3 : 1); s++) {
+                const int n = (rows + (ty << s) - 1) / (ty << s) + least[tmx::sweep_end(x, nx, 32 >> s)];
+                if (s == 0 || n < least[x]) {
+                    least[x] = n;
+                    wide[b][x] = s;
+                }
+            }
+    }
     for (int z0 = 2; z0 <= G.nz - 1; z0 += zchunk)
         for (int b = 0; b < 2; b++)
-            for (int y0 = 0; y0 < G.ny[b]; y0 += ty)
-                for (int x0 = 0; x0 < G.nx[b]; x0 = tmx::sweep_end(x0, G.nx[b]))
-                    out.push_back(make_int4((mixer * 2 + b) | std::min(zchunk, G.nz - z0) << 20, x0, y0, z0));
+            // rows 0 .. ny-2 of box 0 (the opening's included), 1 .. ny-1 of box 1
+            for (int r = 0; r < G.ny[b] - 1; r += ty)
+                for (int x0 = 0; x0 < G.nx[b]; x0 = tmx::sweep_end(x0, G.nx[b], 32 >> wide[b][x0])) {
+                    const int s = wide[b][x0];
+                    if (r % (ty << s) == 0)
+                        out.push_back(make_int4((mixer * 2 + b) | std::min(zchunk, G.nz - z0) << 20 | s << 29, x0, r + b,
+                                                z0));
+                }
 }
 
 // Steps of one captured graph where many are asked for (an even number: the
@@ -220,15 +243,19 @@ void error_flag_give(int* flag);
 
 // Planes per 32 x 4 tile of a new FP16 handle: the fewest from 3 whose tiles the
 // GPU holds at once (slots blocks), 8 where none does.  A tile goes through its
-// planes one after another, so a small mixer wants short tiles (W=8 step 19.5 us
-// by 3 planes, 29.8 us by 8; W=24 31.8 by 4, 39.3 by 8), and a second, partly
-// filled wave costs a whole one (W=32 75.5 us by 6 planes, 60.3 by 8).
-inline int sweep_planes(const Geom& G, int slots)
+// planes one after another, so a small mixer wants short tiles (221,184 nodes 27.7
+// us by 4 planes, 35.8 by 8), and a second, partly filled wave costs a whole one
+// (221,184 nodes 31.8 us by 3 planes).  1 or 2 planes, whose tiles read most records
+// twice or three times, only where half of the GPU holds them with the boundary's
+// blocks (rest): 1,024 nodes 12.2 / 14.0 us by 1 / 3 planes, 8,192 nodes 13.0 / 14.5,
+// 27,648 nodes 13.9 / 16.7 by 2 / 3; but 43,904 nodes 18.6 / 15.8.
+inline int sweep_planes(const Geom& G, int slots, int rest)
 {
-    for (int z = 3; z < 8; z++) {
+    for (int z = 1; z < 8; z++) {
         std::vector<int4> t;
-        sweep_tiles(G, 0, 4, z, t);
-        if ((int)t.size() <= slots) return z;
+        sweep_tiles(G, 0, 4, z, false, t);
+        const int n = (int)t.size();
+        if (z < 3 ? 2 * (n + rest) <= slots : n <= slots) return z;
     }
     return 8;
 }

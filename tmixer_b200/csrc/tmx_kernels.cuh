@@ -102,17 +102,44 @@ __global__ void k_run_batch_f32(const MixerDesc* D, const int4* runs, const int2
                                 int write_macro, int what, int* error);
 TMX_DECLARE_BATCH_KERNELS(f16)
 
-// The FP16 form's interior by tiles of 32 x TY nodes swept through z
-// (tmx_engine.cuh sweep_tile): tiles[t] = {mixer * 2 + box | planes << 20,
+// The FP16 form's interior by tiles of 32 TY nodes of a plane swept through z
+// (tmx_engine.cuh sweep_tile): tiles[t] = {mixer * 2 + box | planes << 20 | s << 29,
 // x0, y0, z0}; the single-mixer kernels take mixer 0, the batched ones read
 // the tile count from counts[3] and hand the tiles out by counts[5 + parity].
-// Dynamic shared memory: sweep_smem_host(TY).
-// The end of a tile's columns: 32 on, but never the box's last column alone (an
-// x wall's species come from its neighbour in the same warp).
-__host__ __device__ constexpr int sweep_end(int x0, int nx)
+// Dynamic shared memory: sweep_smem_host.
+// A tile is w = 32 >> s columns wide.  In tiles with groups (s = 0, 1 or 2) a warp's
+// lanes are 1 << s groups of w, group c TY rows above group c - 1, side by side in
+// shared memory with a halo each (rows of sweep_pitch records), so that boxes narrower
+// than 32 columns, and what is left of wider ones, fill the lanes.  Their code costs
+// every tile a little: a batch takes them where they save a tenth of its tiles or
+// more (8 mixers of 544,000 nodes in boxes 16 to 192 columns wide, 13% fewer: 86.7 ->
+// 79.8 us; 64 of 41M nodes, 3% fewer: 3.56 -> 3.58 ms), a single mixer never
+// (221,184 nodes, 14% fewer: 27.8 -> 28.6 us; 4.2M, none: 318 -> 336 us).
+__host__ __device__ constexpr int sweep_pitch(bool groups) { return groups ? 40 : 34; }
+// The end of a tile's columns: w on, but never the box's last column alone (an
+// x wall's species come from its neighbour in the same group).
+__host__ __device__ constexpr int sweep_end(int x0, int nx, int w)
 {
-    return x0 + 32 >= nx ? nx : (x0 + 32 == nx - 1 ? x0 + 31 : x0 + 32);
+    return x0 + w >= nx ? nx : (x0 + w == nx - 1 ? x0 + w - 1 : x0 + w);
 }
+// A lane's place in its warp's row of a tile: column and row from the tile's
+// first, and its record's column in shared memory, less the halo's one.
+struct SweepLane {
+    int x, y, col;
+};
+__host__ __device__ constexpr SweepLane sweep_lane(int s, int lane, int warp, int ty)
+{
+    const int c = lane >> (5 - s);
+    return SweepLane{lane & ((32 >> s) - 1), warp + c * ty, lane + 2 * c};
+}
+// The place of record column col of a row of shared memory: column from the tile's
+// first, and group (1 << s or more: unused).
+__host__ __device__ constexpr int sweep_group(int s, int col)
+{
+    const int p = (32 >> s) + 2;
+    return (col >= p) + (col >= 2 * p) + (col >= 3 * p);
+}
+__host__ __device__ constexpr int sweep_column(int s, int col) { return col - sweep_group(s, col) * ((32 >> s) + 2) - 1; }
 constexpr int kSweepWalls = 256;  // wall row entries that a batch's block takes at a time
 #define TMX_DECLARE_SWEEP(SUFFIX)                                                                               \
     __global__ void k_sweep##SUFFIX##_f16(StepPtrs X, Geom G, Phys P, int write_macro, const int4* tiles,     \
@@ -120,12 +147,17 @@ constexpr int kSweepWalls = 256;  // wall row entries that a batch's block takes
     __global__ void k_sweepw##SUFFIX##_f16(const __grid_constant__ StepPtrs X, const __grid_constant__ Geom G, \
                                           const __grid_constant__ Phys P, int write_macro, const int4* tiles,  \
                                           int ntiles, const int* bnode, const unsigned char* bcls, int nw,     \
-                                          int e0, int ne);                                                     \
+                                          int e0, int ne);
+#define TMX_DECLARE_SWEEP_BATCH(SUFFIX)                                                                       \
     __global__ void k_sweep_batch##SUFFIX##_f16(const MixerDesc* D, const int4* tiles, const int2* walls,     \
                                                 int* counts, int parity, int write_macro);
 TMX_DECLARE_SWEEP(8)
+TMX_DECLARE_SWEEP_BATCH(8)
+TMX_DECLARE_SWEEP_BATCH(4)
+TMX_DECLARE_SWEEP_BATCH(8g)
+TMX_DECLARE_SWEEP_BATCH(4g)
 TMX_DECLARE_SWEEP(4)
-constexpr int sweep_smem_host(int ty) { return 2 * 4 * (ty + 2) * 34 * 16; }
+constexpr int sweep_smem_host(int ty, bool groups) { return 2 * 4 * (ty + 2) * sweep_pitch(groups) * 16; }
 
 // Threads per species of the row kernels (blocks of 3 kRowPart; the pressure and
 // power kernel has kRowPart).
