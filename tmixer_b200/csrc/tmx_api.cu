@@ -70,8 +70,8 @@ struct tmx_handle {
     bool inited = false;
     long long bytes = 0;
     int bulk_blocks = 0;
-    // the boundary kernel runs on a second stream, concurrently with the bulk
-    // kernel (disjoint outputs, read-only shared inputs)
+    // FP16: the face and edge kernels run on these beside the interior kernel
+    // (disjoint outputs, read-only shared inputs)
     cudaStream_t aux = nullptr, aux2 = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr, join2 = nullptr;
     int nface = 0;  // the first nface boundary nodes are face classes
@@ -88,6 +88,7 @@ struct tmx_handle {
     cudaGraphExec_t graph[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
     // ... and kGraphSteps of them by state buffer
     cudaGraphExec_t graph_many[2] = {nullptr, nullptr};
+    int singles = 0;  // steps launched one by one (graph_length)
     int sbytes = 8, tbytes = 8;  // storage / arithmetic bytes per value of the form
     const struct StepKernels* K = nullptr;
     // interior kernel shape (tmx_set_shape): TMX_SHAPE_*, planes per tile,
@@ -568,7 +569,7 @@ int enqueue_sweep(tmx_handle* h, const SweepShape* sh, const tmx::StepPtrs& X, i
 
 // Queue one step from buffer `cur`: the face and the edge kernel on the two
 // auxiliary streams, forked from and joined back into the main stream, and the
-// bulk kernel on the main stream (FP64 and FP32: enqueue_run).  With ev (4
+// interior kernel on the main stream (FP64 and FP32: enqueue_run).  With ev (4
 // events) each part is bracketed by its own pair of events.  The state and density
 // buffers flip together every step, so one parity index selects both.
 int enqueue_step(tmx_handle* h, int cur, int write_macro, cudaEvent_t* ev, bool overlap = false)
@@ -1005,7 +1006,8 @@ int tmx_step(tmx_handle* h, int nsteps)
     if (nsteps < 0) return fail(TMX_E_INVALID, "negative step count");
     TMX_CK(cudaSetDevice(h->device));
     for (int left = nsteps; left > 0;) {
-        const int n = left > kGraphSteps ? kGraphSteps : 1;
+        const int n = graph_length(left, h->graph_many[h->cur], h->singles);
+        if (n == 1 && h->singles < kGraphWorth) h->singles++;
         const int rc = graph_steps(h, n, left == 1);
         if (rc) return rc;
         left -= n;

@@ -1,11 +1,12 @@
 // tmx_batch.cu -- the batched engine behind tmx_batch_* (include/tmx.h): many
-// T-mixers of uneven size and parameters stepped together, every step one
-// launch per kernel kind over all of them.
+// T-mixers of uneven size and parameters stepped together, every step a
+// few launches over all of them.
 //
 //   - Device memory: one arena of the batch's budget, allocated once; each
 //     mixer's state is a first-fit range of it (admission by footprint).
-//   - Work lists: the bulk kernel walks a concatenated list of cell blocks
-//     {mixer, first node, node count}; the boundary kernels walk the
+//   - Work lists: the FP64 and FP32 forms' kernel walks a concatenated list of
+//     runs and the edge list; the FP16 form's walk one of tiles (or cell blocks
+//     {mixer, first node, node count}), its boundary kernels the
 //     concatenated face and edge node lists {node, mixer * 256 + class}.  A
 //     mixer's descriptor (buffers per step parity, geometry, physics) is
 //     read from device memory; the sweep and boundary kernels copy it into
@@ -234,6 +235,7 @@ struct tmx_batch {
     int nblocks = 0, nfaces = 0, nedges = 0, ntiles = 0, nactive = 0;
     cudaGraphExec_t graph[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
     cudaGraphExec_t graph_many[2] = {nullptr, nullptr};  // kGraphSteps steps
+    int singles = 0;  // steps launched one by one (graph_length)
 };
 
 namespace {
@@ -781,7 +783,8 @@ int tmx_batch_step(tmx_batch* b, int nsteps, int write_macro_last)
         if (rc) return rc;
     }
     for (int left = nsteps; left > 0;) {
-        const int n = left > kGraphSteps ? kGraphSteps : 1;
+        const int n = graph_length(left, b->graph_many[b->parity], b->singles);
+        if (n == 1 && b->singles < kGraphWorth) b->singles++;
         const int rc = graph_steps(b, n, left == 1 && write_macro_last ? 1 : 0);
         if (rc) return rc;
         left -= n;

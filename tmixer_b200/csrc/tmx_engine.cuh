@@ -7,25 +7,27 @@
 //
 // One step of the reference (equilibrium, collision, streaming,
 // boundary_conditions, calculate_velocity_density; Tmixer.cpp:10469-10475)
-// runs as launches over disjoint node sets:
+// runs over disjoint node sets, in one launch (FP64 and FP32: tmx_run64.cuh,
+// tmx_run32.cuh; small FP16 mixers) or several (FP16: tiles or the flat interior
+// kernel, faces, edges):
 //
-//   bulk      every node that no boundary case touches: pull the 76
+//   interior  every node that no boundary case touches: pull the 76
 //             post-collision populations of the previous step from their
 //             upstream neighbours, take moments, equilibrium, BGK collision
 //             plus reaction, write the 76 new post-collision populations.
-//   boundary  every boundary node (compact list, sorted by case; faces and
-//             edges/corners in two kernels): the same, with the reference's
-//             closure for its case between the pull and the moments.
+//   boundary  every face, edge and corner node (compact list, sorted by case):
+//             the same, with the reference's closure for its case between the
+//             pull and the moments.
 //
 // The state between steps is the post-collision population set (the
 // reference's fn/gn/hn/pn), double-buffered (A-B pull).  Boundary closures
 // read, besides their own pulled populations: their own post-collision
 // values ("undo streaming"), the previous step's densities of a few nodes
-// (kept in R, written by both kernels for the nodes that are read), the
+// (kept in R, written for the nodes that are read), the
 // current step's flow density of an inlet node (recomputed from that node's
 // pulled populations), and the pulled species populations of an interior
 // node (zero-gradient copies).  None of these is written during the step, so
-// all boundary nodes run in parallel and the kernels need no ordering.
+// all nodes run in parallel and a step's launches need no ordering.
 #pragma once
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -2071,8 +2073,7 @@ __device__ __noinline__ void sweep_edge(const StepPtrs& X, const Geom& G, const 
     TMX_SWEEP_BATCH_KERNEL(PR, NAME, 8, 2, 8g, true)    \
     TMX_SWEEP_BATCH_KERNEL(PR, NAME, 4, 4, 4g, true)
 
-// The face and the edge list as two launches (the FP32 and FP16-storage steps;
-// the FP64 step is k_run_f64).
+// The face and the edge list as two launches (FP16).
 #define TMX_DEFINE_BOUNDARY_KERNELS(PR, NAME)                                                                     \
     __global__ void __launch_bounds__(kBoundaryThreads) k_bfaces_##NAME(                                       \
         StepPtrs X, const int* bnode, const unsigned char* bcls, int nb, Geom G, Phys P, int write_macro)       \

@@ -160,6 +160,15 @@ inline void sweep_tiles(const Geom& G, int mixer, int ty, int zchunk, bool group
 // buffers are back in place).  A graph of its own per step costs a small mixer a
 // microsecond or two between steps.
 constexpr int kGraphSteps = 16;
+// The next launch's steps where `left` are asked for: building such a graph costs
+// what 50 to 150 steps save by it (W=32, the first 20 steps of a handle: FP64 123 us a
+// step by a new graph of 16, 117 one by one, 113 by one that is there), so one by
+// one until kGraphWorth steps have gone that way or are asked for.
+constexpr int kGraphWorth = 64;
+inline int graph_length(int left, bool built, int singles)
+{
+    return left > kGraphSteps && (built || left + singles > kGraphWorth) ? kGraphSteps : 1;
+}
 
 // Launch a step's kernel; overlap: as soon as the step before it in the stream
 // leaves room, which the kernel waits for by itself (step_wait).
