@@ -332,8 +332,8 @@ def reference_cpu_run(params: dict, budget_s: float, steps: int = REF_SAMPLE_STE
 
 
 def profile_traffic(form: str = "fp64") -> dict | None:
-    """DRAM bytes per launch of the bulk kernel from the committed ncu summary."""
-    p = os.path.join(ROOT, "profiles", "k_bulk_%s_w32.json" % form)
+    """DRAM bytes per launch of the interior kernel from the committed ncu summary."""
+    p = os.path.join(ROOT, "profiles", "interior_%s_w32.json" % form)
     if not os.path.exists(p):
         return None
     with open(p) as fh:
@@ -437,7 +437,7 @@ def run_ours(args, dist: Dist) -> dict | None:
                                                                                else min(args.steps, 1000)),
                            "bulk_gbs": m["achieved"], "bulk_frac": m["achieved"] / peaks["hbm_gbs"],
                            "bytes_per_lup": FORM_BYTES[form],
-                           "interior_kernel": "sweep4:%d" % FP16_SHAPE[1] if form == "fp16" else "flat"}
+                           "interior_kernel": "sweep4:%d" % FP16_SHAPE[1] if form == "fp16" else "runs"}
             pc = pattern_ceiling(T.PRECISIONS[form], m["bulk_nodes"], m["achieved"], dist.local_rank)
             forms[form]["bulk_pattern_frac"] = pc["frac"] if pc else None
 

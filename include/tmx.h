@@ -232,7 +232,7 @@ int tmx_inlet_profile(tmx_handle *h, double *uin1, double *uin2);
  * handle's stream and return the summed device times (ms) of the bulk
  * (interior) kernel, of the boundary kernels and of the whole step loop.
  * The interior kernel runs after the boundary kernels here in every form
- * (tmx_step overlaps them in the FP32 and FP16 forms), so that each time is
+ * (tmx_step overlaps them), so that each time is
  * that of its kernels alone.  Benchmark support; no counterpart in the
  * reference. */
 int tmx_step_timed(tmx_handle *h, int nsteps, double *ms_bulk, double *ms_boundary, double *ms_total);
@@ -281,10 +281,8 @@ void tmx_destroy(tmx_handle *h);
 
 /* ------------------------------------------------------------------------
  * Batched engine: many mixers of uneven size and parameters stepped together,
- * each step one launch per kernel kind over all of them (a persistent bulk
- * kernel over a concatenated cell-block list, and persistent boundary kernels
- * over the concatenated boundary-node lists), with the step captured as a
- * CUDA graph.  The reference runs one case per process and has no
+ * each step one to three launches of persistent kernels over concatenated work
+ * lists, with the steps captured as CUDA graphs.  The reference runs one case per process and has no
  * counterpart for any of these functions.  One batch is used from one host
  * thread at a time.
  * ------------------------------------------------------------------------ */
