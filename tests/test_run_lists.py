@@ -25,7 +25,7 @@ def checker(tmp_path_factory):
 
 def _cases():
     keys = ("inx", "iny", "nz", "mnx", "mny", "ia")
-    out = [[5, 3, 3, 3, 3, 2], [401, 51, 51, 101, 750, 151][:6], [8, 3, 3, 3, 3, 5]]
+    out = [[5, 3, 3, 3, 3, 2], [12, 4, 520, 4, 5, 4], [401, 51, 51, 101, 750, 151][:6], [8, 3, 3, 3, 3, 5]]
     out += [[c[k] for k in keys] for c in [v[0] for v in GOLDEN_CASES.values()] + list(ORACLE_CASES.values())]
     rng = random.Random(7)
     for _ in range(60):
