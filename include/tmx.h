@@ -263,9 +263,9 @@ int tmx_pattern_ceiling(int precision, long long nodes, int reps, int device, do
  * them through zchunk planes (zchunk >= 1), the writers' moment records
  * staged in shared memory: TMX_SHAPE_SWEEP8 (TY 8), TMX_SHAPE_SWEEP4 (TY 4).
  * Every shape gives the same results bit for bit.  Default: TMX_SHAPE_SWEEP4
- * for the FP16 form (set by tmx_create, 3 to 8 planes by the case's size),
+ * for the FP16 form (set by tmx_create, 1 to 8 planes by the case's size),
  * TMX_SHAPE_FLAT for the others.  A new FP16 batch starts with TMX_SHAPE_SWEEP4
- * and 4 planes. */
+ * and 4 planes, 8 where its mixers make four rounds of such tiles or more. */
 #define TMX_SHAPE_FLAT 0
 #define TMX_SHAPE_SWEEP8 1
 #define TMX_SHAPE_SWEEP4 2

@@ -224,6 +224,7 @@ struct tmx_batch {
     int cells = 4096;    // nodes per cell block
     int sweep = 0;       // 0: the flat kernel; else the TMX_SHAPE_SWEEP* shape of the interior
     int zchunk = 8;      // planes per sweep tile
+    bool by_size = false; // no shape was set: zchunk by the mixers' size (rebuild)
     bool groups = false; // the sweep tiles have groups (by rebuild)
     int bound_bps = 0;   // boundary kernels' blocks per SM (0: as many as fit)
     int bound_after = 0; // reduced-precision forms: interior kernel after the boundary kernels (1) or beside them
@@ -308,6 +309,12 @@ int rebuild(tmx_batch* b)
     const bool by_runs = b->B->run != nullptr;
     std::vector<int2> faces, edges;
     int nactive = 0;
+    if (b->by_size && b->sweep) {
+        for (const Slot& s : b->slots)
+            if (s.used) sweep_tiles(s.G, 0, sweep_shape(b->sweep)->ty, 2 * kBatchPlanes, false, tiles);
+        b->zchunk = (int)tiles.size() >= kBatchRounds * b->grid_sweep[b->sweep] ? 2 * kBatchPlanes : kBatchPlanes;
+        tiles.clear();
+    }
     for (size_t m = 0; m < b->slots.size(); m++) {
         const Slot& s = b->slots[m];
         if (!s.used) continue;
@@ -577,6 +584,7 @@ int tmx_batch_create(int precision, long long budget_bytes, int device, tmx_batc
     if (b->K->moments) {
         b->sweep = TMX_SHAPE_SWEEP4;
         b->zchunk = kBatchPlanes;
+        b->by_size = true;
     }
     const long long budget = align_up(budget_bytes);
     cudaError_t e = cudaMalloc((void**)&b->arena_base, (size_t)budget);
@@ -928,6 +936,7 @@ int tmx_batch_set_shape(tmx_batch* b, int threads, int cells)
     if (cells != b->cells || b->sweep) b->dirty = true;
     b->cells = cells;
     b->sweep = 0;
+    b->by_size = false;
     return TMX_OK;
 }
 
@@ -943,6 +952,7 @@ int tmx_batch_set_sweep(tmx_batch* b, int kind, int zchunk)
     if (kind != b->sweep || zchunk != b->zchunk) b->dirty = true;
     b->sweep = kind;
     b->zchunk = zchunk;
+    b->by_size = false;
     return TMX_OK;
 }
 

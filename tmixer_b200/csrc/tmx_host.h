@@ -268,10 +268,11 @@ inline int sweep_planes(const Geom& G, int slots, int rest)
     }
     return 8;
 }
-// ... and of a new FP16 batch, whose mixers are not known yet (8 mixers of
-// 544,000 nodes: 123 us by the flat kernel, 85 by 4 planes, 95 by 8; 4 mixers of
-// 4.3M nodes: 585, 409, 401 us)
-constexpr int kBatchPlanes = 4;
+// ... and of an FP16 batch that no shape was set for: 4, or 8 where those make
+// kBatchRounds rounds of tiles or more (by 4 / 8 planes: 8 mixers of 544,000 nodes,
+// one round, 81 / 90 us; 4 of 4.3M nodes, 7 rounds, 409 / 401 us; 64 of 41M nodes,
+// 68 rounds, 3.71 / 3.58 ms).
+constexpr int kBatchPlanes = 4, kBatchRounds = 4;
 
 // Checkpoint layout (tmx_checkpoint, tmx_batch_checkpoint): this header, then
 // the sections in the order of `bytes`: the population buffer the next step
