@@ -803,7 +803,7 @@ __device__ __forceinline__ void zwall_node(const StepPtrs& X, const Geom& G, con
     }
 }
 
-// One interior node of the FP32 / FP16 forms in the flat bulk kernels.  (The
+// One interior node of the FP16 form in the flat bulk kernels.  (The
 // z wall faces stay with the face kernel here: updated by these kernels as
 // well, the walls cost them registers (168 B of spills) and the 4-mixer FP16
 // batch step went from 571 to 680-697 us, the W=32 FP16 step from 69.2 to
