@@ -1010,6 +1010,20 @@ __device__ __forceinline__ typename PR::T inlet_rho_now(const BCtx<PR>& c, int s
                                   T(2) * (v[1] + v[7] + v[10] + v[11] + v[14]));
 }
 
+// a * b + c of a closure, rounded once in the reduced-precision forms and twice,
+// as in the reference, in FP64 (-a and -c are exact there).  Not left to
+// contraction: the compiler chose it kernel by kernel, and in densities of a few
+// of FP32's smallest denormals (species ahead of the front) the choice shows in
+// leading digits.  Elsewhere the closures' products are by powers of two or stand
+// alone, and round the same either way.
+__device__ __forceinline__ double mul_add(double a, double b, double c) { return a * b + c; }
+__device__ __forceinline__ float mul_add(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+// x less (plus) a quarter of d, the momentum along an edge
+template <class T>
+__device__ __forceinline__ T quarter_off(T x, T d) { return mul_add(T(-0.25), d, x); }
+template <class T>
+__device__ __forceinline__ T quarter_on(T x, T d) { return mul_add(T(0.25), d, x); }
+
 // corners: six bounce-backs, buried pairs averaged from their own
 // post-collision values, and (corners 1-12) one pair closed from a density.
 struct CornerSpec {
@@ -1087,8 +1101,9 @@ __device__ __forceinline__ void wall_flow_closure(int cls, T rout, T (&v)[19])
         v[7] = v[9] - A; v[8] = v[10] + A;
     } break;
     case K_OUTLET: {  // Case 13 flow (:3162-3190); species copy from y+1 (:3192-3273)
-        const T uy = T(1) - (T(1) / rout) * ((v[0] + v[1] + v[3] + v[5] + v[6] + v[11] + v[12] + v[13] + v[14]) +
-                                                T(2) * (v[4] + v[9] + v[10] + v[16] + v[17]));
+        const T m = (v[0] + v[1] + v[3] + v[5] + v[6] + v[11] + v[12] + v[13] + v[14]) +
+                    T(2) * (v[4] + v[9] + v[10] + v[16] + v[17]);
+        const T uy = mul_add(-(T(1) / rout), m, T(1));
         const T A = (rout * uy) / T(6);
         const T B = T(0.5) * ((v[3] + v[12] + v[13]) - (v[1] + v[11] + v[14]));
         const T C = T(0.5) * ((v[6] + v[13] + v[14]) - (v[5] + v[11] + v[12]));
@@ -1146,11 +1161,11 @@ __device__ __forceinline__ void closure_face(const BCtx<PR>& c, int cls, int fld
             v[7] = v[9] - (A + B); v[10] = v[8] - (A - B); v[11] = v[13] - (A + C); v[14] = v[12] - (A - C);
         } else {
             const T cin = pick_species(c.P->cin, fld, 0);
-            v[1] = -v[3] + T(2.0 / 18.0) * cin;
-            v[7] = -v[9] + T(2.0 / 36.0) * cin;
-            v[10] = -v[8] + T(2.0 / 36.0) * cin;
-            v[11] = -v[13] + T(2.0 / 36.0) * cin;
-            v[14] = -v[12] + T(2.0 / 36.0) * cin;
+            v[1] = mul_add(T(2.0 / 18.0), cin, -v[3]);
+            v[7] = mul_add(T(2.0 / 36.0), cin, -v[9]);
+            v[10] = mul_add(T(2.0 / 36.0), cin, -v[8]);
+            v[11] = mul_add(T(2.0 / 36.0), cin, -v[13]);
+            v[14] = mul_add(T(2.0 / 36.0), cin, -v[12]);
         }
     } break;
     case K_INLET2: {  // Inlet2 (:2668-2730)
@@ -1165,11 +1180,11 @@ __device__ __forceinline__ void closure_face(const BCtx<PR>& c, int cls, int fld
             v[9] = v[7] + (A + B); v[8] = v[10] + (A - B); v[13] = v[11] + (A + C); v[12] = v[14] + (A - C);
         } else {
             const T cin = pick_species(c.P->cin, fld, 1);
-            v[3] = -v[1] + T(2.0 / 18.0) * cin;
-            v[9] = -v[7] + T(2.0 / 36.0) * cin;
-            v[8] = -v[10] + T(2.0 / 36.0) * cin;
-            v[13] = -v[11] + T(2.0 / 36.0) * cin;
-            v[12] = -v[14] + T(2.0 / 36.0) * cin;
+            v[3] = mul_add(T(2.0 / 18.0), cin, -v[1]);
+            v[9] = mul_add(T(2.0 / 36.0), cin, -v[7]);
+            v[8] = mul_add(T(2.0 / 36.0), cin, -v[10]);
+            v[13] = mul_add(T(2.0 / 36.0), cin, -v[11]);
+            v[12] = mul_add(T(2.0 / 36.0), cin, -v[14]);
         }
     } break;
     case K_FACE_YT:
@@ -1222,19 +1237,19 @@ __device__ __forceinline__ void closure_edge(const BCtx<PR>& c, int cls, int fld
         v[2] = v[4]; v[6] = v[5]; v[7] = v[9]; v[8] = v[10]; v[13] = v[11]; v[14] = v[12]; v[18] = v[16];
         v[15] = T(0.5) * (own_fn(c, fld, 15) + own_fn(c, fld, 17));
         v[17] = v[15];
-        const T A = T(0.25) * (v[1] - v[3]);
-        v[7] = v[9] - A; v[8] = v[10] + A; v[13] = v[11] + A; v[14] = v[12] - A;
+        const T A = v[1] - v[3];
+        v[7] = quarter_off(v[9], A); v[8] = quarter_on(v[10], A); v[13] = quarter_on(v[11], A); v[14] = quarter_off(v[12], A);
     } break;
     case K_EDGE_X1_ZTOP: {  // Case 4 (:2343-2476); field C keeps p13 = pn13 (:2474)
-        const T B = T(0.25) * (v[2] - v[4]);
-        v[1] = v[3]; v[6] = v[5]; v[7] = v[9] - B; v[10] = v[8] + B; v[14] = v[12]; v[17] = v[15] + B; v[18] = v[16] - B;
+        const T B = v[2] - v[4];
+        v[1] = v[3]; v[6] = v[5]; v[7] = quarter_off(v[9], B); v[10] = quarter_on(v[8], B); v[14] = v[12]; v[17] = quarter_on(v[15], B); v[18] = quarter_off(v[16], B);
         v[13] = own_fn(c, fld, 13);
         v[11] = T(0.5) * (rprev(c, fld, 0, 1, c.j, G.nz - 1) - sum_but(v, 11, 13));
         if (fld != 3) v[13] = v[11];
     } break;
     case K_EDGE_XT_ZTOP: {  // Case 6 (:2477-2605)
-        const T B = T(0.25) * (v[2] - v[4]);
-        v[3] = v[1]; v[6] = v[5]; v[9] = v[7] + B; v[8] = v[10] - B; v[13] = v[11]; v[17] = v[15] + B; v[18] = v[16] - B;
+        const T B = v[2] - v[4];
+        v[3] = v[1]; v[6] = v[5]; v[9] = quarter_on(v[7], B); v[8] = quarter_off(v[10], B); v[13] = v[11]; v[17] = quarter_on(v[15], B); v[18] = quarter_off(v[16], B);
         v[12] = T(0.5) * (rprev(c, fld, 0, G.inx, c.j, G.nz - 1) - sum_but(v, 12, 14));
         v[14] = v[12];
     } break;
@@ -1242,54 +1257,54 @@ __device__ __forceinline__ void closure_edge(const BCtx<PR>& c, int cls, int fld
         v[4] = v[2]; v[6] = v[5]; v[17] = v[15];
         v[16] = T(0.5) * (own_fn(c, fld, 16) + own_fn(c, fld, 18));
         v[18] = v[16];
-        const T A = T(0.25) * (v[1] - v[3]);
-        v[9] = v[7] + A; v[10] = v[8] - A; v[13] = v[11] + A; v[14] = v[12] - A;
+        const T A = v[1] - v[3];
+        v[9] = quarter_on(v[7], A); v[10] = quarter_off(v[8], A); v[13] = quarter_on(v[11], A); v[14] = quarter_off(v[12], A);
     } break;
     case K_EDGE_YT_Z1: {  // Case 21 (:4386-4533)
         v[4] = v[2]; v[5] = v[6]; v[16] = v[18];
         v[15] = T(0.5) * (own_fn(c, fld, 15) + own_fn(c, fld, 17));
         v[17] = v[15];
-        const T A = T(0.25) * (v[1] - v[3]);
-        v[9] = v[7] + A; v[10] = v[8] - A; v[11] = v[13] - A; v[12] = v[14] + A;
+        const T A = v[1] - v[3];
+        v[9] = quarter_on(v[7], A); v[10] = quarter_off(v[8], A); v[11] = quarter_off(v[13], A); v[12] = quarter_on(v[14], A);
     } break;
     case K_EDGE_X1_Z1: {  // Case 22 (:4534-4656); flow density of (1,j,2) from this step
-        const T B = T(0.25) * (v[2] - v[4]);
-        v[1] = v[3]; v[5] = v[6]; v[7] = v[9] - B; v[10] = v[8] + B; v[11] = v[13]; v[15] = v[17] - B; v[16] = v[18] + B;
+        const T B = v[2] - v[4];
+        v[1] = v[3]; v[5] = v[6]; v[7] = quarter_off(v[9], B); v[10] = quarter_on(v[8], B); v[11] = v[13]; v[15] = quarter_off(v[17], B); v[16] = quarter_on(v[18], B);
         const T R = flow ? inlet_rho_now(c, 0, c.j, 2) : rprev(c, fld, 0, 1, c.j, 2);
         v[12] = T(0.5) * (R - sum_but(v, 12, 14));
         v[14] = v[12];
     } break;
     case K_EDGE_XT_Z1: {  // Case 23 (:4657-4779)
-        const T B = T(0.25) * (v[2] - v[4]);
-        v[3] = v[1]; v[5] = v[6]; v[8] = v[10] - B; v[9] = v[7] + B; v[12] = v[14]; v[15] = v[17] - B; v[16] = v[18] + B;
+        const T B = v[2] - v[4];
+        v[3] = v[1]; v[5] = v[6]; v[8] = quarter_off(v[10], B); v[9] = quarter_on(v[7], B); v[12] = v[14]; v[15] = quarter_off(v[17], B); v[16] = quarter_on(v[18], B);
         const T R = flow ? inlet_rho_now(c, 1, c.j, 2) : rprev(c, fld, 0, G.inx, c.j, 2);
         v[11] = T(0.5) * (R - sum_but(v, 11, 13));
         v[13] = v[11];
     } break;
     case K_EDGE_X1_Y1: {  // Case 24 (:4780-4909)
-        const T C = T(0.25) * (v[5] - v[6]);
-        v[1] = v[3]; v[2] = v[4]; v[7] = v[9]; v[11] = v[13] - C; v[14] = v[12] + C; v[15] = v[17] - C; v[18] = v[16] + C;
+        const T C = v[5] - v[6];
+        v[1] = v[3]; v[2] = v[4]; v[7] = v[9]; v[11] = quarter_off(v[13], C); v[14] = quarter_on(v[12], C); v[15] = quarter_off(v[17], C); v[18] = quarter_on(v[16], C);
         const T R = flow ? inlet_rho_now(c, 0, 2, c.k) : rprev(c, fld, 0, 1, 2, c.k);
         v[8] = T(0.5) * (R - sum_but(v, 8, 10));
         v[10] = v[8];
     } break;
     case K_EDGE_X1_YT: {  // Case 25 (:4910-5032)
-        const T C = T(0.25) * (v[5] - v[6]);
-        v[1] = v[3]; v[4] = v[2]; v[10] = v[8]; v[11] = v[13] - C; v[14] = v[12] + C; v[16] = v[18] - C; v[17] = v[15] + C;
+        const T C = v[5] - v[6];
+        v[1] = v[3]; v[4] = v[2]; v[10] = v[8]; v[11] = quarter_off(v[13], C); v[14] = quarter_on(v[12], C); v[16] = quarter_off(v[18], C); v[17] = quarter_on(v[15], C);
         const T R = flow ? inlet_rho_now(c, 0, G.iny - 1, c.k) : rprev(c, fld, 0, 1, G.iny - 1, c.k);
         v[7] = T(0.5) * (R - sum_but(v, 7, 9));
         v[9] = v[7];
     } break;
     case K_EDGE_XT_Y1: {  // Case 26 (:5033-5159)
-        const T C = T(0.25) * (v[5] - v[6]);
-        v[3] = v[1]; v[2] = v[4]; v[8] = v[10]; v[12] = v[14] - C; v[13] = v[11] + C; v[15] = v[17] - C; v[18] = v[16] + C;
+        const T C = v[5] - v[6];
+        v[3] = v[1]; v[2] = v[4]; v[8] = v[10]; v[12] = quarter_off(v[14], C); v[13] = quarter_on(v[11], C); v[15] = quarter_off(v[17], C); v[18] = quarter_on(v[16], C);
         const T R = flow ? inlet_rho_now(c, 1, 2, c.k) : rprev(c, fld, 0, G.inx, 2, c.k);
         v[7] = T(0.5) * (R - sum_but(v, 7, 9));
         v[9] = v[7];
     } break;
     case K_EDGE_XT_YT: {  // Case 27 (:5160-5281)
-        const T C = T(0.25) * (v[5] - v[6]);
-        v[3] = v[1]; v[4] = v[2]; v[9] = v[7]; v[12] = v[14] - C; v[13] = v[11] + C; v[16] = v[18] - C; v[17] = v[15] + C;
+        const T C = v[5] - v[6];
+        v[3] = v[1]; v[4] = v[2]; v[9] = v[7]; v[12] = quarter_off(v[14], C); v[13] = quarter_on(v[11], C); v[16] = quarter_off(v[18], C); v[17] = quarter_on(v[15], C);
         const T R = flow ? inlet_rho_now(c, 1, G.iny - 1, c.k) : rprev(c, fld, 0, G.inx, G.iny - 1, c.k);
         v[8] = T(0.5) * (R - sum_but(v, 8, 10));
         v[10] = v[8];
@@ -1298,58 +1313,58 @@ __device__ __forceinline__ void closure_edge(const BCtx<PR>& c, int cls, int fld
         v[2] = v[4]; v[5] = v[6]; v[15] = v[17];
         v[16] = T(0.5) * (own_fn(c, fld, 16) + own_fn(c, fld, 18));
         v[18] = v[16];
-        const T A = T(0.25) * (v[1] - v[3]);
-        v[7] = v[9] - A; v[8] = v[10] + A; v[11] = v[13] - A; v[12] = v[14] + A;
+        const T A = v[1] - v[3];
+        v[7] = quarter_off(v[9], A); v[8] = quarter_on(v[10], A); v[11] = quarter_off(v[13], A); v[12] = quarter_on(v[14], A);
     } break;
     case K_MEDGE_AB: {  // (:7788-7868)
-        const T A = T(0.25) * (v[1] - v[3]);
-        v[2] = v[4]; v[5] = v[6]; v[7] = v[9] - A; v[8] = v[10] + A; v[11] = v[13] - A; v[12] = v[14] + A; v[15] = v[17];
+        const T A = v[1] - v[3];
+        v[2] = v[4]; v[5] = v[6]; v[7] = quarter_off(v[9], A); v[8] = quarter_on(v[10], A); v[11] = quarter_off(v[13], A); v[12] = quarter_on(v[14], A); v[15] = v[17];
         const T R = flow ? T(c.P->rho_out) : rprev(c, fld, 1, c.i, 2, 1);
         v[18] = T(0.5) * (R - sum_but(v, 16, 18));
         v[16] = v[18];
     } break;
     case K_MEDGE_ApBp: {  // (:7870-7950)
-        const T A = T(0.25) * (v[1] - v[3]);
-        v[2] = v[4]; v[6] = v[5]; v[7] = v[9] - A; v[8] = v[10] + A; v[13] = v[11] + A; v[14] = v[12] - A; v[18] = v[16];
+        const T A = v[1] - v[3];
+        v[2] = v[4]; v[6] = v[5]; v[7] = quarter_off(v[9], A); v[8] = quarter_on(v[10], A); v[13] = quarter_on(v[11], A); v[14] = quarter_off(v[12], A); v[18] = v[16];
         const T R = flow ? T(c.P->rho_out) : rprev(c, fld, 1, c.i, 2, G.nz);
         v[15] = T(0.5) * (R - sum_but(v, 15, 17));
         v[17] = v[15];
     } break;
     case K_MEDGE_AAp: {  // (:7951-8043)
-        const T C = T(0.25) * (v[5] - v[6]);
-        v[1] = v[3]; v[2] = v[4]; v[7] = v[9]; v[11] = v[13] - C; v[14] = v[12] + C; v[15] = v[17] - C; v[18] = v[16] + C;
+        const T C = v[5] - v[6];
+        v[1] = v[3]; v[2] = v[4]; v[7] = v[9]; v[11] = quarter_off(v[13], C); v[14] = quarter_on(v[12], C); v[15] = quarter_off(v[17], C); v[18] = quarter_on(v[16], C);
         const T R = flow ? T(c.P->rho_out) : rprev(c, fld, 1, 1, 2, c.k);
         v[8] = T(0.5) * (R - sum_but(v, 8, 10));
         v[10] = v[8];
     } break;
     case K_MEDGE_BBp: {  // (:8044-8136)
-        const T C = T(0.25) * (v[5] - v[6]);
-        v[3] = v[1]; v[2] = v[4]; v[8] = v[10]; v[12] = v[14] - C; v[13] = v[11] + C; v[15] = v[17] - C; v[18] = v[16] + C;
+        const T C = v[5] - v[6];
+        v[3] = v[1]; v[2] = v[4]; v[8] = v[10]; v[12] = quarter_off(v[14], C); v[13] = quarter_on(v[11], C); v[15] = quarter_off(v[17], C); v[18] = quarter_on(v[16], C);
         const T R = flow ? T(c.P->rho_out) : rprev(c, fld, 1, G.mnx, 2, c.k);
         v[7] = T(0.5) * (R - sum_but(v, 7, 9));
         v[9] = v[7];
     } break;
     case K_MEDGE_AD: {  // (:8137-8244)
-        const T B = T(0.25) * (v[2] - v[4]);
-        v[1] = v[3]; v[5] = v[6]; v[7] = v[9] - B; v[10] = v[8] + B; v[11] = v[13]; v[15] = v[17] - B; v[16] = v[18] + B;
+        const T B = v[2] - v[4];
+        v[1] = v[3]; v[5] = v[6]; v[7] = quarter_off(v[9], B); v[10] = quarter_on(v[8], B); v[11] = v[13]; v[15] = quarter_off(v[17], B); v[16] = quarter_on(v[18], B);
         v[14] = T(0.5) * (own_fn(c, fld, 12) + own_fn(c, fld, 14));
         v[12] = v[14];
     } break;
     case K_MEDGE_ApDp: {  // (:8245-8344)
-        const T B = T(0.25) * (v[2] - v[4]);
-        v[1] = v[3]; v[6] = v[5]; v[7] = v[9] - B; v[10] = v[8] + B; v[14] = v[12]; v[17] = v[15] + B; v[18] = v[16] - B;
+        const T B = v[2] - v[4];
+        v[1] = v[3]; v[6] = v[5]; v[7] = quarter_off(v[9], B); v[10] = quarter_on(v[8], B); v[14] = v[12]; v[17] = quarter_on(v[15], B); v[18] = quarter_off(v[16], B);
         v[13] = T(0.5) * (own_fn(c, fld, 11) + own_fn(c, fld, 13));
         v[11] = v[13];
     } break;
     case K_MEDGE_BC: {  // (:8345-8445)
-        const T B = T(0.25) * (v[2] - v[4]);
-        v[3] = v[1]; v[5] = v[6]; v[8] = v[10] - B; v[9] = v[7] + B; v[12] = v[14]; v[15] = v[17] - B; v[16] = v[18] + B;
+        const T B = v[2] - v[4];
+        v[3] = v[1]; v[5] = v[6]; v[8] = quarter_off(v[10], B); v[9] = quarter_on(v[7], B); v[12] = v[14]; v[15] = quarter_off(v[17], B); v[16] = quarter_on(v[18], B);
         v[13] = T(0.5) * (own_fn(c, fld, 11) + own_fn(c, fld, 13));
         v[11] = v[13];
     } break;
     case K_MEDGE_BpCp: {  // (:8446-8550)
-        const T B = T(0.25) * (v[2] - v[4]);
-        v[3] = v[1]; v[6] = v[5]; v[9] = v[7] + B; v[8] = v[10] - B; v[13] = v[11]; v[17] = v[15] + B; v[18] = v[16] - B;
+        const T B = v[2] - v[4];
+        v[3] = v[1]; v[6] = v[5]; v[9] = quarter_on(v[7], B); v[8] = quarter_off(v[10], B); v[13] = v[11]; v[17] = quarter_on(v[15], B); v[18] = quarter_off(v[16], B);
         v[14] = T(0.5) * (own_fn(c, fld, 12) + own_fn(c, fld, 14));
         v[12] = v[14];
     } break;
@@ -1619,8 +1634,8 @@ __device__ __forceinline__ void edge_node(const StepPtrs& X, const Geom& G, cons
         for (int f = 0; f < 4; f++) {
             T x = buf[f * 20 + opp];
             if (bit & (rule.minus | rule.plus)) {
-                const T A = T(0.25) * (buf[f * 20 + a] - buf[f * 20 + c]);
-                x = bit & rule.minus ? x - A : x + A;
+                const T A = buf[f * 20 + a] - buf[f * 20 + c];
+                x = bit & rule.minus ? quarter_off(x, A) : quarter_on(x, A);
             }
             buf[f * 20 + q] = x;
         }
