@@ -371,8 +371,12 @@ int rebuild(tmx_batch* b)
     if (!edges.empty()) TMX_CK(cudaMemcpyAsync(b->d_edges, edges.data(), edges.size() * sizeof(int2), h2d, b->stream));
     if (!tiles.empty()) TMX_CK(cudaMemcpyAsync(b->d_tiles, tiles.data(), tiles.size() * sizeof(int4), h2d, b->stream));
     if (!runs.empty()) TMX_CK(cudaMemcpyAsync(b->d_runs, runs.data(), runs.size() * sizeof(int4), h2d, b->stream));
-    const int counts[5] = {(int)blocks.size(), (int)faces.size(), (int)edges.size(), (int)tiles.size(),
-                           (int)runs.size()};
+    // the counters that hand out the tiles and runs start at 0: a step clears the
+    // other parity's only, which steps by the flat kernel in between (they take
+    // none and clear none) leave as it was.  Every change of the kernel comes
+    // through here.
+    const int counts[tmx::kCounts] = {(int)blocks.size(), (int)faces.size(), (int)edges.size(), (int)tiles.size(),
+                                      (int)runs.size(), 0, 0};
     TMX_CK(cudaMemcpyAsync(b->d_counts, counts, sizeof counts, h2d, b->stream));
     TMX_CK(cudaStreamSynchronize(b->stream));
     b->nblocks = counts[0];
