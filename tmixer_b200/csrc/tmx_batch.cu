@@ -301,6 +301,16 @@ MixerDesc desc_of(const tmx_batch* b, const Slot& s)
     return d;
 }
 
+// Planes per sweep tile: the ones set, or by the mixers' size (kBatchPlanes).
+int tile_planes(const tmx_batch* b)
+{
+    if (!b->by_size || !b->sweep) return b->zchunk;
+    std::vector<int4> tiles;
+    for (const Slot& s : b->slots)
+        if (s.used) sweep_tiles(s.G, 0, sweep_shape(b->sweep)->ty, 2 * kBatchPlanes, false, tiles);
+    return (int)tiles.size() >= kBatchRounds * b->grid_sweep[b->sweep] ? 2 * kBatchPlanes : kBatchPlanes;
+}
+
 // Rebuild descriptors and work lists of the used slots and upload them.
 int rebuild(tmx_batch* b)
 {
@@ -309,12 +319,7 @@ int rebuild(tmx_batch* b)
     const bool by_runs = b->B->run != nullptr;
     std::vector<int2> faces, edges;
     int nactive = 0;
-    if (b->by_size && b->sweep) {
-        for (const Slot& s : b->slots)
-            if (s.used) sweep_tiles(s.G, 0, sweep_shape(b->sweep)->ty, 2 * kBatchPlanes, false, tiles);
-        b->zchunk = (int)tiles.size() >= kBatchRounds * b->grid_sweep[b->sweep] ? 2 * kBatchPlanes : kBatchPlanes;
-        tiles.clear();
-    }
+    b->zchunk = tile_planes(b);
     for (size_t m = 0; m < b->slots.size(); m++) {
         const Slot& s = b->slots[m];
         if (!s.used) continue;
@@ -988,7 +993,7 @@ int tmx_batch_shape(const tmx_batch* b, int out[4])
     out[0] = b->sweep ? b->sweep : TMX_SHAPE_FLAT;
     out[1] = b->sweep ? sweep_shape(b->sweep)->threads() : kBulkThreads[b->variant];
     out[2] = b->cells;
-    out[3] = b->zchunk;
+    out[3] = tile_planes(b);  // (mixers may have come or gone since the last step)
     return TMX_OK;
 }
 
