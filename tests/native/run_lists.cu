@@ -15,13 +15,13 @@
 
 using namespace tmx;
 
-static int check(const Geom& G, int nt)
+static int check(const Geom& G, int nt, int mixer)
 {
     std::vector<int4> runs;
-    tmx_host::step_runs(G, 5, nt, runs);
+    tmx_host::step_runs(G, mixer, nt, runs);
     std::vector<char> seen(G.nnodes, 0);
     for (const int4& t : runs) {
-        if (run_mixer(t) != 5) return std::printf("mixer\n"), 1;
+        if (run_mixer(t) != mixer) return std::printf("mixer\n"), 1;
         const Run R = run_of(G, t);
         if (R.n < 1 || R.n > nt) return std::printf("run of %d\n", R.n), 1;
         int first[4][19], count[4][19];
@@ -105,21 +105,21 @@ static int check(const Geom& G, int nt)
 // among them, the opening's ends not) in exactly one, the species' source of an x wall
 // in the same group of lanes, and every record of a node's sources staged in the
 // place that the node reads.
-static int check_tiles(const Geom& G, int ty, int planes, bool groups)
+static int check_tiles(const Geom& G, int ty, int planes, bool groups, int mixer)
 {
     std::vector<int4> tiles;
-    tmx_host::sweep_tiles(G, 5, ty, planes, groups, tiles);
+    tmx_host::sweep_tiles(G, mixer, ty, planes, groups, tiles);
     std::vector<char> seen(G.nnodes, 0);
     const int pitch = sweep_pitch(groups);
     for (const int4& t : tiles) {
-        const int b = t.x & 1, s = t.x >> 29, z1 = t.w + (t.x >> 20 & 511), w = 32 >> s;
+        const int b = t.x & 1, s = t.z >> 29, z1 = t.w + (t.x >> 23), w = 32 >> s;
         const int nx = box_nx(G, b), ny = box_ny(G, b), x1 = sweep_end(t.y, nx, w);
-        if ((t.x & 0xfffff) >> 1 != 5 || (!groups && s)) return std::printf("mixer or groups\n"), 1;
+        if ((t.x & 0x7fffff) >> 1 != mixer || (!groups && s)) return std::printf("mixer or groups\n"), 1;
         if (x1 - t.y < 2 || x1 - t.y > w || t.w < 2 || z1 > G.nz) return std::printf("tile\n"), 1;
         for (int warp = 0; warp < ty; warp++)
             for (int lane = 0; lane < 32; lane++) {
                 const SweepLane at = sweep_lane(s, lane, warp, ty);
-                const int x = t.y + at.x, y = t.z + at.y;
+                const int x = t.y + at.x, y = (t.z & 0x1fffffff) + at.y;
                 if (x >= x1 || y >= ny || (b ? y < 1 : y >= ny - 1)) continue;
                 if (b == 0 && y == 0 && (x < G.ia || x >= G.ib - 1)) continue;
                 for (int k = t.w; k < z1; k++)
@@ -159,8 +159,14 @@ int main(int argc, char** argv)
         c.ia = atoi(argv[a + 5]);
         Geom G;
         tmx_host::geometry_of(c, G);
-        int bad = check(G, 128) || check(G, 256);
-        for (int v = 0; v < 12 && !bad; v++) bad = check_tiles(G, v & 1 ? 8 : 4, v < 4 ? 1 : (v < 8 ? 3 : 1000), v & 2);
+        int bad = 0;
+        // a mixer's slot as small batches have it, in the first two cases also large ones
+        for (int m : {5, 65536, kMaxMixers - 1}) {
+            if (bad || (m > 5 && a > 7)) break;
+            bad = check(G, 128, m) || check(G, 256, m);
+            for (int v = 0; v < 12 && !bad; v++)
+                bad = check_tiles(G, v & 1 ? 8 : 4, v < 4 ? 1 : (v < 8 ? 3 : 1000), v & 2, m);
+        }
         if (bad) {
             std::printf("case %d %d %d %d %d %d\n", c.inx, c.iny, c.nz, c.mnx, c.mny, c.ia);
             return 1;

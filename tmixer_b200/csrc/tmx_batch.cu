@@ -712,6 +712,10 @@ int admit(tmx_batch* b, const tmx_case* c, const void* buf, long long size, int*
         b->arena.release(off, cv.total);
         b->slots[m] = Slot();
         return rc;
+    if (m < 0 && b->slots.size() >= (size_t)tmx::kMaxMixers) {
+        b->arena.release(off, cv.total);
+        return fail(TMX_E_INVALID, "a batch holds %d mixers at most", tmx::kMaxMixers);
+    }
     }
     b->dirty = true;
     *slot = m;

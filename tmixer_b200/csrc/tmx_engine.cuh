@@ -860,7 +860,7 @@ __device__ __forceinline__ int tile_rec_node(const Geom& G, int b, int x, int y,
     return -1;
 }
 
-// One tile {mixer * 2 + box | planes << 20 | s << 29, x0, y0, z0} (0-based columns
+// One tile {mixer * 2 + box | planes << 23, x0, y0 | s << 29, z0} (0-based columns
 // from x0, sweep_end, and y0; the interior planes z0 .. z1-1, 2 <= z0 < z1 <= nz).
 // A row's ends are the inlets or the mixing box's x walls, updated with it (as
 // face nodes of a list their 8-byte values were read a sector each, and the
@@ -875,8 +875,8 @@ __device__ __forceinline__ void sweep_tile(const StepPtrs& X, const Geom& G, con
                                            float4* A, float4* B)
 {
     constexpr int RW = sweep_pitch(GROUPS), PLANE = (TY + 2) * RW, NT = kSweepX * TY;
-    const int b = t.x & 1, s = GROUPS ? t.x >> 29 : 0;
-    const int x0 = t.y, y0 = t.z, z0 = t.w, z1 = z0 + (GROUPS ? t.x >> 20 & 511 : t.x >> 20);
+    const int b = t.x & 1, s = GROUPS ? t.z >> 29 : 0;
+    const int x0 = t.y, y0 = GROUPS ? t.z & 0x1fffffff : t.z, z0 = t.w, z1 = z0 + (t.x >> 23);
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     const int nx = box_nx(G, b), ny = box_ny(G, b), x1 = sweep_end(x0, nx, GROUPS ? kSweepX >> s : kSweepX);
     const SweepLane at = sweep_lane(s, tx, ty, TY);
@@ -2062,7 +2062,7 @@ __device__ __noinline__ void sweep_edge(const StepPtrs& X, const Geom& G, const 
         const int n = counts[3], nw = counts[1];                                                                \
         if (blockIdx.x == 0 && threadIdx.x == 0) counts[5 + (1 - parity)] = 0; /* the next step's */             \
         for (int t = blockIdx.x; t < n + (nw + kSweepWalls - 1) / kSweepWalls; t = next) {                      \
-            const int at = (t - n) * kSweepWalls, m = t < n ? (tiles[t].x & 0xfffff) >> 1 : walls[at].y >> 8;    \
+            const int at = (t - n) * kSweepWalls, m = t < n ? (tiles[t].x & 0x7fffff) >> 1 : walls[at].y >> 8;   \
             __syncthreads();                                                                                    \
             /* the tile after this one, by the launch's counter */                                              \
             if (threadIdx.x == 0) next = gridDim.x + atomicAdd(counts + 5 + parity, 1);                         \

@@ -121,15 +121,15 @@ inline cudaError_t sweep_allow_smem()
 }
 
 // Tiles of the sweep kernels (tmx_engine.cuh sweep_tile) for one mixer:
-// {mixer * 2 + box | planes << 20 | s << 29, x0, y0, z0}, the columns from x0
+// {mixer * 2 + box | planes << 23, x0, y0 | s << 29, z0}, the columns from x0
 // (sweep_end) by ty << s rows of a box (0-based x0, y0; the rows of interior nodes)
-// over zchunk interior planes from z0 (500 at most), z-chunks outermost.  groups: the widths
+// over zchunk interior planes from z0 (250 at most), z-chunks outermost.  groups: the widths
 // are those that cover the box with the fewest tiles, the wider of equals
 // (24, 40 and 48 columns by 47, 79 and 95 rows of 4: 9, 25 and 36 tiles a plane where
 // 32 columns each take 24, 40 and 48); else s = 0.
 inline void sweep_tiles(const Geom& G, int mixer, int ty, int zchunk, bool groups, std::vector<int4>& out)
 {
-    zchunk = zchunk < 500 ? zchunk : 500;
+    zchunk = zchunk < 250 ? zchunk : 250;
     std::vector<int> wide[2];  // per box: the s of a tile from column x
     for (int b = 0; b < 2; b++) {
         const int nx = G.nx[b], rows = G.ny[b] - 1;
@@ -151,8 +151,8 @@ inline void sweep_tiles(const Geom& G, int mixer, int ty, int zchunk, bool group
                 for (int x0 = 0; x0 < G.nx[b]; x0 = tmx::sweep_end(x0, G.nx[b], 32 >> wide[b][x0])) {
                     const int s = wide[b][x0];
                     if (r % (ty << s) == 0)
-                        out.push_back(make_int4((mixer * 2 + b) | std::min(zchunk, G.nz - z0) << 20 | s << 29, x0, r + b,
-                                                z0));
+                        out.push_back(make_int4((mixer * 2 + b) | std::min(zchunk, G.nz - z0) << 23, x0,
+                                                (r + b) | s << 29, z0));
                 }
 }
 
@@ -214,7 +214,7 @@ inline void step_runs(const Geom& G, int mixer, int nt, std::vector<int4>& out)
                     // (ends at multiples of 32 nodes: whole 256-byte stores)
                     const int n = std::min(end - g, nt - g % 32);
                     (n > nt / 2 ? out : rest)
-                        .push_back(make_int4(g, n | kind << 9 | b << 12 | iface << 13 | mixer << 15, i, k));
+                        .push_back(make_int4(g, n | kind << 9 | b << 12 | iface << 13, i, mixer));
                     g += n;
                     i = (i - 1 + n) % G.nx[b] + 1;
                 }

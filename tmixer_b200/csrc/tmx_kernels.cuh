@@ -44,7 +44,7 @@ TMX_DECLARE_STEP_KERNELS(f16)
 TMX_DECLARE_BOUNDARY_KERNELS(f16)
 
 // Runs of the FP64 and FP32 steps (tmx_run64.cuh, tmx_run32.cuh): {first node, nodes | kind << 9 |
-// box << 12 | iface << 13 | mixer << 15, x of the first node, z}, up to
+// box << 12 | iface << 13, x of the first node, mixer}, up to
 // NT consecutive nodes of one plane of a box, NT the kernel's threads (128 or
 // 256; run_threads in tmx_host.h).  iface: the row whose ey = 1 (1) or ey = -1
 // (2) sources lie in the other box.
@@ -61,6 +61,11 @@ constexpr int run_smem_host(int nt) { return 2 * 19 * (nt + 4) * 8 + nt / 32 * 8
 TMX_DECLARE_RUN(128, f64)
 TMX_DECLARE_RUN(256, f64)
 TMX_DECLARE_RUN(128, f32)
+
+// Mixers that a batch can hold: a tile's entry has 22 bits for the mixer's slot
+// (the boundary lists' mixer * 256 + class 23, a run's 31).  As many of the
+// smallest mixers that the FP16 form can have take 247 GB.
+constexpr int kMaxMixers = 1 << 22;
 
 // One mixer of a batch: its buffers for either parity of the batch's step
 // counter, its geometry and its physics constants (device memory, read by
@@ -103,8 +108,8 @@ __global__ void k_run_batch_f32(const MixerDesc* D, const int4* runs, const int2
 TMX_DECLARE_BATCH_KERNELS(f16)
 
 // The FP16 form's interior by tiles of 32 TY nodes of a plane swept through z
-// (tmx_engine.cuh sweep_tile): tiles[t] = {mixer * 2 + box | planes << 20 | s << 29,
-// x0, y0, z0}; the single-mixer kernels take mixer 0, the batched ones read
+// (tmx_engine.cuh sweep_tile): tiles[t] = {mixer * 2 + box | planes << 23, x0,
+// y0 | s << 29, z0}; the single-mixer kernels take mixer 0, the batched ones read
 // the tile count from counts[3] and hand the tiles out by counts[5 + parity].
 // Dynamic shared memory: sweep_smem_host.
 // A tile is w = 32 >> s columns wide.  In tiles with groups (s = 0, 1 or 2) a warp's

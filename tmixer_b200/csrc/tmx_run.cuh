@@ -52,7 +52,7 @@ struct Run {
     int g0, n, kind, b, i0, nx;
     int shift, op, om, ops, oms, sz, szp, szm;
 };
-__host__ __device__ inline int run_mixer(const int4& t) { return t.y >> 15; }
+__host__ __device__ inline int run_mixer(const int4& t) { return t.w; }
 __host__ __device__ inline Run run_of(const Geom& G, const int4& t)
 {
     Run R;
@@ -60,7 +60,7 @@ __host__ __device__ inline Run run_of(const Geom& G, const int4& t)
     R.n = t.y & 511;
     R.kind = (t.y >> 9) & 7;
     R.b = (t.y >> 12) & 1;
-    const int iface = (t.y >> 13) & 3, k0 = t.w - 1;
+    const int iface = (t.y >> 13) & 3;
     R.i0 = t.z;
     R.nx = box_nx(G, R.b);
     R.sz = R.szp = R.szm = R.nx * box_ny(G, R.b);
@@ -73,6 +73,7 @@ __host__ __device__ inline Run run_of(const Geom& G, const int4& t)
         R.szm = G.inx * G.iny;
         R.om = k0 * R.szm + G.ia - 1 - G.base[1] - (k0 * G.mny + G.mny - 1) * G.mnx;
     }
+    const int k0 = iface ? (R.g0 - box_base(G, R.b)) / R.sz : 0;
     const int dk = R.kind == kRunZ1 ? 1 : (R.kind == kRunZT ? -1 : 0);
     R.shift = dk ? dk * R.sz : (R.kind == kRunYT ? -R.nx : (R.kind == kRunY1 ? R.nx : 0));
     R.ops = R.op + dk * (R.szp - R.sz);

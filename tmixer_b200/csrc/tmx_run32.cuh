@@ -111,7 +111,7 @@ __device__ __forceinline__ void run32_loop(const Get& get, const int4* __restric
         meanwhile();
         return;
     }
-    const int4 none = make_int4(0, 0, 1, 1);
+    const int4 none = make_int4(0, 0, 1, 0);
     if (t == 0) {
         mbar_init(smem_addr(&S.full), 1);
         S.done = 0;

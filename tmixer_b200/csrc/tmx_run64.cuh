@@ -317,7 +317,7 @@ __device__ __forceinline__ void run_loop(const Get& get, const int4* __restrict_
                 }
                 if (t == NT - 1) {
                     if (next < nruns) cp_async16(&S.run[ord ^ 1], runs + next);
-                    else S.run[ord ^ 1] = make_int4(0, 0, 1, 1);
+                    else S.run[ord ^ 1] = make_int4(0, 0, 1, 0);
                 }
             } else if (f != 2) {
                 if (inlet()) {
