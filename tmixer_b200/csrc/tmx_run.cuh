@@ -64,6 +64,7 @@ __host__ __device__ inline Run run_of(const Geom& G, const int4& t)
     R.i0 = t.z;
     R.nx = box_nx(G, R.b);
     R.sz = R.szp = R.szm = R.nx * box_ny(G, R.b);
+    const int k0 = iface ? (R.g0 - box_base(G, R.b)) / R.sz : 0;
     R.op = -R.nx;
     R.om = R.nx;
     if (iface == 1) {
@@ -73,7 +74,6 @@ __host__ __device__ inline Run run_of(const Geom& G, const int4& t)
         R.szm = G.inx * G.iny;
         R.om = k0 * R.szm + G.ia - 1 - G.base[1] - (k0 * G.mny + G.mny - 1) * G.mnx;
     }
-    const int k0 = iface ? (R.g0 - box_base(G, R.b)) / R.sz : 0;
     const int dk = R.kind == kRunZ1 ? 1 : (R.kind == kRunZT ? -1 : 0);
     R.shift = dk ? dk * R.sz : (R.kind == kRunYT ? -R.nx : (R.kind == kRunY1 ? R.nx : 0));
     R.ops = R.op + dk * (R.szp - R.sz);
