@@ -1635,7 +1635,7 @@ __device__ __forceinline__ void edge_node(const StepPtrs& X, const Geom& G, cons
             T x = buf[f * 20 + opp];
             if (bit & (rule.minus | rule.plus)) {
                 const T A = buf[f * 20 + a] - buf[f * 20 + c];
-                x = bit & rule.minus ? quarter_off(x, A) : quarter_on(x, A);
+                x = mul_add(bit & rule.minus ? T(-0.25) : T(0.25), A, x);
             }
             buf[f * 20 + q] = x;
         }
