@@ -20,11 +20,11 @@ __device__ __forceinline__ void mbar_expect(unsigned bar, unsigned bytes)
 {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-// Wait for a phase of a barrier; false if it does not come within some
-// seconds (the caller gives up and reports it).
+// Wait for a phase of a barrier; false if it does not come within two seconds
+// (a try that fails takes 4 us; the caller gives up and reports it).
 __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity)
 {
-    for (int i = 0; i < (1 << 22); i++) {
+    for (int i = 0; i < (1 << 19); i++) {
         unsigned done;
         asm volatile(
             "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
@@ -34,6 +34,15 @@ __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity)
         if (done) return true;
     }
     return false;
+}
+// What a thread does that gave up waiting: it sets the error flag and waits once
+// more for the copies of bar that are in flight (they write shared memory that the
+// block leaves), whichever its phase is.
+__device__ __forceinline__ void mbar_give_up(int* error, unsigned bar)
+{
+    *error = 1;
+    mbar_wait(bar, 0);
+    mbar_wait(bar, 1);
 }
 __device__ __forceinline__ void bulk_load(unsigned dst, const void* src, unsigned bytes, unsigned bar)
 {

@@ -233,10 +233,7 @@ __device__ __forceinline__ void run_loop(const Get& get, const int4* __restrict_
     meanwhile();
     for (int ord = 0;; ord ^= 1) {
         // (each barrier goes through two phases a run: the parities repeat)
-        if (!mbar_wait(smem_addr(&S.full[0]), 0)) {
-            *error = 1;
-            return;
-        }
+        if (!mbar_wait(smem_addr(&S.full[0]), 0)) goto gave_up;
         const int4 tr = S.run[ord];
         if ((tr.y & 511) == 0) return;
         const RunView M = get(tr);
@@ -263,10 +260,7 @@ __device__ __forceinline__ void run_loop(const Get& get, const int4* __restrict_
 #pragma unroll 1
         for (int f = 0; f < 4; f++) {
             const int s = f & 1;
-            if (s && !mbar_wait(smem_addr(&S.full[1]), f >> 1)) {
-                *error = 1;
-                return;
-            }
+            if (s && !mbar_wait(smem_addr(&S.full[1]), f >> 1)) goto gave_up;
             run_read<NT>(&S.slot[s][t + (f ? ((what >> 1) & 3) - 1 : 0)], S.par[ord][f ? 1 : 0], v);
             // the slot is free once every warp has read it; the last fills it
             // with the field after the next
@@ -335,10 +329,7 @@ __device__ __forceinline__ void run_loop(const Get& get, const int4* __restrict_
                     __syncwarp();
                     if (S.run[ord ^ 1].y & 511) run_prepare(S, ord ^ 1, *get(S.run[ord ^ 1]).G);
                 }
-                if (!mbar_wait(smem_addr(&S.full[0]), 1)) {
-                    *error = 1;
-                    return;
-                }
+                if (!mbar_wait(smem_addr(&S.full[0]), 1)) goto gave_up;
                 double* __restrict__ rb = &S.slot[0][t + ((what >> 1) & 3) - 1];
                 if (inlet()) {
                     run_inlet_species<NT>(rb, S.par[ord][1], cls(), P.cin[1][cls() == K_INLET2]);
@@ -367,6 +358,9 @@ __device__ __forceinline__ void run_loop(const Get& get, const int4* __restrict_
             }
         }
     }
+gave_up:
+    mbar_give_up(error, smem_addr(&S.full[0]));
+    mbar_give_up(error, smem_addr(&S.full[1]));
 }
 
 }  // namespace tmx
