@@ -117,7 +117,10 @@ int tmx_init(tmx_handle *h);
  * handle's stream; the macroscopic fields of the last step are kept. */
 int tmx_step(tmx_handle *h, int nsteps);
 
-/* Wait for all work queued on the handle. */
+/* Wait for all work queued on the handle.  TMX_E_CUDA, from here and from every
+ * call that waits and reads, if a step gave up waiting for its copies (FP64 and
+ * FP32; the wait is bounded, it does not happen on a sound GPU): the state is not
+ * valid until tmx_init or tmx_restore. */
 int tmx_sync(tmx_handle *h);
 
 /* Number of steps completed since tmx_init. */
@@ -318,7 +321,8 @@ int tmx_batch_restore(tmx_batch *b, const tmx_case *c, const void *buf, long lon
  * tmx_batch_fields and tmx_batch_outlet_im read. */
 int tmx_batch_step(tmx_batch *b, int nsteps, int write_macro_last);
 
-/* Wait for the batch's queued work. */
+/* Wait for the batch's queued work.  TMX_E_CUDA as tmx_sync's, until every mixer
+ * that was there has been removed. */
 int tmx_batch_sync(tmx_batch *b);
 
 /* Slot numbers in use (at most cap written to slots; *n = how many there are). */

@@ -971,6 +971,7 @@ int tmx_init(tmx_handle* h)
 {
     if (!h) return fail(TMX_E_INVALID, "null handle");
     TMX_CK(cudaSetDevice(h->device));
+    TMX_CK(cudaStreamSynchronize(h->stream));
     int rc = inlet_profile_form(h->c, h->stream, h->uin1, h->uin2);
     if (rc) return rc;
     if (h->tbytes == 8) {
@@ -994,6 +995,7 @@ int tmx_init(tmx_handle* h)
     // a step clears the other parity's run counter; the first finds both clear
     if (h->counters) TMX_CK(cudaMemsetAsync(h->counters, 0, 2 * sizeof(int), h->stream));
     TMX_CK(cudaStreamSynchronize(h->stream));
+    if (h->error) *(volatile int*)h->error = 0;  // the earlier state's
     h->steps = 0;
     h->inited = true;
     return TMX_OK;
@@ -1097,6 +1099,7 @@ int tmx_restore(tmx_handle* h, const void* buf, long long size)
         TMX_CK(cudaMemsetAsync(h->counters, 0, 2 * sizeof(int), h->stream));
         TMX_CK(cudaStreamSynchronize(h->stream));
     }
+    if (h->error) *(volatile int*)h->error = 0;  // the earlier state's
     h->cur = 0;
     h->rcur = 0;
     h->steps = hd.steps;
@@ -1375,7 +1378,7 @@ int tmx_step_timed(tmx_handle* h, int nsteps, double* ms_bulk, double* ms_bounda
     if (ms_bulk) *ms_bulk = sb;
     if (ms_boundary) *ms_boundary = sbd;
     if (ms_total) *ms_total = tot;
-    return TMX_OK;
+    return settled(h);
 }
 
 int tmx_time_steps(tmx_handle* h, int nsteps, double* ms)

@@ -557,6 +557,12 @@ int settled(const tmx_batch* b)
     return TMX_OK;
 }
 
+// ... and that flag cleared, where no state from before is left.
+void clear_error(tmx_batch* b)
+{
+    if (b->error) *(volatile int*)b->error = 0;
+}
+
 bool valid_slot(const tmx_batch* b, int slot) { return slot >= 0 && slot < (int)b->slots.size() && b->slots[slot].used; }
 
 }  // namespace
@@ -696,12 +702,20 @@ int admit(tmx_batch* b, const tmx_case* c, const void* buf, long long size, int*
     s.used = true;
     // the stream must be idle before a range of the arena is reused
     TMX_CK(cudaStreamSynchronize(b->stream));
+    // the first mixer of an empty batch: the flag was an earlier one's
+    bool empty = true;
+    for (const Slot& o : b->slots) empty = empty && !o.used;
+    if (empty) clear_error(b);
     int m = -1;
     for (size_t i = 0; i < b->slots.size(); i++)
         if (!b->slots[i].used) {
             m = (int)i;
             break;
         }
+    if (m < 0 && b->slots.size() >= (size_t)tmx::kMaxMixers) {
+        b->arena.release(off, cv.total);
+        return fail(TMX_E_INVALID, "a batch holds %d mixers at most", tmx::kMaxMixers);
+    }
     if (m < 0) {
         m = (int)b->slots.size();
         b->slots.emplace_back();
@@ -712,10 +726,6 @@ int admit(tmx_batch* b, const tmx_case* c, const void* buf, long long size, int*
         b->arena.release(off, cv.total);
         b->slots[m] = Slot();
         return rc;
-    if (m < 0 && b->slots.size() >= (size_t)tmx::kMaxMixers) {
-        b->arena.release(off, cv.total);
-        return fail(TMX_E_INVALID, "a batch holds %d mixers at most", tmx::kMaxMixers);
-    }
     }
     b->dirty = true;
     *slot = m;
@@ -1027,6 +1037,7 @@ int tmx_batch_tune(tmx_batch* b, int steps_per_trial, int* threads_out, int* cel
         float ms = 0;
         cudaEventElapsedTime(&ms, t0, t1);
         ms_step = ms / steps_per_trial;
+        if (rc == TMX_OK) rc = settled(b);
     };
     // the FP64 and FP32 forms have one kernel: their shape stays as it is
     if (b->B->run) trial(best);
@@ -1148,7 +1159,7 @@ int tmx_batch_step_timed(tmx_batch* b, int nsteps, double* ms_interior, double* 
     if (ms_interior) *ms_interior = si;
     if (ms_boundary) *ms_boundary = sb;
     if (ms_total) *ms_total = tot;
-    return TMX_OK;
+    return settled(b);
 }
 
 int tmx_batch_time_steps(tmx_batch* b, int nsteps, double* ms)
@@ -1172,7 +1183,7 @@ int tmx_batch_time_steps(tmx_batch* b, int nsteps, double* ms)
     cudaEventDestroy(t0);
     cudaEventDestroy(t1);
     *ms = f;
-    return rc;
+    return rc ? rc : settled(b);
 }
 
 void tmx_batch_destroy(tmx_batch* b)
