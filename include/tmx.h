@@ -301,7 +301,7 @@ int tmx_batch_create(int precision, long long budget_bytes, int device, tmx_batc
 /* Admit one mixer: carve its state from the arena (TMX_E_NOMEM if no free
  * range of its footprint is left), compute its inlet profiles and initial
  * state (as tmx_init does), and return its slot number.  It joins the next
- * step of the batch. */
+ * step of the batch.  A batch holds 4,194,304 mixers at most. */
 int tmx_batch_add(tmx_batch *b, const tmx_case *c, int *slot);
 
 /* Retire a mixer and return its range to the arena; the slot number may be
@@ -349,15 +349,17 @@ int tmx_batch_fields(tmx_batch *b, int slot, int box, int field, double *host_ou
  * out[6] batch steps taken, out[7] bytes of the batch's work lists. */
 int tmx_batch_info(const tmx_batch *b, long long out[8]);
 
-/* Set the bulk kernel's launch shape: threads per block (128, 256 or 512) and
- * nodes per cell block (a multiple of it). */
+/* Take the FP16 form's flat kernel with this launch shape: threads per block (128,
+ * 256 or 512) and nodes per cell block (a multiple of it).  The FP64 and FP32 forms
+ * have one kernel of its own shape: the values are checked and reported, and
+ * change nothing. */
 int tmx_batch_set_shape(tmx_batch *b, int threads, int cells);
 
 /* Autotune the launch shape on the batch's current mixers: time
- * steps_per_trial steps of every shape of the interior kernel (the flat
- * kernel's (threads, cells) choices; for the FP16 form also every sweep
- * shape with 4, 8, 16 or 32 planes per tile, i.e. nodes per thread), keep
- * the fastest, then with it the boundary kernels' grid (1, 2 or 4 blocks per
+ * steps_per_trial steps of every shape of the FP16 form's interior kernel (the
+ * flat kernel's (threads, cells) choices and every sweep shape with 4, 8, 16
+ * or 32 planes per tile, i.e. nodes per thread; FP64 and FP32: of the one that
+ * there is), keep the fastest, then with it the boundary kernels' grid (1, 2 or 4 blocks per
  * SM or as many as fit) and order (beside the interior kernel or before it,
  * tmx_batch_set_boundary), keep the fastest, then
  * start every mixer again from its initial state.  Returns the threads per
@@ -374,19 +376,17 @@ int tmx_batch_set_sweep(tmx_batch *b, int kind, int zchunk);
 /* The boundary (face and edge) kernels' persistent grid: blocks_per_sm
  * blocks of 128 threads per SM, at most as many as fit; 0 (the default): as
  * many as fit.  after = 1 runs the interior kernel after them, 0 (the
- * default) beside them; the FP64 form always runs it after them.
+ * default) beside them.  (FP16; the FP64 and FP32 forms' step is one launch, the
+ * values only show in tmx_batch_boundary, FP64 always with after = 1.)
  * tmx_batch_boundary returns the face kernel's blocks per SM in use and the
  * order (after may be NULL).  No counterpart in the reference. */
 int tmx_batch_set_boundary(tmx_batch *b, int blocks_per_sm, int after);
 int tmx_batch_boundary(const tmx_batch *b, int *blocks_per_sm, int *after);
 
-/* The interior kernel's shape: out[0] TMX_SHAPE_*,
+/* The interior kernel's shape, as the next step takes it: out[0] TMX_SHAPE_*,
  * out[1] threads per block, out[2] nodes per cell block of the flat kernel,
  * out[3] planes per sweep tile. */
 int tmx_batch_shape(const tmx_batch *b, int out[4]);
-
-/* Run nsteps steps between two CUDA events on the batch's stream and return
- * the elapsed device time (ms). */
 
 /* Run nsteps steps (without the captured graphs) with CUDA events around the
  * interior kernel and around the boundary kernels, the interior kernel after
@@ -394,6 +394,9 @@ int tmx_batch_shape(const tmx_batch *b, int out[4]);
  * kernels alone, and return the summed device times (ms) and that of the
  * whole loop.  Benchmark support; no counterpart in the reference. */
 int tmx_batch_step_timed(tmx_batch *b, int nsteps, double *ms_interior, double *ms_boundary, double *ms_total);
+
+/* Run nsteps steps between two CUDA events on the batch's stream and return
+ * the elapsed device time (ms). */
 int tmx_batch_time_steps(tmx_batch *b, int nsteps, double *ms);
 
 /* Free the batch, its arena and its mixers. */

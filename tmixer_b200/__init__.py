@@ -406,7 +406,7 @@ class Solver:
         """Launch shape of the interior kernel (tmx_set_shape): SHAPE_FLAT, or
         for the FP16 form a sweep shape (SHAPE_SWEEP8, SHAPE_SWEEP4) with zchunk
         planes per tile.  Every shape gives the same bits.  Default: SHAPE_SWEEP4
-        with 3 to 8 planes by size for the FP16 form, SHAPE_FLAT for the others."""
+        with 1 to 8 planes by size for the FP16 form, SHAPE_FLAT for the others."""
         _check(lib().tmx_set_shape(self._h, int(kind), int(zchunk)))
         return self
 
@@ -417,9 +417,9 @@ class Solver:
 
 
 class Batch:
-    """Many mixers of one precision stepped together (tmx_batch_*): one
-    launch per kernel kind per step over all of them, state carved from one
-    device arena of ``budget`` bytes."""
+    """Many mixers of one precision stepped together (tmx_batch_*): one to
+    three launches per step over all of them, state carved from one device
+    arena of ``budget`` bytes."""
 
     def __init__(self, precision: int = TMX_FP16, budget: int = 1 << 30, device: int = 0):
         self.precision = int(precision)
@@ -511,7 +511,8 @@ class Batch:
                     steps=o[6], table_bytes=o[7])
 
     def set_shape(self, threads: int, cells: int) -> None:
-        """The flat interior kernel with this block size and cell-block size."""
+        """The FP16 form's flat interior kernel with this block size and
+        cell-block size (the other forms' step has its own shape)."""
         _check(lib().tmx_batch_set_shape(self._b, int(threads), int(cells)))
 
     def set_sweep(self, kind: int, zchunk: int) -> None:
@@ -522,7 +523,7 @@ class Batch:
     def set_boundary(self, blocks_per_sm: int, after: bool = False) -> None:
         """The boundary kernels' persistent grid in blocks per SM (0: as many
         as fit), and whether the interior kernel runs after them (else beside
-        them; the FP64 form always after)."""
+        them).  FP16; the other forms' step is one launch."""
         _check(lib().tmx_batch_set_boundary(self._b, int(blocks_per_sm), 1 if after else 0))
 
     def shape(self) -> dict:

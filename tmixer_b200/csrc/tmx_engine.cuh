@@ -130,27 +130,8 @@ struct F64 {
         for (int m = 0; m < 4; m++)
             if (m >= first && m < last) v[m] = __ldg(Pin + off(m, q, ps, s));
     }
-    __device__ static void store4(S* __restrict__ Pout, int q, long long ps, int g, const T (&v)[4], const T (&)[4])
-    {
-#pragma unroll
-        for (int m = 0; m < 4; m++) Pout[off(m, q, ps, g)] = v[m];
-    }
-    // collide and store the four fields of direction q (collide_store's
-    // operations, per field)
-    __device__ static void collide_dir(S* __restrict__ Pout, int q, long long ps, int g, const T (&in)[4],
-                                       const T (&r)[4], T pw, const T (&c1)[4], const T (&c2)[4], T w, T rt)
-    {
-        T o[4], f[4];
-#pragma unroll
-        for (int m = 0; m < 4; m++) {
-            f[m] = feq(r[m], pw, q, tiny(r[m]));
-            o[m] = in[m] * c1[m] + c2[m] * f[m];
-        }
-        o[1] = o[1] - w * rt;
-        o[2] = o[2] - w * rt;
-        o[3] = o[3] + (w * rt) * T(2);
-        store4(Pout, q, ps, g, o, f);
-    }
+    // collide and store the four fields of direction q of an edge node, from its
+    // shared-memory row (n[20 f + q]): collide_store's operations, a loop
     __device__ static void collide_edge(S* __restrict__ Pout, int q, long long ps, int g, const T* n, const T (&r)[4],
                                         T pw, const Phys& P, T w, T rt)
     {
@@ -166,9 +147,7 @@ struct F64 {
     }
 };
 
-// The four fields of direction q of an edge node from its shared-memory row
-// (n[20 f + q]) by collide_dir (FP64: a loop over the fields with the same
-// operations, which is shorter).
+// The same of the reduced-precision forms, by their collide_dir.
 template <class PR>
 __device__ __forceinline__ void collide_edge_pairs(typename PR::S* __restrict__ Pout, int q, long long ps, int g,
                                                    const typename PR::T* n, const typename PR::T (&r)[4],
@@ -206,14 +185,6 @@ struct F32 {
         v[2] = x.z;
         v[3] = x.w;
     }
-    __device__ static void encode4(S* p, const T (&v)[4], const T (&)[4])
-    {
-        *(float4*)p = make_float4(v[0], v[1], v[2], v[3]);
-    }
-    __device__ static void store4(S* Pout, int q, long long ps, int g, const T (&v)[4], const T (&feq)[4])
-    {
-        encode4(Pout + off(0, q, ps, g), v, feq);
-    }
     // poly holds w_q * poly_q, so that an equilibrium value is one multiply
     __device__ static void poly(T ux, T uy, T uz, T (&p)[19])
     {
@@ -228,32 +199,7 @@ struct F32 {
     {
         return __fmul_rn(poly_e_omt(ex, ey, ez, ux, uy, uz, omt_term(ux, uy, uz)), w);
     }
-    // the four fields pulled from source s along (ex, ey, ez) of direction q,
-    // as the pairs (flow, A), (B, C)
-    __device__ static void decode_pairs(const S* __restrict__ Pin, const float4* __restrict__, long long ps, int q, int,
-                                        int, int, T, int s, float2& v01, float2& v23)
-    {
-        const float4 x = __ldg((const float4*)(Pin + off(0, q, ps, s)));
-        v01 = make_float2(x.x, x.y);
-        v23 = make_float2(x.z, x.w);
-    }
-    // the stored bytes of (q, s): one 16-byte access
-    using Raw = float4;
-    __device__ static Raw load_raw(const S* __restrict__ Pin, long long ps, int q, int s)
-    {
-        return __ldg((const float4*)(Pin + off(0, q, ps, s)));
-    }
-    __device__ static void decode_raw(const Raw& x, int, int, int, T, const float4&, const float4&, float2& v01,
-                                      float2& v23)
-    {
-        v01 = make_float2(x.x, x.y);
-        v23 = make_float2(x.z, x.w);
-    }
-    __device__ static void decode_pairs_rec(const S* __restrict__ Pin, long long ps, int q, int ex, int ey, int ez,
-                                            T w, int s, const float4& mf, const float4& ms, float2& v01, float2& v23)
-    {
-        decode_raw(load_raw(Pin, ps, q, s), ex, ey, ez, w, mf, ms, v01, v23);
-    }
+    // the four fields pulled from source s: one 16-byte access
     __device__ static void decode4(const S* __restrict__ Pin, const float4* __restrict__, long long ps, int q, int,
                                    int, int, T, int s, T (&v)[4])
     {
@@ -316,28 +262,6 @@ struct F16 {
     __host__ __device__ static long long off(int fld, int q, long long ps, long long g)
     {
         return (((long long)q * ps + g) << 2) + fld;
-    }
-    __device__ static void load4(const S* p, T (&v)[4])
-    {
-        const uint2 x = __ldg((const uint2*)p);
-        const float2 lo = __half22float2(*(const __half2*)&x.x), hi = __half22float2(*(const __half2*)&x.y);
-        v[0] = lo.x;
-        v[1] = lo.y;
-        v[2] = hi.x;
-        v[3] = hi.y;
-    }
-    __device__ static void encode4(S* p, const T (&v)[4], const T (&feq)[4])
-    {
-        const __half2 lo = __floats2half2_rn(v[0] - feq[0], v[1] - feq[1]);
-        const __half2 hi = __floats2half2_rn(v[2] - feq[2], v[3] - feq[3]);
-        uint2 x;
-        x.x = *(const unsigned*)&lo;
-        x.y = *(const unsigned*)&hi;
-        *(uint2*)p = x;
-    }
-    __device__ static void store4(S* Pout, int q, long long ps, int g, const T (&v)[4], const T (&feq)[4])
-    {
-        encode4(Pout + off(0, q, ps, g), v, feq);
     }
     // poly holds w_q * poly_q (rounded as below), so that an equilibrium
     // value is one multiply
@@ -644,11 +568,10 @@ __device__ __forceinline__ void lp_finish(const StepPtrs& X, const Geom& G, cons
     }
 }
 
-// One interior node (b, i, j, k) = g for the reduced-precision forms (FP32
-// arithmetic): every source index and (FP16 form) every writer's record
-// (from rec) is fetched once per direction and all 76 populations decoded in
-// one pass, which the FP32 register budget affords (the FP64 form loads field
-// by field).  The arithmetic does not depend on where the records and the
+// One interior node (b, i, j, k) = g of the FP16 form: every source index and
+// every writer's record (from rec) is fetched once per direction and all 76
+// populations decoded in one pass, which the FP32 register budget affords (the
+// FP64 form's step goes field by field).  The arithmetic does not depend on where the records and the
 // stored populations (pop) come from.
 //
 // With XF the node may be an x face (xf.cls; the sweep kernels): the flow is
@@ -1704,11 +1627,9 @@ __device__ __forceinline__ void edge_node(const StepPtrs& X, const Geom& G, cons
     __syncwarp();  // buf is free again
 }
 
-// The post-closure populations of field fld of the boundary node in c.  A
-// species on a wall face is a zero-gradient copy of an interior node's pulled
-// populations (Tmixer.cpp:2766-4237), so it pulls that node directly.
 // The interior neighbour whose pulled species populations a face node copies
-// (zero-gradient closure), or (0, 0, 0) for a face without that closure.
+// (zero-gradient closure, Tmixer.cpp:2766-4237), or (0, 0, 0) for a face without
+// that closure.
 __device__ __forceinline__ void face_copy_offset(int cls, int& di, int& dj, int& dk)
 {
     di = dj = dk = 0;
@@ -1725,7 +1646,7 @@ __device__ __forceinline__ void face_copy_offset(int cls, int& di, int& dj, int&
 }
 
 // ---------------------------------------------------------------------------
-// boundary nodes of a compact, class-sorted list, four threads per node: lane
+// boundary nodes of a compact, class-sorted list (FP16), four threads per node: lane
 // fld (0 flow, 1 A, 2 B, 3 C) pulls, closes and collides its own field.  Every
 // closure reads only its own field, so the lanes need each other only for
 // the moments: the flow lane's density and velocity and the species
@@ -1756,13 +1677,14 @@ __device__ __forceinline__ bool lane_dir(int lane, int& q, int& ex, int& ey, int
 //      (one vector load, one moment record and one polynomial per
 //      direction), species of a zero-gradient face from the interior
 //      neighbour, into the node's 76-value buffer in shared memory;
-//   2. fields: lane fld closes field fld (the same closures as
-//      boundary_lane) and forms its density; moments by shuffle;
+//   2. fields: lane fld closes field fld and forms its density; moments by
+//      shuffle;
 //   3. directions again: collide and store the four fields of each of its
 //      directions with one vector store.
-// Every value is computed with the operations, in the order, of the
-// one-field-per-thread step (pull_node, the closures, sum19, momentum,
-// collide_store), so the FP64 form stays bit-exact.
+// The FP16 form's face kernel, and its edge kernel beside the tiles and the flat
+// kernel.  (A warp per edge node, edge_node, is slower beside them: a step at
+// W=16 29 us against 20.7, at W=32 64 against 55, the boundary kernels of 64 mixers
+// 584 against 448.)
 template <class PR, bool FACES>
 __device__ __forceinline__ void boundary_lane_lp(const StepPtrs& X, const Geom& G, const Phys& P, int write_macro,
                                                  int g, int cls, int fld, unsigned mask, int lead,
