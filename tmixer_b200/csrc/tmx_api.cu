@@ -587,9 +587,12 @@ int enqueue_step(tmx_handle* h, int cur, int write_macro, cudaEvent_t* ev, bool 
     X.uin2 = h->uin_d[1];
     if (h->K->run[0]) return enqueue_run(h, X, cur, write_macro, ev, overlap);
     // FP16 by up to four rounds of tiles: the wall rows with them.  Beyond, and for
-    // the timed parts, a face kernel: tiles without the walls' and edges' code beside
-    // them run faster (together / apart: 524,288 nodes 55.2 / 56.4 us, 1.8M 149.4 /
-    // 150.6, 4.2M 318.6 / 317.7, 4.9M 428 / 421).
+    // the timed parts, a face kernel: tiles without the walls' and edges' code spill
+    // less (76 B loaded back a thread against 104), and the face kernel's share
+    // falls with the size.  Together / apart (each repeats to 0.2%): 0.75M nodes 75.0 /
+    // 80.2 us, 1.0M 97.9 / 94.7, 1.4M 117.2 / 120.9, 1.8M 146.5 / 148.4; beyond four
+    // rounds 2.2M 186.6 / 187.4, 2.8M 225.6 / 226.9, 4.2M 311.7 / 311.7, the reference
+    // case's 4.9M 420.5 / 415.3.
     const SweepShape* sh = sweep_shape(h->shape);
     if (sh && !ev && h->ntiles <= 4 * h->sweep_slots) return enqueue_sweep(h, sh, X, write_macro, overlap);
     TMX_CK(cudaEventRecord(h->fork, h->stream));

@@ -269,9 +269,12 @@ inline int sweep_planes(const Geom& G, int slots, int rest)
     return 8;
 }
 // ... and of an FP16 batch that no shape was set for: 4, or 8 where those make
-// kBatchRounds rounds of tiles or more (by 4 / 8 planes: 8 mixers of 544,000 nodes,
-// one round, 81 / 90 us; 4 of 4.3M nodes, 7 rounds, 409 / 401 us; 64 of 41M nodes,
-// 68 rounds, 3.71 / 3.58 ms).
+// kBatchRounds rounds of tiles or more.  Up to two rounds the end of the last one
+// decides, either way (by 4 / 8 planes: 8 mixers of 544,000 nodes, one round, 81 /
+// 90 us; 3 of 415,000, 0.9 rounds, 63.4 / 55.6; 3 of 1.1M, 2.0 rounds, 125.8 / 127.2);
+// then fewer records read twice count for more with the size (2.6 rounds 163.5 /
+// 161.6, 4.7 rounds 257.4 / 256.1, 7.2 rounds 381 / 377, 12 rounds 625 / 605, 23
+// rounds 1,228 / 1,186, 64 mixers of 41M nodes, 68 rounds, 3.71 / 3.58 ms).
 constexpr int kBatchPlanes = 4, kBatchRounds = 4;
 
 // Checkpoint layout (tmx_checkpoint, tmx_batch_checkpoint): this header, then
