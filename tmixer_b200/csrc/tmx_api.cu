@@ -1145,7 +1145,10 @@ int tmx_populations(tmx_handle* h, int box, int fld, double* host_out)
         return settled(h);
     }
     // reduced precision: widen on the host; the FP16 form adds back feq of
-    // the writing node's moments exactly as the kernels do (tmx_engine.cuh)
+    // the writing node's moments exactly as the kernels do (tmx_engine.cuh).  (The
+    // copies below do not wait for the handle's stream by themselves.)
+    TMX_CK(cudaStreamSynchronize(h->stream));
+    if (const int rc = settled(h)) return rc;
     std::vector<double> wide(n);
     std::vector<unsigned char> raw(4 * n * h->sbytes);
     // moment records {(rho, cA, cB, cC), (ux, uy, uz, 1 - 1.5|u|^2)}, 8 floats per node
