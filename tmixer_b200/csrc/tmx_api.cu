@@ -461,6 +461,11 @@ void error_flag_give(int* flag)
 
 namespace {
 
+// cudaMemcpy from pageable memory may return before the last of it has arrived, and
+// a handle's stream does not wait for such copies: a call whose copies a step
+// reads ends with this.
+cudaError_t copies_arrived() { return cudaStreamSynchronize(cudaStreamLegacy); }
+
 void drop_graphs(tmx_handle* h)
 {
     cudaGraphExec_t* all[6] = {&h->graph[0][0], &h->graph[0][1],   &h->graph[1][0],
@@ -948,6 +953,7 @@ int tmx_set_shape(tmx_handle* h, int kind, int zchunk)
         if (!t.empty()) {
             cudaError_t e = cudaMalloc((void**)&d, t.size() * sizeof(int4));
             if (e == cudaSuccess) e = cudaMemcpy(d, t.data(), t.size() * sizeof(int4), cudaMemcpyHostToDevice);
+            if (e == cudaSuccess) e = copies_arrived();
             if (e != cudaSuccess) {
                 cudaFree(d);
                 cudaGetLastError();
@@ -986,6 +992,7 @@ int tmx_init(tmx_handle* h)
         TMX_CK(cudaMemcpy(h->uin_d[0], a.data(), a.size() * sizeof(float), cudaMemcpyHostToDevice));
         TMX_CK(cudaMemcpy(h->uin_d[1], b.data(), b.size() * sizeof(float), cudaMemcpyHostToDevice));
     }
+    TMX_CK(copies_arrived());
     h->cur = 0;
     h->rcur = 0;
     tmx::StepPtrs X{};
@@ -1098,6 +1105,7 @@ int tmx_restore(tmx_handle* h, const void* buf, long long size)
         TMX_CK(cudaMemcpy(h->uin_d[0], a.data(), nu * 4, cudaMemcpyHostToDevice));
         TMX_CK(cudaMemcpy(h->uin_d[1], c.data(), nu * 4, cudaMemcpyHostToDevice));
     }
+    TMX_CK(copies_arrived());
     if (h->counters) {
         TMX_CK(cudaMemsetAsync(h->counters, 0, 2 * sizeof(int), h->stream));
         TMX_CK(cudaStreamSynchronize(h->stream));
